@@ -35,7 +35,7 @@ void release_plan(hyset_ctx* ctx, BatchPlan& bp) {
                           &bj->ix_mid.pos, &bj->bits_r, &bj->bits_s, &bj->pairs};
         for (DevBuf* d : bufs) d->release(s);
     }
-    DevBuf* bufs[] = {&bp.desc, &bp.unit_off, &bp.counts, &bp.work};
+    DevBuf* bufs[] = {&bp.desc, &bp.unit_off, &bp.counts, &bp.work, &bp.sorts};
     for (DevBuf* d : bufs) d->release(s);
     bp.sc.release(s);
     cudaStreamSynchronize(s);
@@ -85,6 +85,7 @@ hyset_status batch_record(hyset_ctx* ctx, BatchPlan& bp) {
     }
     CK(launch_batch_join(bp.desc.as<BatchDesc>(), bp.unit_off.as<uint32_t>(), n, bp.work.as<unsigned int>(),
                          ctx->sm_count, s));
+    CK(sort_pairs_clusters(bp.sorts.as<PairSortJob>(), bp.n_sorts, s));
     return HYSET_OK;
 }
 
@@ -235,6 +236,7 @@ hyset_status batch_prepare(hyset_ctx* ctx, const hyset_join_desc* joins, uint32_
     CK(plan->work.ensure(16 + 8 * (size_t)n, s));  // the shared launch's counter, then two per solo join
     std::vector<BatchDesc> ordered(n);
     std::vector<uint32_t> unit_off(n + 1, 0);
+    std::vector<PairSortJob> sorts;
     for (uint32_t k = 0; k < n; ++k) {
         const uint32_t j = plan->order[k];
         ordered[k] = desc[j];
@@ -243,12 +245,18 @@ hyset_status batch_prepare(hyset_ctx* ctx, const hyset_join_desc* joins, uint32_
                                 plan->counts.as<unsigned long long>() + j, bj.cap, bj.o.count_only ? 1 : 0,
                                 bj.swapped ? 1 : 0};
         unit_off[k + 1] = unit_off[k] + bj.units;
+        if (bj.o.sort_pairs && !bj.o.count_only) sorts.push_back(pair_sort_job(ordered[k].P));
     }
     plan->host_desc = ordered;
     CK(plan->desc.ensure(n * sizeof(BatchDesc), s));
     CK(plan->unit_off.ensure((n + 1) * 4, s));
     CK(cudaMemcpyAsync(plan->desc.p, ordered.data(), n * sizeof(BatchDesc), cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(plan->unit_off.p, unit_off.data(), (n + 1) * 4, cudaMemcpyHostToDevice, s));
+    plan->n_sorts = (uint32_t)sorts.size();
+    if (!sorts.empty()) {
+        CK(plan->sorts.ensure(sorts.size() * sizeof(PairSortJob), s));
+        CK(cudaMemcpyAsync(plan->sorts.p, sorts.data(), sorts.size() * sizeof(PairSortJob), cudaMemcpyHostToDevice, s));
+    }
     CK(cudaStreamSynchronize(s));
     ctx->batch = std::move(plan);
     BatchPlan& bp = *ctx->batch;
@@ -307,12 +315,28 @@ hyset_status hyset_batch_join(hyset_ctx* ctx, const hyset_join_desc* joins, uint
     CK(cudaGraphLaunch(bp.exec, s));
     CK(cudaEventRecord(ctx->ev1, s));
     std::vector<unsigned long long> counts(n_joins);
-    CK(cudaMemcpyAsync(counts.data(), bp.counts.p, n_joins * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+    void* stage = nullptr;
+    ST(host_stage(ctx, n_joins * sizeof(unsigned long long), &stage));
+    CK(cudaMemcpyAsync(stage, bp.counts.p, n_joins * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    std::memcpy(counts.data(), stage, n_joins * sizeof(unsigned long long));
     float ms = 0;
     CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
+    // the joins' pairs come back through pinned memory in one go when they are
+    // a few MB together (a copy into pageable memory waits for itself, one join
+    // after the other)
+    constexpr uint64_t STAGED_PAIRS = 2ull << 20;
+    uint64_t total = 0;
+    for (uint32_t j = 0; j < n_joins; ++j)
+        if (!bp.joins[j]->o.count_only && !bp.joins[j]->o.device_pairs && counts[j] <= bp.joins[j]->cap)
+            total += counts[j];
+    const bool staged = total <= STAGED_PAIRS;
+    if (staged && total) ST(host_stage(ctx, total * sizeof(hyset_pair), &stage));
+    hyset_pair* from = static_cast<hyset_pair*>(stage);
     std::vector<std::unique_ptr<hyset_result>> out(n_joins);
     hyset_status st = HYSET_OK;
+    bool overflowed = false;
+    uint64_t at = 0;
     for (uint32_t j = 0; j < n_joins && st == HYSET_OK; ++j) {
         BatchJoin& bj = *bp.joins[j];
         out[j] = std::make_unique<hyset_result>();
@@ -322,15 +346,12 @@ hyset_status hyset_batch_join(hyset_ctx* ctx, const hyset_join_desc* joins, uint
         r->probe_batch = bj.unit_probes;
         r->device_ms = ms;  // the whole batch: one launch sequence
         r->count = counts[j];
-        if (!bj.o.count_only && counts[j] > bj.cap) {
-            // the join's buffer overflowed: run it alone with room for every pair
-            hyset_join_opts o2 = bj.o;
-            o2.pair_capacity = counts[j] + 1024;
-            st = do_join(ctx, bj.swapped ? bj.S : bj.R, bj.swapped ? bj.R : bj.S, &o2, r);
+        if (bj.o.count_only) continue;
+        if (counts[j] > bj.cap) {
+            overflowed = true;
             continue;
         }
-        if (bj.o.count_only) continue;
-        if (bj.o.sort_pairs) {
+        if (bj.o.sort_pairs && counts[j] > PAIR_SORT_MAX) {  // more than the graph's sort holds
             st = sort_device_pairs(ctx, bj.pairs.as<uint2>(), counts[j], bj.swapped ? bj.R->n : bj.S->n,
                                    bj.swapped ? bj.S->n : bj.R->n);
             if (st != HYSET_OK) break;
@@ -339,16 +360,35 @@ hyset_status hyset_batch_join(hyset_ctx* ctx, const hyset_join_desc* joins, uint
             r->device_pairs = bj.pairs.p;
             continue;
         }
-        r->pairs.resize(counts[j]);
         r->has_pairs = 1;
+        r->pairs.resize(counts[j]);
         if (counts[j]) {
-            cudaError_t e = cudaMemcpyAsync(r->pairs.data(), bj.pairs.p, counts[j] * sizeof(hyset_pair),
-                                            cudaMemcpyDeviceToHost, s);
+            cudaError_t e = cudaMemcpyAsync(staged ? from + at : r->pairs.data(), bj.pairs.p,
+                                            counts[j] * sizeof(hyset_pair), cudaMemcpyDeviceToHost, s);
             if (e != cudaSuccess) st = fail(ctx, HYSET_E_CUDA, "batch pair copy", e);
+            at += counts[j];
         }
     }
-    if (st == HYSET_OK) CK(cudaStreamSynchronize(s));
+    const cudaError_t e = cudaStreamSynchronize(s);  // also when a step failed: the copies write into `out`
     if (st != HYSET_OK) return st;
+    CK(e);
+    if (staged) {
+        at = 0;
+        for (uint32_t j = 0; j < n_joins; ++j) {
+            hyset_result* r = out[j].get();
+            if (!r->has_pairs) continue;
+            std::copy(from + at, from + at + r->count, r->pairs.data());
+            at += r->count;
+        }
+    }
+    // a join whose buffer overflowed is run alone with room for every pair
+    for (uint32_t j = 0; overflowed && j < n_joins; ++j) {
+        BatchJoin& bj = *bp.joins[j];
+        if (bj.o.count_only || counts[j] <= bj.cap) continue;
+        hyset_join_opts o2 = bj.o;
+        o2.pair_capacity = counts[j] + 1024;
+        ST(do_join(ctx, bj.swapped ? bj.S : bj.R, bj.swapped ? bj.R : bj.S, &o2, out[j].get()));
+    }
     for (uint32_t j = 0; j < n_joins; ++j) results[j] = out[j].release();
     return HYSET_OK;
 }

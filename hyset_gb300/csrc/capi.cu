@@ -91,7 +91,7 @@ hyset_status hyset_create(int device, hyset_ctx** out) {
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev1);
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ek0);
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ek1);
-    if (e == cudaSuccess) e = cudaMallocHost((void**)&ctx->h_flags, 64);
+    if (e == cudaSuccess) e = cudaMallocHost((void**)&ctx->h_flags, 128);
     if (e == cudaSuccess) {
         cudaMemPool_t pool;
         if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) {

@@ -118,6 +118,9 @@ hyset_status autotune_bits(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const h
                            bool self, uint32_t p_lo, uint32_t p_hi, uint32_t* bits, int* vmode = nullptr,
                            uint32_t* batch = nullptr, float* est_ms = nullptr);
 
+// `count` pairs from device memory into out, through pinned memory up to a
+// few MB (a copy into pageable memory waits for itself).
+hyset_status read_pairs(hyset_ctx* ctx, const void* d_pairs, uint64_t count, std::vector<hyset_pair>& out);
 // ---- joins (join_host.cu) -----------------------------------------------------
 hyset_status sort_device_pairs(hyset_ctx* ctx, uint2* pairs, uint64_t n, uint32_t n_probe, uint32_t n_indexed);
 bool swap_sides(const hyset_coll* R, const hyset_coll* S, const hyset_join_opts* o);
@@ -127,8 +130,17 @@ hyset_status run_join(hyset_ctx* ctx, JoinParams P, int tech, int vmode, const h
 // segments (JoinParams::heavy_from, segs, seg_slots); none for banded joins.
 // The launch's work buffer then needs two zeroed counters.
 void split_heavy(const hyset_coll* S, const Bounds* b, JoinParams& P);
+// Behind a join's launch, before the host knows its number of pairs: orders
+// the pairs when asked (up to PAIR_SORT_MAX) and starts the copies of their
+// number (joined_count, after the stream has synchronised) and of the first
+// EARLY_PAIRS of them.
+constexpr uint64_t EARLY_PAIRS = 8192;
+PairSortJob pair_sort_job(const JoinParams& P);
+hyset_status enqueue_result(hyset_ctx* ctx, const JoinParams& P, const hyset_join_opts* o);
+uint64_t joined_count(const hyset_ctx* ctx);
 // The pairs of a finished join (res->count of them in the context's pair
-// buffer): sorted when asked, left on the device or copied to the host.
+// buffer, enqueue_result done and the stream synchronised): sorted when asked,
+// left on the device or copied to the host.
 hyset_status deliver_pairs(hyset_ctx* ctx, const JoinParams& P, const hyset_join_opts* o, hyset_result* res);
 hyset_status do_join(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const hyset_join_opts* o, hyset_result* res);
 

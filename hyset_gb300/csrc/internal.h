@@ -151,7 +151,8 @@ struct BatchPlan {
     Scratch sc;  // owned by the plan: its graph holds these addresses
     std::vector<std::unique_ptr<BatchJoin>> joins;
     std::vector<uint32_t> order;  // joins[order[k]] is descriptor k (heaviest first)
-    DevBuf desc, unit_off, counts, work;
+    DevBuf desc, unit_off, counts, work, sorts;
+    uint32_t n_sorts = 0;  // joins whose pairs are put in order by the graph (sorts: their PairSortJobs)
     std::vector<BatchDesc> host_desc;  // the joins' descriptors in launch order (solo joins launch from them)
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -173,7 +174,7 @@ struct hyset_ctx {
     hs::Scratch own;
     hs::Scratch* sc = &own;
     hs::DevBuf s_pairs, s_count, s_work, s_stats, s_flags;
-    uint32_t* h_flags = nullptr;  // pinned host words for small device-to-host reads
+    uint32_t* h_flags = nullptr;  // pinned host words for small device-to-host reads ([16..17]: a join's count)
     void* h_stage = nullptr;      // pinned staging for larger reads (grows)
     size_t h_stage_bytes = 0;
     std::unique_ptr<hs::BatchPlan> batch;

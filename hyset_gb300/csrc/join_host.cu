@@ -77,10 +77,10 @@ hyset_status run_join(hyset_ctx* ctx, JoinParams P, int tech, int vmode, const h
         }
         CK(cudaEventRecord(ctx->ek1, s));
         CK(cudaEventRecord(ctx->ev1, s));
-        unsigned long long count = 0;
-        CK(cudaMemcpyAsync(&count, ctx->s_count.p, 8, cudaMemcpyDeviceToHost, s));
+        ST(enqueue_result(ctx, P, o));
         if (P.stats) CK(cudaMemcpyAsync(res->stats, P.stats, 64, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
+        const uint64_t count = joined_count(ctx);
         float ms = 0, kms = 0;
         CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
         CK(cudaEventElapsedTime(&kms, ctx->ek0, ctx->ek1));
@@ -110,23 +110,62 @@ void split_heavy(const hyset_coll* S, const Bounds* b, JoinParams& P) {
         }
 }
 
-hyset_status deliver_pairs(hyset_ctx* ctx, const JoinParams& P, const hyset_join_opts* o, hyset_result* res) {
+PairSortJob pair_sort_job(const JoinParams& P) {
+    return PairSortJob{P.out.pairs, P.out.count, P.out.cap, (int)bits_for(P.out.swap ? P.R.n : P.S.n),
+                       (int)bits_for(P.out.swap ? P.S.n : P.R.n)};
+}
+
+hyset_status enqueue_result(hyset_ctx* ctx, const JoinParams& P, const hyset_join_opts* o) {
     cudaStream_t s = ctx->stream;
-    const bool count_only = o->count_only != 0;
-    if (!count_only && o->sort_pairs)
+    if (!o->count_only && o->sort_pairs) CK(sort_pairs_cluster(pair_sort_job(P), s));
+    CK(cudaMemcpyAsync(ctx->h_flags + 16, P.out.count, 8, cudaMemcpyDeviceToHost, s));
+    if (!o->count_only && !o->device_pairs) {
+        const uint64_t early = std::min<uint64_t>(P.out.cap, EARLY_PAIRS);
+        void* stage = nullptr;
+        ST(host_stage(ctx, early * sizeof(hyset_pair), &stage));
+        if (early)
+            CK(cudaMemcpyAsync(stage, P.out.pairs, early * sizeof(hyset_pair), cudaMemcpyDeviceToHost, s));
+    }
+    return HYSET_OK;
+}
+
+uint64_t joined_count(const hyset_ctx* ctx) {
+    uint64_t count = 0;
+    std::memcpy(&count, ctx->h_flags + 16, 8);
+    return count;
+}
+
+hyset_status read_pairs(hyset_ctx* ctx, const void* d_pairs, uint64_t count, std::vector<hyset_pair>& out) {
+    constexpr uint64_t STAGED_BYTES = 16ull << 20;  // larger results are copied straight to their place
+    out.resize(count);
+    if (count == 0) return HYSET_OK;
+    const size_t bytes = count * sizeof(hyset_pair);
+    void* to = out.data();
+    if (bytes <= STAGED_BYTES) ST(host_stage(ctx, bytes, &to));
+    CK(cudaMemcpyAsync(to, d_pairs, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    if (to != out.data()) std::memcpy(out.data(), to, bytes);
+    return HYSET_OK;
+}
+
+hyset_status deliver_pairs(hyset_ctx* ctx, const JoinParams& P, const hyset_join_opts* o, hyset_result* res) {
+    if (o->count_only) return HYSET_OK;
+    const bool resort = o->sort_pairs && res->count > PAIR_SORT_MAX;  // not sorted behind the join
+    if (resort)
         ST(sort_device_pairs(ctx, ctx->s_pairs.as<uint2>(), res->count, P.out.swap ? P.R.n : P.S.n,
                              P.out.swap ? P.S.n : P.R.n));
-    if (!count_only && o->device_pairs) {
-        if (o->sort_pairs) CK(cudaStreamSynchronize(s));  // device pairs are final when the call returns
+    if (o->device_pairs) {
+        if (resort) CK(cudaStreamSynchronize(ctx->stream));  // device pairs are final when the call returns
         res->device_pairs = ctx->s_pairs.p;
-    } else if (!count_only) {
-        res->pairs.resize(res->count);
-        if (res->count)
-            CK(cudaMemcpyAsync(res->pairs.data(), ctx->s_pairs.p, res->count * sizeof(hyset_pair),
-                               cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        res->has_pairs = 1;
+        return HYSET_OK;
     }
+    if (!resort && res->count <= std::min<uint64_t>(P.out.cap, EARLY_PAIRS)) {  // all of them have come with their number
+        const hyset_pair* early = static_cast<const hyset_pair*>(ctx->h_stage);
+        res->pairs.assign(early, early + res->count);
+    } else {
+        ST(read_pairs(ctx, ctx->s_pairs.p, res->count, res->pairs));
+    }
+    res->has_pairs = 1;
     return HYSET_OK;
 }
 

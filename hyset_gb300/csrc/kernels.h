@@ -172,6 +172,23 @@ cudaError_t iota_u32(uint32_t* out, uint64_t n, cudaStream_t s);
 cudaError_t sort_pair_list(uint2* pairs, uint64_t n, int first_bits, int second_bits, uint32_t* a, uint32_t* b,
                            uint32_t* c, uint32_t* d, uint32_t* scratch, cudaStream_t s);
 
+// ---- sort.cu ---------------------------------------------------------------
+// The same order in one launch, for results of at most PAIR_SORT_MAX pairs:
+// the number of pairs is read on the device, so the sort is enqueued behind
+// the join without a host round trip.  A result of more pairs (or one that
+// overflowed its buffer: *count > cap) is left as it is.
+constexpr uint64_t PAIR_SORT_MAX = 65536;
+struct PairSortJob {
+    uint2* pairs;
+    const unsigned long long* count;
+    unsigned long long cap;
+    int first_bits, second_bits;  // at most 32 each
+};
+cudaError_t prepare_sort_kernels();
+cudaError_t sort_pairs_cluster(const PairSortJob& job, cudaStream_t s);
+// Many results in one launch, a cluster each (jobs in device memory).
+cudaError_t sort_pairs_clusters(const PairSortJob* d_jobs, uint32_t n_jobs, cudaStream_t s);
+
 // Input contract check of an uploaded collection.  flags[0] gets bit 1 for an
 // empty set, 2 for a set whose tokens are not strictly ascending, 4 for a size
 // smaller than the previous set's, 8 for a set reaching past n_tokens;

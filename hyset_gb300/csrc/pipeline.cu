@@ -547,13 +547,12 @@ hyset_status hyset_self_join_host(hyset_ctx* ctx, const uint32_t* tokens, uint64
             CK(cudaEventRecord(ctx->ek1, s));
             CK(cudaEventRecord(ctx->ev1, s));
             CK(cudaMemcpyAsync(f, ctx->s_flags.p, 8, cudaMemcpyDeviceToHost, s));
-            CK(cudaMemcpyAsync(f + 10, ctx->s_count.p, 8, cudaMemcpyDeviceToHost, s));
+            ST(enqueue_result(ctx, SP, o));
             if (SP.stats) CK(cudaMemcpyAsync(res->stats, SP.stats, 64, cudaMemcpyDeviceToHost, s));
             CK(cudaStreamSynchronize(s));
             const hyset_status vs = verdict();
             if (vs != HYSET_OK) return bail(vs);
-            unsigned long long count = 0;
-            std::memcpy(&count, f + 10, 8);
+            const uint64_t count = joined_count(ctx);
             // a list that outgrew its record, a token past the assumed universe
             // or a full pair buffer: the join is run again below (records, then lists)
             if (!(f[0] & REC_OVERFLOW) && f[1] + 1 <= U && (o->count_only || count <= cap)) {

@@ -848,6 +848,8 @@ size_t radix_scratch_words(uint64_t n) {
 }
 
 cudaError_t prepare_kernels() {
+    const cudaError_t e = prepare_sort_kernels();
+    if (e != cudaSuccess) return e;
     // the downsweep's per-warp digit counts need more than the default 48 KB
     return cudaFuncSetAttribute(k_radix_downsweep, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)sizeof(RadixSmem));
