@@ -22,7 +22,7 @@ BUILD = os.path.join(PKG, "_build")
 LIB = os.path.join(PKG, "libhyset_gb300.so")
 SYNTH = os.path.join(PKG, "libhyset_synth.so")
 
-CUDA_SOURCES = ["primitives.cu", "sort.cu", "join.cu", "join_tm.cu", "batch.cu", "mlp.cu", "stats.cu", "parse.cu", "noalloc.cu",
+CUDA_SOURCES = ["primitives.cu", "sort.cu", "join.cu", "window.cu", "join_tm.cu", "batch.cu", "mlp.cu", "stats.cu", "parse.cu", "noalloc.cu",
                 # host side of the C ABI
                 "capi.cu", "collection.cu", "bounds.cu", "index_host.cu", "plan.cu", "join_host.cu", "pipeline.cu",
                 "batch_host.cu", "handlers.cu", "verifier.cu", "ring.cu"]

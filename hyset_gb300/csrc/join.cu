@@ -199,7 +199,10 @@ cudaError_t launch_join(const JoinParams& P, int technique, int vmode, int sm_co
     if (P.p_hi <= P.p_lo) return cudaSuccess;
     if (technique == TECH_FGSS)
         return vmode == 2 ? dispatch_words<TECH_FGSS, 2>(P, sm_count, s) : dispatch_words<TECH_FGSS, 1>(P, sm_count, s);
-    // BITMAP and DIRECT share the enumeration kernel; DIRECT runs without signatures.
+    // signatures over the windows: tiles of probes (window.cu), whose lanes do
+    // not count their work; the enumeration kernel serves a launch with work
+    // counters and DIRECT, which has no signatures
+    if (technique == TECH_BITMAP && P.bits_R && P.words && !P.stats) return launch_window(P, vmode, sm_count, s);
     JoinParams Q = P;
     if (technique == TECH_DIRECT) Q.bits_R = Q.bits_S = nullptr;
     return vmode == 2 ? dispatch_words<TECH_BITMAP, 2>(Q, sm_count, s) : dispatch_words<TECH_BITMAP, 1>(Q, sm_count, s);

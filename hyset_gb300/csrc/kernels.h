@@ -267,6 +267,11 @@ cudaError_t launch_join(const JoinParams& P, int technique, int vmode, int sm_co
 // Warps of one launch_join (the blocks per SM its kernels are compiled for).
 uint32_t join_resident_warps(int sm_count);
 
+// ---- window.cu ---------------------------------------------------------------
+// The signature technique over the length windows (P.words in {1, 2, 4, 8},
+// signatures set, no work counters): one launch.
+cudaError_t launch_window(const JoinParams& P, int vmode, int sm_count, cudaStream_t s);
+
 // ---- join_tm.cu ------------------------------------------------------------
 // Token groups: for every token, the entries (set, pos | size << 16) of the sets
 // whose first pre[size] tokens contain it.  counts must be zeroed; cursor holds
