@@ -136,6 +136,7 @@ hyset_status hyset_handler_join_blocks(hyset_handler* h, const hyset_block* firs
     } else {
         P.bits_R = P.bits_S = h->bits.as<uint64_t>();
         P.words = h->words;
+        split_window(h->coll, h->coll, h->bounds, h->words, P);
     }
     const int tech = h->technique == HYSET_TECH_FGSS ? TECH_FGSS : TECH_BITMAP;
     const int vmode = 1;

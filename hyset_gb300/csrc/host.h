@@ -138,6 +138,9 @@ constexpr uint64_t EARLY_PAIRS = 8192;
 PairSortJob pair_sort_job(const JoinParams& P);
 hyset_status enqueue_result(hyset_ctx* ctx, const JoinParams& P, const hyset_join_opts* o);
 uint64_t joined_count(const hyset_ctx* ctx);
+// The signature technique's probes that are taken in small units
+// (JoinParams::heavy_from, heavy_lo); words: 64-bit words per signature.
+void split_window(const hyset_coll* R, const hyset_coll* S, const Bounds* b, int words, JoinParams& P);
 // The pairs of a finished join (res->count of them in the context's pair
 // buffer, enqueue_result done and the stream synchronised): sorted when asked,
 // left on the device or copied to the host.

@@ -110,6 +110,22 @@ void split_heavy(const hyset_coll* S, const Bounds* b, JoinParams& P) {
         }
 }
 
+void split_window(const hyset_coll* R, const hyset_coll* S, const Bounds* b, int words, JoinParams& P) {
+    P.heavy_from = 0xFFFFFFFFu;
+    // two sets of many tokens differ in half of the signature's bits, give or
+    // take sqrt(bits) / 2: from an admissible distance of three eighths on,
+    // unrelated pairs start to pass (64 bits: at 24, two deviations short of 32)
+    const uint32_t bits = 64u * (uint32_t)words, L = std::min(S->max_size, b->L);
+    for (uint32_t l = 1; l <= L; ++l) {
+        const uint32_t mo = minoverlap_of(b->sim, l, l, b->tau);
+        if (2 * l - 2 * mo < bits * 3 / 8) continue;
+        P.heavy_from = S->h_first_ge[l];
+        const uint32_t ms = std::min(b->minsize[l], R->max_size + 1);
+        P.heavy_lo = R->h_first_ge[ms];
+        return;
+    }
+}
+
 PairSortJob pair_sort_job(const JoinParams& P) {
     return PairSortJob{P.out.pairs, P.out.count, P.out.cap, (int)bits_for(P.out.swap ? P.R.n : P.S.n),
                        (int)bits_for(P.out.swap ? P.S.n : P.R.n)};
@@ -288,6 +304,7 @@ hyset_status do_join(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const hyset_j
         if (P.X2.set) P.grab = std::min<uint32_t>(P.grab, 16);  // two bands per probe share a warp batch
         split_heavy(S, b, P);
     }
+    if (tech == HYSET_TECH_BITMAP && words) split_window(R, S, b, words, P);
     if (words) CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_join, 0));
     int ktech = tech == HYSET_TECH_FGSS ? TECH_FGSS : (tech == HYSET_TECH_DIRECT ? TECH_DIRECT : TECH_BITMAP);
     if (token_major) {

@@ -257,6 +257,10 @@ struct JoinParams {
     // prefix slots each, taken one per steal from work[1] before the batches
     uint32_t heavy_from = 0xFFFFFFFFu;
     uint32_t segs = 0, seg_slots = 0;
+    // signature technique: probes from heavy_from on hold more tokens than their
+    // signatures can tell apart (most of their window is verified); the first
+    // candidate any of them can have
+    uint32_t heavy_lo = 0;
 };
 
 enum Technique : int { TECH_BITMAP = 1, TECH_FGSS = 2, TECH_DIRECT = 3 };

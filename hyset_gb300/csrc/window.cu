@@ -115,38 +115,49 @@ __device__ __forceinline__ void verify_queued(const JoinParams& P, const uint2* 
     }
 }
 
-// Units (tile of tile_probes probes) x (segment of seg candidates of its
-// window) are taken one per steal, the longest sets first; a unit past the end
-// of its tile's window is empty.
+// How probes [p_lo, p_hi) and their windows are cut into units.
+struct WinCut {
+    uint32_t tile, seg, segs;  // probes and candidates per unit, units per tile of probes
+};
+
+// Units (tile of probes) x (segment of its window's candidates) are taken one
+// per steal, the longest sets first; a unit past the end of its tile's window
+// is empty.  Probes from heavy_from on are cut finer: their signatures are
+// full, so most pairs are verified, a merge of long sets each, and a unit of
+// 64 x 8,192 of them outlasted the rest of the launch (SMs active 47 % of
+// it at 64 bits and 200,000 short sets).
 template <int VMODE, int W>
-__global__ void __launch_bounds__(WIN_THREADS, 4) k_window(JoinParams P, uint32_t tile_probes, uint32_t seg,
-                                                           uint32_t segs) {
+__global__ void __launch_bounds__(WIN_THREADS, 4) k_window(JoinParams P, WinCut heavy, WinCut rest) {
     constexpr int NW = 2 * W, NC = win_cands<W>();
     static_assert(WIN_GROUP * NC <= 32, "a group's outcomes fill one mask");
     __shared__ __align__(16) WinSmem<W> sm;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint2* queue = sm.queue[warp];
     uint32_t qn = 0;  // queued pairs (warp-uniform)
-    const uint32_t nprobe = P.p_hi - P.p_lo;
-    const uint64_t units = (uint64_t)((nprobe + tile_probes - 1) / tile_probes) * segs;
+    const uint32_t split = max(P.p_lo, min(P.p_hi, P.heavy_from));  // probes [split, p_hi) are the heavy ones
+    const uint32_t units_heavy = (P.p_hi - split + heavy.tile - 1) / heavy.tile * heavy.segs;
+    const uint32_t units = units_heavy + (split - P.p_lo + rest.tile - 1) / rest.tile * rest.segs;
     const uint32_t* __restrict__ sig_R = reinterpret_cast<const uint32_t*>(P.bits_R);
     const uint32_t* __restrict__ sig_S = reinterpret_cast<const uint32_t*>(P.bits_S);
     for (;;) {
         __syncthreads();  // the previous unit's tile is no longer read
         if (threadIdx.x == 0) sm.unit = atomicAdd(P.work, 1u);
         __syncthreads();
-        const uint32_t u = sm.unit;
+        uint32_t u = sm.unit;
         if (u >= units) break;
-        const uint32_t tile = u / segs, s = u - tile * segs;
-        const uint32_t p_end = P.p_hi - tile * tile_probes;
-        const uint32_t np = min(tile_probes, p_end - P.p_lo), p0 = p_end - np;
+        const bool hv = u < units_heavy;
+        if (!hv) u -= units_heavy;
+        const WinCut cut = hv ? heavy : rest;
+        const uint32_t tile = u / cut.segs, s = u - tile * cut.segs;
+        const uint32_t p_end = (hv ? P.p_hi : split) - tile * cut.tile;
+        const uint32_t np = min(cut.tile, p_end - (hv ? split : P.p_lo)), p0 = p_end - np;
         const uint32_t lmin = P.S.meta[p0].y, lmax = P.S.meta[p_end - 1].y;
         // the union of the tile's windows (minsize and max_partner grow with the size)
         const uint32_t lo = max(P.first_ge[min(P.B.minsize[lmin], P.R_L + 1)], P.r_lo);
         const uint32_t hi = min(P.self ? p_end - 1 : P.first_ge[min(P.B.max_partner[lmax] + 1, P.R_L + 1)], P.r_hi);
-        const uint64_t a64 = (uint64_t)(lo & ~31u) + (uint64_t)s * seg;
+        const uint64_t a64 = (uint64_t)(lo & ~31u) + (uint64_t)s * cut.seg;
         if (a64 >= hi) continue;
-        const uint32_t a = (uint32_t)a64, b = (uint32_t)min((uint64_t)hi, a64 + seg);
+        const uint32_t a = (uint32_t)a64, b = (uint32_t)min((uint64_t)hi, a64 + cut.seg);
         for (uint32_t i = threadIdx.x; i < WIN_TILE * NW; i += WIN_THREADS)
             sm.sig[0][i] = i < np * NW ? sig_S[(uint64_t)p0 * NW + i] : 0u;
         for (uint32_t i = threadIdx.x; i < WIN_TILE; i += WIN_THREADS) sm.len[i] = P.S.meta[p0 + min(i, np - 1)].y;
@@ -254,15 +265,25 @@ cudaError_t launch_window_w(const JoinParams& P, int sm_count, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     const uint32_t blocks = (uint32_t)(sm_count * std::max(per_sm, 1));
     // units small enough that the blocks have several each, down to 16 probes x 1,024 candidates
-    const uint64_t nprobe = P.p_hi - P.p_lo, ncand = P.r_hi > P.r_lo ? P.r_hi - P.r_lo : 1;
-    uint32_t tile = WIN_TILE, seg = 8192;
-    auto units = [&] { return (nprobe + tile - 1) / tile * ((ncand + 31 + seg - 1) / seg); };
-    while (units() < 8ull * blocks && seg > 1024) seg /= 2;
-    while (units() < 8ull * blocks && tile > 16) tile /= 2;
-    while (units() > 0xFFFF0000ull) seg *= 2;  // the steal counter has 32 bits
-    const uint32_t segs = (uint32_t)((ncand + 31 + seg - 1) / seg);  // a window starts up to 31 ids early
+    const uint64_t ncand = P.r_hi > P.r_lo ? P.r_hi - P.r_lo : 1;
+    const uint32_t split = std::max(P.p_lo, std::min(P.p_hi, P.heavy_from));
+    auto segments = [](uint64_t cands, uint32_t seg) { return (cands + 31 + seg - 1) / seg; };  // a window starts up to 31 ids early
+    auto units = [&](uint64_t probes, uint64_t cands, uint32_t tile, uint32_t seg) {
+        return (probes + tile - 1) / tile * segments(cands, seg);
+    };
+    // small enough that the blocks have several each, down to 16 probes x 1,024 candidates
+    WinCut rest{WIN_TILE, 8192, 0}, heavy{8, 1024, 0};
+    const uint64_t np = split - P.p_lo, nh = P.p_hi - split;
+    const uint64_t hcand = P.r_hi > std::max(P.r_lo, P.heavy_lo) ? P.r_hi - std::max(P.r_lo, P.heavy_lo) : 1;
+    while (units(np, ncand, rest.tile, rest.seg) < 8ull * blocks && rest.seg > 1024) rest.seg /= 2;
+    while (units(np, ncand, rest.tile, rest.seg) < 8ull * blocks && rest.tile > 16) rest.tile /= 2;
+    while (units(np, ncand, rest.tile, rest.seg) > 0x7FFF0000ull) rest.seg *= 2;  // the steal counter has 32 bits
+    while (units(nh, hcand, heavy.tile, heavy.seg) > 0x7FFF0000ull) heavy.seg *= 2;
+    rest.segs = (uint32_t)segments(ncand, rest.seg);
+    heavy.segs = (uint32_t)segments(hcand, heavy.seg);
+    const uint64_t all = units(np, ncand, rest.tile, rest.seg) + units(nh, hcand, heavy.tile, heavy.seg);
     note_launches();
-    k_window<VMODE, W><<<(unsigned)std::min<uint64_t>(blocks, units()), WIN_THREADS, 0, s>>>(P, tile, seg, segs);
+    k_window<VMODE, W><<<(unsigned)std::min<uint64_t>(blocks, all), WIN_THREADS, 0, s>>>(P, heavy, rest);
     return cudaGetLastError();
 }
 
