@@ -66,6 +66,7 @@ void size_meta_from_first_ge(hyset_coll* c, const uint32_t* first_ge, uint32_t L
 uint32_t size_at(const hyset_coll* c, uint32_t i);
 std::vector<uint64_t> range_hist(const hyset_coll* c, uint32_t lo, uint32_t hi);
 uint64_t prefix_entries(const hyset_coll* c, const std::vector<uint32_t>& pre);
+uint64_t prefix_entries_of(const std::vector<uint64_t>& hist, const std::vector<uint32_t>& pre);
 uint32_t bits_for(uint64_t v);
 // The entry layout of an index's token records: the low rec_bits hold the
 // longest probe the entry's positional bound admits (*bound: a self-join's
@@ -82,7 +83,8 @@ uint32_t first_long_prefix(const hyset_coll* c, const std::vector<uint32_t>& pre
 int key_bits_for(uint32_t universe);
 hyset_status build_sorted_index(hyset_ctx* ctx, hyset_coll* c, const Bounds* b, int kind, Index& ix,
                                 const std::vector<uint32_t>* pre = nullptr, const uint32_t* d_pre = nullptr,
-                                int force_pb = -1, bool records_ok = false);
+                                int force_pb = -1, bool records_ok = false, uint32_t lo = 0,
+                                uint32_t hi = 0xFFFFFFFFu);
 bool use_bands(const Bounds* b, bool self);
 hyset_status build_fgss_indexes(hyset_ctx* ctx, hyset_coll* R, const Bounds* b, bool self, Index& ix, Index& ix_mid,
                                 JoinParams& P);

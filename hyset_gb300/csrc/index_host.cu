@@ -76,6 +76,12 @@ uint64_t prefix_entries(const hyset_coll* c, const std::vector<uint32_t>& pre) {
     return E;
 }
 
+uint64_t prefix_entries_of(const std::vector<uint64_t>& hist, const std::vector<uint32_t>& pre) {
+    uint64_t E = 0;
+    for (size_t l = 0; l < hist.size(); ++l) E += hist[l] * (uint64_t)pre[l];
+    return E;
+}
+
 BoundFields bound_fields(const Bounds* b) {
     return BoundFields{b->view.max_sum, b->view.lp_row, b->view.lp_tab};
 }
@@ -123,9 +129,10 @@ int key_bits_for(uint32_t universe) {
 // read back on the collection's first build with the table; that build's
 // lists are converted), afterwards directly from the prefix entries: one emit
 // pass and one ordering pass, no offsets, no scan.
+// [lo, hi): only these sets are indexed (set ids stay absolute).
 hyset_status build_sorted_index(hyset_ctx* ctx, hyset_coll* c, const Bounds* b, int kind, Index& ix,
                                 const std::vector<uint32_t>* pre, const uint32_t* d_pre,
-                                int force_pb, bool records_ok) {
+                                int force_pb, bool records_ok, uint32_t lo, uint32_t hi) {
     // Rebuilt on every join (buffers are reused): a join's timed device work
     // always includes its own index build.  Only asynchronous stream work once
     // the buffers are large enough, so a batch can capture it into a graph.
@@ -135,7 +142,9 @@ hyset_status build_sorted_index(hyset_ctx* ctx, hyset_coll* c, const Bounds* b, 
     }
     cudaStream_t s = ctx->stream;
     const uint32_t n = c->n, U = c->universe;
-    const uint64_t E = prefix_entries(c, *pre);
+    hi = std::min(hi, n);
+    const bool whole = lo == 0 && hi == n;
+    const uint64_t E = whole ? prefix_entries(c, *pre) : prefix_entries_of(range_hist(c, lo, hi), *pre);
     if (E >= (1ull << 32)) return fail(ctx, HYSET_E_UNSUPPORTED, "more than 2^32 prefix entries");
     const uint64_t E1 = E ? E : 1;
     CK(ctx->sc->len.ensure((size_t)n * 4 + 4, s));
@@ -182,7 +191,7 @@ hyset_status build_sorted_index(hyset_ctx* ctx, hyset_coll* c, const Bounds* b, 
             record_layout(c, b, kind, pb, &ix.rec_bits, &ix.rec_bound);
             CK(ix.rec.ensure((size_t)U * REC_CAP * 4, s));
             CK(cudaMemsetAsync(counts, 0, (size_t)U * 4, s));
-            CK(emit_records(v, d_pre, ix.rec_bits, counts, ix.rec.as<uint32_t>(), U, s, 0, 0xFFFFFFFFu,
+            CK(emit_records(v, d_pre, ix.rec_bits, counts, ix.rec.as<uint32_t>(), U, s, lo, hi,
                             ix.rec_bound ? bound_fields(b) : BoundFields{}, first_long_prefix(c, *pre)));
             CK(order_records(counts, U, ix.rec.as<uint32_t>(), s));
             ix.records = true;
@@ -190,24 +199,28 @@ hyset_status build_sorted_index(hyset_ctx* ctx, hyset_coll* c, const Bounds* b, 
             return HYSET_OK;
         }
     }
-    CK(set_prefix_lengths(v, d_pre, 0, n, len, s));
-    CK(scan_exclusive(len, off, n, scr, s));
+    CK(set_prefix_lengths(v, d_pre, lo, hi, len + lo, s));  // len and off by absolute set id
+    CK(scan_exclusive(len + lo, off + lo, hi - lo, scr, s));
     if (packed) {
         uint32_t* counts = ctx->sc->counts.as<uint32_t>();
         CK(ctx->sc->gate.ensure(4, s));
         CK(cudaMemsetAsync(counts, 0, ((size_t)U + 1) * 4, s));
-        CK(emit_packed_entries(v, off, len, pb, ctx->sc->tok.as<uint32_t>(), ix.set.as<uint32_t>(), counts, s, 0,
-                               0xFFFFFFFFu, 0xFFFFFFFFu, first_long_prefix(c, *pre)));
+        CK(emit_packed_entries(v, off, len, pb, ctx->sc->tok.as<uint32_t>(), ix.set.as<uint32_t>(), counts, s, lo,
+                               hi, 0xFFFFFFFFu, first_long_prefix(c, *pre)));
         // the list build's path is read back once per collection and prefix
         // table (not while a batch is being captured into a graph)
         cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
         CK(cudaStreamIsCapturing(s, &capturing));
-        int& path = c->list_path[d_pre];
+        // (a part of the collection has no longer lists than the whole, but says
+        // nothing about it: its own path is not remembered)
+        const auto known = c->list_path.find(d_pre);
+        int part_path = known == c->list_path.end() ? 0 : known->second;
+        int& path = whole ? c->list_path[d_pre] : part_path;
         const bool read_back = path == 0 && capturing == cudaStreamCaptureStatusNone;
         CK(index_lists(ctx->sc->tok.as<uint32_t>(), ix.set.as<uint32_t>(), E, U, counts, ix.list_off.as<uint32_t>(),
                        ctx->sc->altk.as<uint32_t>(), ctx->sc->altv.as<uint32_t>(), ctx->sc->gate.as<uint32_t>(),
                        key_bits_for(U), scr, s, &path, read_back ? ctx->h_flags + 15 : nullptr));
-        if (read_back && E) c->list_longest[d_pre] = ctx->h_flags[15];
+        if (read_back && E && whole) c->list_longest[d_pre] = ctx->h_flags[15];
         ix.pos_bits = pb;
         if (rec_fits && E && read_back && ctx->h_flags[15] <= REC_ENTRIES) {
             // this build's lists become records; later builds emit records directly
@@ -219,7 +232,7 @@ hyset_status build_sorted_index(hyset_ctx* ctx, hyset_coll* c, const Bounds* b, 
         }
         return HYSET_OK;
     }
-    CK(emit_prefix_entries(v, 0, n, off, len, ctx->sc->tok.as<uint32_t>(), ctx->sc->set.as<uint32_t>(),
+    CK(emit_prefix_entries(v, lo, hi, off + lo, len + lo, ctx->sc->tok.as<uint32_t>(), ctx->sc->set.as<uint32_t>(),
                            ctx->sc->pos.as<uint32_t>(), s));
     uint32_t* counts = ctx->sc->counts.as<uint32_t>();
     CK(cudaMemsetAsync(counts, 0, ((size_t)U + 1) * 4, s));

@@ -258,6 +258,7 @@ struct hyset_handler {
     // per-indexed-block inverted index (reference layout: unsorted lists)
     hs::DevBuf counts, list_off, e_len, e_off, e_tok, e_set, e_pos, idx_set, idx_pos, scan;
     uint32_t indexed_block = 0xFFFFFFFFu;
+    hs::Index part;  // the index of an indexed partition joined as a whole
     hs::DevBuf bits, pairs, count, work;
     uint64_t cap = 0;
     uint64_t out_count = 0;
