@@ -32,7 +32,7 @@ void release_plan(hyset_ctx* ctx, BatchPlan& bp) {
     if (bp.graph) cudaGraphDestroy(bp.graph);
     for (auto& bj : bp.joins) {
         DevBuf* bufs[] = {&bj->ix.list_off, &bj->ix.set, &bj->ix.pos, &bj->ix_mid.list_off, &bj->ix_mid.set,
-                          &bj->ix_mid.pos, &bj->bits_r, &bj->bits_s, &bj->pairs};
+                          &bj->ix_mid.pos, &bj->ix.rec, &bj->ix_mid.rec, &bj->bits_r, &bj->bits_s, &bj->pairs};
         for (DevBuf* d : bufs) d->release(s);
     }
     DevBuf* bufs[] = {&bp.desc, &bp.unit_off, &bp.counts, &bp.work, &bp.sorts};

@@ -124,7 +124,7 @@ int key_bits_for(uint32_t universe) {
 // pre / d_pre: the prefix length table (default: the bounds' index prefix);
 // force_pb >= 0 fixes the layout (0 = unpacked, > 0 = packed with that many
 // position bits) so that two indexes of one join share it.
-// records_ok: the caller's kernel reads token records (REC_CAP); they are
+// records_ok: the caller's kernel reads token records (record_shift); they are
 // built once the longest list of this prefix table is known to fit (it is
 // read back on the collection's first build with the table; that build's
 // lists are converted), afterwards directly from the prefix entries: one emit
@@ -177,24 +177,25 @@ hyset_status build_sorted_index(hyset_ctx* ctx, hyset_coll* c, const Bounds* b, 
     // collections whose tokens the library owns (immutable once uploaded) use
     // them; a collection over caller memory can change between joins.
     const bool owned = c->tokens.p != nullptr && c->d_tokens == c->tokens.as<uint32_t>();
-    const bool rec_fits = records_ok && packed && owned && (uint64_t)U <= REC_MAX_TOKENS;
+    const bool rec_fits = records_ok && packed && owned;
     ix.sim = b->sim;
     ix.tau = b->tau;
     ix.kind = kind;
     ix.universe = U;
     ix.entries = E;
-    ix.records = false;
+    ix.records = 0;
     if (rec_fits) {
         const auto lk = c->list_longest.find(d_pre);
-        if (lk != c->list_longest.end() && lk->second <= REC_ENTRIES) {
+        const int shift = lk != c->list_longest.end() ? record_shift(lk->second, U) : 0;
+        if (shift) {
             uint32_t* counts = ctx->sc->counts.as<uint32_t>();
             record_layout(c, b, kind, pb, &ix.rec_bits, &ix.rec_bound);
-            CK(ix.rec.ensure((size_t)U * REC_CAP * 4, s));
+            CK(ix.rec.ensure(((size_t)U << shift) * 4, s));
             CK(cudaMemsetAsync(counts, 0, (size_t)U * 4, s));
-            CK(emit_records(v, d_pre, ix.rec_bits, counts, ix.rec.as<uint32_t>(), U, s, lo, hi,
+            CK(emit_records(v, d_pre, ix.rec_bits, counts, ix.rec.as<uint32_t>(), shift, U, s, lo, hi,
                             ix.rec_bound ? bound_fields(b) : BoundFields{}, first_long_prefix(c, *pre)));
-            CK(order_records(counts, U, ix.rec.as<uint32_t>(), s));
-            ix.records = true;
+            CK(order_records(counts, U, ix.rec.as<uint32_t>(), shift, s));
+            ix.records = shift;
             ix.pos_bits = pb;
             return HYSET_OK;
         }
@@ -222,13 +223,14 @@ hyset_status build_sorted_index(hyset_ctx* ctx, hyset_coll* c, const Bounds* b, 
                        key_bits_for(U), scr, s, &path, read_back ? ctx->h_flags + 15 : nullptr));
         if (read_back && E && whole) c->list_longest[d_pre] = ctx->h_flags[15];
         ix.pos_bits = pb;
-        if (rec_fits && E && read_back && ctx->h_flags[15] <= REC_ENTRIES) {
+        const int shift = rec_fits && E && read_back ? record_shift(ctx->h_flags[15], U) : 0;
+        if (shift) {
             // this build's lists become records; later builds emit records directly
             record_layout(c, b, kind, pb, &ix.rec_bits, &ix.rec_bound);
-            CK(ix.rec.ensure((size_t)U * REC_CAP * 4, s));
-            CK(records_from_lists(ix.list_off.as<uint32_t>(), ix.set.as<uint32_t>(), U, ix.rec.as<uint32_t>(), s,
+            CK(ix.rec.ensure(((size_t)U << shift) * 4, s));
+            CK(records_from_lists(ix.list_off.as<uint32_t>(), ix.set.as<uint32_t>(), U, ix.rec.as<uint32_t>(), shift, s,
                                   ix.rec_bound ? bound_fields(b) : BoundFields{}, c->d_sizes, pb, ix.rec_bits));
-            ix.records = true;
+            ix.records = shift;
         }
         return HYSET_OK;
     }

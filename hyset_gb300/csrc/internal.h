@@ -85,8 +85,8 @@ struct Index {
     double tau = -1;
     int kind = -1;
     DevBuf list_off, set, pos;
-    DevBuf rec;             // token records (REC_CAP words per token) when records is set
-    bool records = false;
+    DevBuf rec;             // token records (2^records words per token) when records is set
+    int records = 0;        // their shift (see record_shift); 0: lists
     uint32_t universe = 0;
     uint64_t entries = 0;
     uint32_t pos_bits = 0;  // > 0: packed (set << pos_bits) | position entries
@@ -102,7 +102,7 @@ struct Index {
         v.universe = universe;
         v.pos_bits = records ? rec_bits : pos_bits;
         v.sorted = 1;
-        v.rec = records ? 1 : 0;
+        v.rec = records;
         v.bound = records && rec_bound ? 1 : 0;
         return v;
     }

@@ -162,13 +162,13 @@ __device__ __forceinline__ void ldg256(const uint32_t* p, uint32_t (&w)[8]) {
 
 // Window [klo, khi) of a token record (length word, then ascending entries
 // padded with 0xFFFFFFFF; 128-byte aligned): the entries below each bound,
-// counted over 32-byte pieces of the one line, the first piece giving the
-// length and the others read only as far as it reaches (no search).
+// counted over 32-byte pieces, the first piece giving the length and the
+// others read only as far as it reaches (no search).
 __device__ __forceinline__ void record_window(const uint32_t* __restrict__ r, uint32_t klo, uint32_t khi,
                                               uint32_t& nlo, uint32_t& nhi) {
     uint32_t w[8];
     ldg256(r, w);
-    const uint32_t len = w[0];
+    const uint32_t len = min(w[0], record_entries(6));
     nlo = 0;
     nhi = 0;
 #pragma unroll
@@ -185,6 +185,15 @@ __device__ __forceinline__ void record_window(const uint32_t* __restrict__ r, ui
                 nlo += w[q] < klo;
                 nhi += w[q] < khi;
             }
+        }
+    }
+#pragma unroll 1
+    for (uint32_t k = 4; len > 8u * k - 1u; ++k) {  // the second line of a wide record
+        ldg256(r + 8 * k, w);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            nlo += w[q] < klo;
+            nhi += w[q] < khi;
         }
     }
 }
@@ -254,12 +263,12 @@ __device__ void fgss_batch(const JoinParams& P, uint32_t i0, uint32_t k, int lan
         uint32_t first = 0, cnt = 0;
         if (sv) {
             const uint32_t tok = __ldg(P.S.tokens + t_pst + j);
-            if (RC && tok < P.X.universe && (t_band ? P.X2.rec : P.X.rec)) {
-                static_assert(REC_CAP == 32, "record_window reads four 32-byte pieces");
+            const int rec = t_band ? P.X2.rec : P.X.rec;
+            if (RC && tok < P.X.universe && rec) {
                 const uint32_t klo = t_lo << P.X.pos_bits, khi = t_hi << P.X.pos_bits;
                 uint32_t nlo, nhi;
-                record_window(x_set + ((uint64_t)tok << 5), klo, khi, nlo, nhi);
-                first = (tok << 5) + 1 + nlo;
+                record_window(x_set + ((uint64_t)tok << rec), klo, khi, nlo, nhi);
+                first = (tok << rec) + 1 + nlo;
                 cnt = nhi - nlo;
             } else if (tok < P.X.universe) {
                 uint32_t b0 = x_off[tok], b1 = x_off[tok + 1];
@@ -529,11 +538,12 @@ __device__ void fgss_carry(const JoinParams& P, uint32_t i0, uint32_t k, int lan
         uint32_t first = 0, cnt = 0;
         if (sv) {
             const uint32_t tok = __ldg(P.S.tokens + t_pst + j);
-            if (tok < P.X.universe && (t_band ? P.X2.rec : P.X.rec)) {
+            const int rec = t_band ? P.X2.rec : P.X.rec;
+            if (tok < P.X.universe && rec) {
                 const uint32_t klo = t_lo << P.X.pos_bits, khi = t_hi << P.X.pos_bits;
                 uint32_t nlo, nhi;
-                record_window(x_set + ((uint64_t)tok << 5), klo, khi, nlo, nhi);
-                first = (tok << 5) + 1 + nlo;
+                record_window(x_set + ((uint64_t)tok << rec), klo, khi, nlo, nhi);
+                first = (tok << rec) + 1 + nlo;
                 cnt = nhi - nlo;
             } else if (tok < P.X.universe) {
                 uint32_t b0 = x_off[tok], b1 = x_off[tok + 1];

@@ -110,15 +110,22 @@ cudaError_t emit_packed_entries(CollView c, const uint32_t* entry_off, const uin
                                 uint32_t lo = 0, uint32_t hi = 0xFFFFFFFFu, uint32_t limit = 0xFFFFFFFFu,
                                 uint32_t big_lo = 0xFFFFFFFFu);
 
-// Token records: when no list holds more than REC_ENTRIES entries, list t is
-// the fixed REC_CAP-word record rec[REC_CAP t, REC_CAP t + REC_CAP): word 0
-// the list's length, then its entries ascending and the rest 0xFFFFFFFF
-// (never a valid packed entry).  A probe finds its window in one 128-byte
+// Token records: when no list holds more than 31 (63) entries, list t is the
+// fixed record rec[2^shift t, 2^shift (t + 1)) of 32 (64) words, shift 5 (6):
+// word 0 the list's length, then its entries ascending and the rest
+// 0xFFFFFFFF (never a valid packed entry).  The wide record costs no more
+// traffic than the narrow one: only the 32-byte pieces that hold entries are
+// read or written.  A probe finds its window in one 128-byte
 // line (32-byte loads, only as many as the length needs) and the build needs
 // no offsets: no scan, no scatter pass.
-constexpr uint32_t REC_CAP = 32;
-constexpr uint32_t REC_ENTRIES = REC_CAP - 1;
-constexpr uint64_t REC_MAX_TOKENS = 1ull << 25;  // records of larger universes would pass 4 GB
+constexpr uint64_t REC_MAX_WORDS = 1ull << 30;  // records of larger universes would pass 4 GB
+__host__ __device__ constexpr uint32_t record_entries(int shift) { return (1u << shift) - 1u; }
+// The shift of the records that hold lists of up to `longest` entries over U
+// tokens; 0: lists.
+constexpr int record_shift(uint32_t longest, uint64_t U) {
+    const int shift = longest <= record_entries(5) ? 5 : longest <= record_entries(6) ? 6 : 0;
+    return shift && (U << shift) <= REC_MAX_WORDS ? shift : 0;
+}
 // Record build, pass 1: the first prefix_tab[size] tokens of every set of c
 // become entries (set << pos_bits) | position, each taking slot
 // atomicAdd(&counts[token], 1) of its token's record (tokens below `limit`;
@@ -126,9 +133,9 @@ constexpr uint64_t REC_MAX_TOKENS = 1ull << 25;  // records of larger universes 
 // bf (optional, a self-join's midprefix index): the low pos_bits of each entry
 // hold its bound field (bound_field_of) instead of the position.
 cudaError_t emit_records(CollView c, const uint32_t* prefix_tab, uint32_t pos_bits, uint32_t* counts, uint32_t* rec,
-                         uint32_t limit, cudaStream_t s, uint32_t lo = 0, uint32_t hi = 0xFFFFFFFFu,
+                         int shift, uint32_t limit, cudaStream_t s, uint32_t lo = 0, uint32_t hi = 0xFFFFFFFFu,
                          BoundFields bf = BoundFields{}, uint32_t big_lo = 0xFFFFFFFFu);
-// Pass 2: each record's min(counts[t], REC_ENTRIES) entries in ascending
+// Pass 2: each record's min(counts[t], record_entries(shift)) entries in ascending
 // order after its length word, padded with 0xFFFFFFFF.  overflow (optional):
 // OR-ed with REC_OVERFLOW when a token had more entries than a record holds
 // (its record is then incomplete and the index must be built as lists).
@@ -140,13 +147,13 @@ cudaError_t emit_records(CollView c, const uint32_t* prefix_tab, uint32_t pos_bi
 // words and the length: a join reading sets below the earlier pass's bound
 // may run beside it.
 constexpr uint32_t REC_OVERFLOW = 16;
-cudaError_t order_records(const uint32_t* counts, uint32_t U, uint32_t* rec, cudaStream_t s,
+cudaError_t order_records(const uint32_t* counts, uint32_t U, uint32_t* rec, int shift, cudaStream_t s,
                           uint32_t* overflow = nullptr, uint32_t* prev = nullptr);
-// Records from index lists already built (every list at most REC_ENTRIES long).
+// Records from index lists already built (every list at most record_entries(shift) long).
 // bf (optional): entries (set << list_bits) | position become
 // (set << rec_bits) | bound field (sizes: the indexed sets' sizes).
 cudaError_t records_from_lists(const uint32_t* list_off, const uint32_t* vals, uint32_t U, uint32_t* rec,
-                               cudaStream_t s, BoundFields bf = BoundFields{}, const uint32_t* sizes = nullptr,
+                               int shift, cudaStream_t s, BoundFields bf = BoundFields{}, const uint32_t* sizes = nullptr,
                                uint32_t list_bits = 0, uint32_t rec_bits = 0);
 
 // Token histogram of n entries into counts[limit] (warp-aggregated atomics;
@@ -228,7 +235,7 @@ struct IndexView {
     uint32_t universe;
     uint32_t pos_bits;                      // packed layout: bits of the position field
     int sorted;                             // lists ordered by set id
-    int rec = 0;                            // token records: list t = set[REC_CAP t, REC_CAP (t + 1)) (see REC_CAP)
+    int rec = 0;                            // token records: list t = set[2^rec t, 2^rec (t + 1)) (see record_shift); 0: lists
     // packed entries carry, in place of the position, the longest probe the
     // entry's side of the positional bound admits (see bound_field)
     int bound = 0;

@@ -401,10 +401,9 @@ hyset_status hyset_self_join_host(hyset_ctx* ctx, const uint32_t* tokens, uint64
         // (this collection's tokens differ), and the join is then run again
         // over lists.
         auto lit = ctx->longest_cache.find(key);
-        bool records = assumed && lit != ctx->longest_cache.end() && lit->second <= REC_ENTRIES &&
-                       (uint64_t)U <= REC_MAX_TOKENS;
+        const int records = assumed && lit != ctx->longest_cache.end() ? record_shift(lit->second, U) : 0;
         if (records) {
-            CK(ix.rec.ensure((size_t)U * REC_CAP * 4, s));
+            CK(ix.rec.ensure(((size_t)U << records) * 4, s));
             record_layout(C, b, 0, pb, &ix.rec_bits, &ix.rec_bound);
         }
         const uint32_t big_lo = first_long_prefix(C, b->index_prefix);  // emitted a warp per set from here on
@@ -430,7 +429,7 @@ hyset_status hyset_self_join_host(hyset_ctx* ctx, const uint32_t* tokens, uint64
         uint32_t join_launches = 0, join_lo = 0;  // probes [0, join_lo) are joined
         uint64_t joined_to = 0;                    // the tokens that had landed at the last join point
         if (streamed) {
-            ix.records = true;
+            ix.records = records;
             ix.sim = b->sim;
             ix.tau = b->tau;
             ix.kind = 0;
@@ -450,7 +449,7 @@ hyset_status hyset_self_join_host(hyset_ctx* ctx, const uint32_t* tokens, uint64
             // while a later pass orders it sees only entries of its own and
             // earlier chunks in place, padding, or entries of later sets (above
             // every window it counts), never a word left from an earlier call
-            CK(cudaMemsetAsync(ix.rec.p, 0xFF, (size_t)U * REC_CAP * 4, s));
+            CK(cudaMemsetAsync(ix.rec.p, 0xFF, ((size_t)U << records) * 4, s));
             CK(cudaMemsetAsync(ctx->s_count.p, 0, 16, s));
             CK(cudaMemsetAsync(ctx->s_work.p, 0, (2 * n_chunks + 4) * 4, s));
             if (o->collect_stats) CK(cudaMemsetAsync(ctx->s_stats.p, 0, 64, s));
@@ -496,7 +495,7 @@ hyset_status hyset_self_join_host(hyset_ctx* ctx, const uint32_t* tokens, uint64
             else
                 CK(validate_collection(part, n_tokens, ctx->s_flags.as<uint32_t>(), C->meta.as<uint2>() + lo, s));
             if (records)
-                CK(emit_records(v, b->view.index_prefix, ix.rec_bits, counts, ix.rec.as<uint32_t>(), U, s, lo, hi,
+                CK(emit_records(v, b->view.index_prefix, ix.rec_bits, counts, ix.rec.as<uint32_t>(), records, U, s, lo, hi,
                                 ix.rec_bound ? bound_fields(b) : BoundFields{}, big_lo));
             else
                 CK(emit_packed_entries(v, off, len, pb, ctx->sc->tok.as<uint32_t>(), ix.set.as<uint32_t>(), counts, s,
@@ -505,7 +504,7 @@ hyset_status hyset_self_join_host(hyset_ctx* ctx, const uint32_t* tokens, uint64
             // one): order the records, then join the probes not joined yet, all
             // in stream order while the next chunks are copied
             if (join_point) {
-                CK(order_records(counts, U, ix.rec.as<uint32_t>(), s, ctx->s_flags.as<uint32_t>(), prev));
+                CK(order_records(counts, U, ix.rec.as<uint32_t>(), records, s, ctx->s_flags.as<uint32_t>(), prev));
                 if (join_launches == 0) CK(cudaEventRecord(ctx->ek0, s));
                 JoinParams Q = SP;
                 Q.p_lo = join_lo;
@@ -574,7 +573,7 @@ hyset_status hyset_self_join_host(hyset_ctx* ctx, const uint32_t* tokens, uint64
             CK(ctx->sc->scan.ensure(std::max(scan_words, scan_scratch_words((uint64_t)U + 1)) * 4, s));
             const bool rec_now = records && attempt == 0;
             if (rec_now) {
-                CK(order_records(counts, U, ix.rec.as<uint32_t>(), s, ctx->s_flags.as<uint32_t>()));
+                CK(order_records(counts, U, ix.rec.as<uint32_t>(), records, s, ctx->s_flags.as<uint32_t>()));
             } else {
                 ST(prepare_lists());
                 if (attempt > 0 || records)  // the list build reordered the entries (or none were emitted): emit them
@@ -589,7 +588,7 @@ hyset_status hyset_self_join_host(hyset_ctx* ctx, const uint32_t* tokens, uint64
                                ix.list_off.as<uint32_t>(), ctx->sc->altk.as<uint32_t>(), ctx->sc->altv.as<uint32_t>(),
                                ctx->sc->gate.as<uint32_t>(), key_bits_for(U), ctx->sc->scan.as<uint32_t>(), s));
             }
-            ix.records = rec_now;
+            ix.records = rec_now ? records : 0;
             ix.sim = b->sim;
             ix.tau = b->tau;
             ix.kind = 0;

@@ -290,7 +290,7 @@ __global__ void k_emit_entries(CollView c, uint32_t lo, uint32_t hi, const uint3
 // set id.  counts may be nullptr (no histogram).
 // REC: instead of the entry arrays, each entry goes straight into its token's
 // record (the histogram atomic returns its slot; tokens at or above `limit`
-// and slots past REC_ENTRIES are dropped); len is then the prefix-length table
+// and slots past the record's end are dropped); len is then the prefix-length table
 // indexed by set size and off is not read.
 constexpr int EMIT_ROUNDS = 8;
 #ifndef HS_REC_EMIT_ROUNDS
@@ -303,7 +303,7 @@ template <bool REC>
 __global__ void __launch_bounds__(256, REC ? HS_REC_EMIT_MINB : 1) k_emit_packed(CollView c, uint32_t lo, const uint32_t* __restrict__ off,
                               const uint32_t* __restrict__ len, uint32_t pos_bits, uint32_t* __restrict__ e_token,
                               uint32_t* __restrict__ e_val, uint32_t* __restrict__ counts, uint32_t limit,
-                              BoundFields bf, uint32_t spw) {
+                              BoundFields bf, uint32_t spw, int shift) {
     constexpr int ROUNDS = REC ? HS_REC_EMIT_ROUNDS : EMIT_ROUNDS;
     const uint32_t maxf = (1u << pos_bits) - 1u;
     const int lane = threadIdx.x & 31;
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(256, REC ? HS_REC_EMIT_MINB : 1) k_emit_packed
                 }
 #pragma unroll
                 for (int u = 0; u < ROUNDS; ++u)
-                    if (slot[u] < REC_ENTRIES) e_val[(uint64_t)tok[u] * REC_CAP + 1 + slot[u]] = val[u];
+                    if (slot[u] < (1u << shift) - 1u) e_val[((uint64_t)tok[u] << shift) + 1 + slot[u]] = val[u];
                 continue;
             }
 #pragma unroll
@@ -509,19 +509,21 @@ __global__ void __launch_bounds__(RANK_THREADS) k_list_rank(const uint32_t* __re
 }
 
 // Orders the token records: a warp takes 32 consecutive records, stages in
-// shared memory (a record per 33 words, so the lanes' sorts hit distinct
-// banks) the 16-byte quarters that hold its length word and entries, lane k
-// sorts record k by insertion (the atomic slots mostly follow emission order,
-// which is set order), pads it and writes its length word, and the warp
+// shared memory (a record per 2^SHIFT + 1 words, so the lanes' sorts hit
+// distinct banks) the 16-byte quarters that hold its length word and entries,
+// lane k sorts record k by insertion (the atomic slots mostly follow emission
+// order, which is set order), pads it and writes its length word, and the warp
 // stores back every 32-byte piece a probe reads for that length (the piece
 // holding word 0 and as many more as the entries reach; see record_window).
 // Pieces past them are neither read nor written.
-constexpr int REC_THREADS = 256;
+constexpr int rec_threads(int shift) { return shift == 5 ? 256 : 128; }  // 33 KB of stages per block either way
 __host__ __device__ constexpr uint32_t record_pieces(uint32_t n) { return n > 7u ? 1u + (n - 7u + 7u) / 8u : 1u; }
-__global__ void __launch_bounds__(REC_THREADS) k_order_records(const uint32_t* __restrict__ counts, uint32_t U,
+template <int SHIFT>
+__global__ void __launch_bounds__(SHIFT == 5 ? 256 : 128) k_order_records(const uint32_t* __restrict__ counts, uint32_t U,
                                                                uint32_t* __restrict__ rec, uint32_t* overflow,
                                                                uint32_t* __restrict__ prev) {
-    __shared__ uint32_t stage_all[REC_THREADS / 32][32 * 33];
+    constexpr uint32_t CAP = 1u << SHIFT, QUARTERS = CAP / 4, STRIDE = CAP + 1;
+    __shared__ uint32_t stage_all[(SHIFT == 5 ? 256 : 128) / 32][32 * STRIDE];
     const int lane = threadIdx.x & 31;
     uint32_t* stage = stage_all[threadIdx.x >> 5];
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
@@ -534,23 +536,23 @@ __global__ void __launch_bounds__(REC_THREADS) k_order_records(const uint32_t* _
             if (!__any_sync(FULL, changed)) continue;
             if (changed) prev[t0 + lane] = cnt;
         }
-        if (overflow && __any_sync(FULL, cnt > REC_ENTRIES) && lane == 0) atomicOr(overflow, REC_OVERFLOW);
-        const uint32_t mine = min(cnt, REC_ENTRIES);
-        uint4* g = reinterpret_cast<uint4*>(rec + t0 * REC_CAP);
-        // quarter k: record k / 8, words 4 (k % 8) .. +3; read if it holds the length or an entry
+        if (overflow && __any_sync(FULL, cnt >= CAP) && lane == 0) atomicOr(overflow, REC_OVERFLOW);
+        const uint32_t mine = min(cnt, CAP - 1u);
+        uint4* g = reinterpret_cast<uint4*>(rec + (t0 << SHIFT));
+        // quarter k: record k / QUARTERS, words 4 (k % QUARTERS) .. +3; read if it holds the length or an entry
 #pragma unroll
-        for (uint32_t it = 0; it < 8; ++it) {  // every lane takes every round: the shuffles stay converged
-            const uint32_t k = (uint32_t)lane + 32u * it;
-            const uint32_t n = __shfl_sync(FULL, mine, k >> 3);
-            if (k < nrec * 8 && 4 * (k & 7) < n + 1) {
+        for (uint32_t it = 0; it < QUARTERS; ++it) {  // every lane takes every round: the shuffles stay converged
+            const uint32_t k = (uint32_t)lane + 32u * it, r = k / QUARTERS, q = k % QUARTERS;
+            const uint32_t n = __shfl_sync(FULL, mine, r);
+            if (r < nrec && 4 * q < n + 1) {
                 const uint4 x = g[k];
-                uint32_t* d = stage + (k >> 3) * 33 + (k & 7) * 4;
+                uint32_t* d = stage + r * STRIDE + q * 4;
                 d[0] = x.x, d[1] = x.y, d[2] = x.z, d[3] = x.w;
             }
         }
         __syncwarp();
         if ((uint32_t)lane < nrec) {
-            uint32_t* r = stage + lane * 33 + 1;  // the entries follow the length word
+            uint32_t* r = stage + lane * STRIDE + 1;  // the entries follow the length word
             const uint32_t n = mine;
             for (uint32_t i = 1; i < n; ++i) {
                 const uint32_t x = r[i];
@@ -567,11 +569,11 @@ __global__ void __launch_bounds__(REC_THREADS) k_order_records(const uint32_t* _
         }
         __syncwarp();
 #pragma unroll
-        for (uint32_t it = 0; it < 8; ++it) {
-            const uint32_t k = (uint32_t)lane + 32u * it;
-            const uint32_t n = __shfl_sync(FULL, mine, k >> 3);
-            if (k < nrec * 8 && 4 * (k & 7) < 8 * record_pieces(n)) {
-                const uint32_t* d = stage + (k >> 3) * 33 + (k & 7) * 4;
+        for (uint32_t it = 0; it < QUARTERS; ++it) {
+            const uint32_t k = (uint32_t)lane + 32u * it, r = k / QUARTERS, q = k % QUARTERS;
+            const uint32_t n = __shfl_sync(FULL, mine, r);
+            if (r < nrec && 4 * q < 8 * record_pieces(n)) {
+                const uint32_t* d = stage + r * STRIDE + q * 4;
                 g[k] = make_uint4(d[0], d[1], d[2], d[3]);
             }
         }
@@ -579,21 +581,23 @@ __global__ void __launch_bounds__(REC_THREADS) k_order_records(const uint32_t* _
     }
 }
 
-// Records from built lists: a warp per token, lane 0 writes the length, lane
-// i > 0 entry i - 1 or the pad.
+// Records from built lists: a warp per token, the record's word 0 the length,
+// word i > 0 entry i - 1 or the pad.
 __global__ void k_records_from_lists(const uint32_t* __restrict__ list_off, const uint32_t* __restrict__ vals,
-                                     uint32_t U, uint32_t* __restrict__ rec, BoundFields bf,
+                                     uint32_t U, uint32_t* __restrict__ rec, int shift, BoundFields bf,
                                      const uint32_t* __restrict__ sizes, uint32_t list_bits, uint32_t rec_bits) {
-    const int lane = threadIdx.x & 31;
+    const uint32_t lane = threadIdx.x & 31;
     const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     for (uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < U; t += warps) {
         const uint32_t a = list_off[t], b = list_off[t + 1];
-        uint32_t w = lane == 0 ? b - a : (a + lane - 1 < b ? vals[a + lane - 1] : 0xFFFFFFFFu);
-        if (bf.on() && lane > 0 && a + lane - 1 < b) {  // (set, position) -> (set, bound field)
-            const uint32_t set = w >> list_bits, pos = w & ((1u << list_bits) - 1u);
-            w = (set << rec_bits) | bound_field_of(bf, sizes[set], pos, (1u << rec_bits) - 1u);
+        for (uint32_t i = lane; i < 1u << shift; i += 32) {
+            uint32_t w = i == 0 ? b - a : (a + i - 1 < b ? vals[a + i - 1] : 0xFFFFFFFFu);
+            if (bf.on() && i > 0 && a + i - 1 < b) {  // (set, position) -> (set, bound field)
+                const uint32_t set = w >> list_bits, pos = w & ((1u << list_bits) - 1u);
+                w = (set << rec_bits) | bound_field_of(bf, sizes[set], pos, (1u << rec_bits) - 1u);
+            }
+            rec[(t << shift) + i] = w;
         }
-        rec[t * REC_CAP + lane] = w;
     }
 }
 
@@ -993,7 +997,7 @@ namespace {
 template <bool REC>
 cudaError_t launch_emit(CollView c, uint32_t lo, uint32_t hi, uint32_t big_lo, const uint32_t* off,
                         const uint32_t* len, uint32_t pos_bits, uint32_t* e_token, uint32_t* e_val, uint32_t* counts,
-                        uint32_t limit, BoundFields bf, cudaStream_t s) {
+                        uint32_t limit, BoundFields bf, int shift, cudaStream_t s) {
     if (hi == 0xFFFFFFFFu) hi = c.n;
     const uint32_t mid = std::min(std::max(lo, big_lo), hi);
     CollView v = c;
@@ -1001,14 +1005,14 @@ cudaError_t launch_emit(CollView c, uint32_t lo, uint32_t hi, uint32_t big_lo, c
         note_launches();
         v.n = mid;  // the kernel walks ids [lo, mid)
         k_emit_packed<REC><<<grid_for((uint64_t)(mid - lo), 256), 256, 0, s>>>(v, lo, off, len, pos_bits, e_token,
-                                                                             e_val, counts, limit, bf, 32u);
+                                                                             e_val, counts, limit, bf, 32u, shift);
     }
     if (hi > mid) {
         note_launches();
         v.n = hi;
         k_emit_packed<REC><<<grid_for((uint64_t)(hi - mid) * 32u, 256), 256, 0, s>>>(v, mid, off, len, pos_bits,
                                                                                    e_token, e_val, counts, limit,
-                                                                                   bf, 1u);
+                                                                                   bf, 1u, shift);
     }
     return cudaGetLastError();
 }
@@ -1018,30 +1022,33 @@ cudaError_t emit_packed_entries(CollView c, const uint32_t* entry_off, const uin
                                 uint32_t* e_token, uint32_t* e_val, uint32_t* counts, cudaStream_t s, uint32_t lo,
                                 uint32_t hi, uint32_t limit, uint32_t big_lo) {
     return launch_emit<false>(c, lo, hi, big_lo, entry_off, len, pos_bits, e_token, e_val, counts, limit,
-                              BoundFields{}, s);
+                              BoundFields{}, 0, s);
 }
 
 cudaError_t emit_records(CollView c, const uint32_t* prefix_tab, uint32_t pos_bits, uint32_t* counts, uint32_t* rec,
-                         uint32_t limit, cudaStream_t s, uint32_t lo, uint32_t hi, BoundFields bf,
+                         int shift, uint32_t limit, cudaStream_t s, uint32_t lo, uint32_t hi, BoundFields bf,
                          uint32_t big_lo) {
-    return launch_emit<true>(c, lo, hi, big_lo, nullptr, prefix_tab, pos_bits, nullptr, rec, counts, limit, bf, s);
+    return launch_emit<true>(c, lo, hi, big_lo, nullptr, prefix_tab, pos_bits, nullptr, rec, counts, limit, bf, shift, s);
 }
 
-cudaError_t order_records(const uint32_t* counts, uint32_t U, uint32_t* rec, cudaStream_t s, uint32_t* overflow,
-                          uint32_t* prev) {
+cudaError_t order_records(const uint32_t* counts, uint32_t U, uint32_t* rec, int shift, cudaStream_t s,
+                          uint32_t* overflow, uint32_t* prev) {
     if (U == 0) return cudaSuccess;
     note_launches();
-    k_order_records<<<grid_for(((uint64_t)U + 31) / 32 * 32, REC_THREADS), REC_THREADS, 0, s>>>(counts, U, rec,
-                                                                                              overflow, prev);
+    const uint64_t lanes = ((uint64_t)U + 31) / 32 * 32;
+    if (shift == 5)
+        k_order_records<5><<<grid_for(lanes, rec_threads(5)), rec_threads(5), 0, s>>>(counts, U, rec, overflow, prev);
+    else
+        k_order_records<6><<<grid_for(lanes, rec_threads(6)), rec_threads(6), 0, s>>>(counts, U, rec, overflow, prev);
     return cudaGetLastError();
 }
 
 cudaError_t records_from_lists(const uint32_t* list_off, const uint32_t* vals, uint32_t U, uint32_t* rec,
-                               cudaStream_t s, BoundFields bf, const uint32_t* sizes, uint32_t list_bits,
+                               int shift, cudaStream_t s, BoundFields bf, const uint32_t* sizes, uint32_t list_bits,
                                uint32_t rec_bits) {
     if (U == 0) return cudaSuccess;
     note_launches();
-    k_records_from_lists<<<grid_for((uint64_t)U * 32, 256), 256, 0, s>>>(list_off, vals, U, rec, bf, sizes,
+    k_records_from_lists<<<grid_for((uint64_t)U * 32, 256), 256, 0, s>>>(list_off, vals, U, rec, shift, bf, sizes,
                                                                          list_bits, rec_bits);
     return cudaGetLastError();
 }
