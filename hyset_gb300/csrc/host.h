@@ -129,7 +129,7 @@ bool swap_sides(const hyset_coll* R, const hyset_coll* S, const hyset_join_opts*
 hyset_status run_join(hyset_ctx* ctx, JoinParams P, int tech, int vmode, const hyset_join_opts* o, hyset_result* res,
                       bool timed_from_ev0, TokenJoinParams* T = nullptr);
 // The probe-major prefix filter's split of the longest probes of S into slot
-// segments (JoinParams::heavy_from, segs, seg_slots); none for banded joins.
+// segments (JoinParams::heavy_from, segs, seg_slots).
 // The launch's work buffer then needs two zeroed counters.
 void split_heavy(const hyset_coll* S, const Bounds* b, JoinParams& P);
 // Behind a join's launch, before the host knows its number of pairs: orders

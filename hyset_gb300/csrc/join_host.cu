@@ -94,13 +94,18 @@ hyset_status run_join(hyset_ctx* ctx, JoinParams P, int tech, int vmode, const h
     return deliver_pairs(ctx, P, o, res);
 }
 
+// A probe of a long prefix is one warp's work: unsplit, the longest probes of
+// the 61,003 x 147,001 dice join at 0.75 (1,400 slots in two bands) held the
+// launch for twice its other warps' time (kernel 0.79 ms at its best batch of
+// one probe, 1.04 at three; 0.47 split).  Above 64 / 96 / 128 slots, a call of
+// that join: 0.865 / 0.789 / 0.776 ms; units of 32 / 64 / 128 slots 0.809 /
+// 0.776 / 0.801.
 void split_heavy(const hyset_coll* S, const Bounds* b, JoinParams& P) {
     constexpr uint32_t HEAVY_SLOTS = 128;  // probes with longer prefixes are split
     constexpr uint32_t SEG_SLOTS = 64;     // prefix slots per unit of a split probe
     P.heavy_from = 0xFFFFFFFFu;
     P.segs = 0;
     P.seg_slots = SEG_SLOTS;
-    if (P.X2.set) return;  // banded R-S joins keep two lanes per probe
     const uint32_t L = std::min(S->max_size, b->L);
     for (uint32_t l = 0; l <= L; ++l)
         if (b->probe_prefix[l] > HEAVY_SLOTS) {

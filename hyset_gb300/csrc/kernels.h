@@ -261,7 +261,8 @@ struct JoinParams {
     unsigned long long* stats;  // optional [8] counters (nullptr = off)
     // probe-major prefix filter: probes from heavy_from on (the longest
     // prefixes; 0xFFFFFFFF = none) are split into `segs` units of seg_slots
-    // prefix slots each, taken one per steal from work[1] before the batches
+    // prefix slots each (of both bands, in a banded R-S join), taken one per
+    // steal from work[1] before the batches
     uint32_t heavy_from = 0xFFFFFFFFu;
     uint32_t segs = 0, seg_slots = 0;
     // signature technique: probes from heavy_from on hold more tokens than their

@@ -60,3 +60,25 @@ def test_host_join_whose_lists_grow(ctx, before, after):
         exp = oracle.as_set(oracle.join(c.tokens, c.starts, c.sizes, 0.8))
         r = ctx.self_join_host(c.tokens, c.sizes, c.starts, threshold=0.8, sort_pairs=True, **PIPELINED)
         assert r.count == len(exp) and oracle.as_set(r.pairs) == exp, k
+
+
+@pytest.mark.parametrize("sim", ["jaccard", "cosine", "dice"])
+def test_split_probes_of_banded_joins(ctx, sim):
+    """Probes of more than 128 prefix slots go in units of 64 slots of both bands."""
+    c = synth.generate(synth.C3, n_sets=1500, universe=12000, size_min=200, size_a=6.3, seed=8)
+    assert c.sizes.max() > 1500
+    side = np.random.default_rng(4).random(c.n) < 0.5
+    parts = []
+    for mask in (side, ~side):
+        ids = np.nonzero(mask)[0]
+        sizes = c.sizes[ids]
+        starts = np.concatenate([[0], np.cumsum(sizes.astype(np.int64))])[:-1].astype(np.uint32)
+        parts.append((np.concatenate([c.set(i) for i in ids]), starts, sizes))
+    R, S = (ctx.upload(t, z, s) for t, s, z in parts)
+    for tau in (0.6, 0.85):
+        exp = oracle.as_set(oracle.brute_rs(parts[0], parts[1], tau, sim=sim))
+        for kw in (dict(bitmap=0), dict(bitmap=512, fgss_batch=16), dict(bitmap=128, verify_mode=2)):
+            for orientation in ("as_given", "swapped"):
+                r = ctx.rs_join(R, S, threshold=tau, sim=sim, technique="fgss", probe_major=True,
+                                orientation=orientation, **kw)
+                assert r.count == len(exp) and oracle.as_set(r.pairs) == exp
