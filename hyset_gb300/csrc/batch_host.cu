@@ -182,7 +182,7 @@ hyset_status batch_prepare(hyset_ctx* ctx, const hyset_join_desc* joins, uint32_
                 if (R->size_hist[l]) max_pre = std::max(max_pre, bj->b->index_prefix[l]);
             const uint32_t pb = bits_for(max_pre), sb = bits_for(R->n);
             bj->ix.universe = R->universe;
-            bj->ix.pos_bits = pb + sb <= 32 ? pb : 0;
+            bj->ix.pos_bits = bj->ix.low_bits = pb + sb <= 32 ? pb : 0;
             P.X = bj->ix.view();
             if (use_bands(bj->b, bj->self)) {  // the midprefix index, same layout
                 const uint64_t E2 = prefix_entries(R, bj->b->mid_prefix);
@@ -190,7 +190,7 @@ hyset_status batch_prepare(hyset_ctx* ctx, const hyset_join_desc* joins, uint32_
                 CK(bj->ix_mid.set.ensure((E2 ? E2 : 1) * 4, s));
                 CK(bj->ix_mid.pos.ensure((E2 ? E2 : 1) * 4, s));
                 bj->ix_mid.universe = R->universe;
-                bj->ix_mid.pos_bits = bj->ix.pos_bits;
+                bj->ix_mid.pos_bits = bj->ix_mid.low_bits = bj->ix.pos_bits;
                 P.X2 = bj->ix_mid.view();
             }
         }

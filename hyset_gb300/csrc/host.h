@@ -68,13 +68,12 @@ std::vector<uint64_t> range_hist(const hyset_coll* c, uint32_t lo, uint32_t hi);
 uint64_t prefix_entries(const hyset_coll* c, const std::vector<uint32_t>& pre);
 uint64_t prefix_entries_of(const std::vector<uint64_t>& hist, const std::vector<uint32_t>& pre);
 uint32_t bits_for(uint64_t v);
-// The entry layout of an index's token records: the low rec_bits hold the
-// longest probe the entry's positional bound admits (*bound: a self-join's
-// midprefix index, kind 0, with a monotone minoverlap table, when set ids and
-// that field fit 32 bits) or the entry's position (rec_bits = pb, the lists'
-// layout).
-void record_layout(const hyset_coll* c, const Bounds* b, int kind, uint32_t pb, uint32_t* rec_bits, bool* bound);
-// The tables a bound-layout record build reads (jaccard, dice: max_sum;
+// The entry layout of a packed index: the low low_bits hold the longest probe
+// the entry's positional bound admits (*bound: a self-join's midprefix index,
+// kind 0, with a monotone minoverlap table, when set ids and that field fit 32
+// bits) or the entry's position (low_bits = pb).
+void entry_layout(const hyset_coll* c, const Bounds* b, int kind, uint32_t pb, uint32_t* low_bits, bool* bound);
+// The tables a bound-layout build reads (jaccard, dice: max_sum;
 // cosine: lp_row / lp_tab).
 BoundFields bound_fields(const Bounds* b);
 // The first set id whose prefix (pre[size] tokens) is long enough to be

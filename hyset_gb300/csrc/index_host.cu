@@ -96,10 +96,10 @@ uint32_t first_long_prefix(const hyset_coll* c, const std::vector<uint32_t>& pre
     return 0xFFFFFFFFu;
 }
 
-void record_layout(const hyset_coll* c, const Bounds* b, int kind, uint32_t pb, uint32_t* rec_bits, bool* bound) {
+void entry_layout(const hyset_coll* c, const Bounds* b, int kind, uint32_t pb, uint32_t* low_bits, bool* bound) {
     const uint32_t fb = bits_for(b->L);  // a field that holds every probe length
     *bound = kind == 0 && (b->view.max_sum != nullptr || b->view.lp_tab != nullptr) && fb + bits_for(c->n) <= 32;
-    *rec_bits = *bound ? fb : pb;
+    *low_bits = *bound ? fb : pb;
 }
 
 // Bits needed to represent v (at least 1).
@@ -184,16 +184,20 @@ hyset_status build_sorted_index(hyset_ctx* ctx, hyset_coll* c, const Bounds* b, 
     ix.universe = U;
     ix.entries = E;
     ix.records = 0;
+    ix.low_bits = packed ? pb : 0;
+    ix.bound = false;
+    // the kernel that reads records reads bound fields, in records or lists
+    if (packed && records_ok) entry_layout(c, b, kind, pb, &ix.low_bits, &ix.bound);
+    const BoundFields bf = ix.bound ? bound_fields(b) : BoundFields{};
     if (rec_fits) {
         const auto lk = c->list_longest.find(d_pre);
         const int shift = lk != c->list_longest.end() ? record_shift(lk->second, U) : 0;
         if (shift) {
             uint32_t* counts = ctx->sc->counts.as<uint32_t>();
-            record_layout(c, b, kind, pb, &ix.rec_bits, &ix.rec_bound);
             CK(ix.rec.ensure(((size_t)U << shift) * 4, s));
             CK(cudaMemsetAsync(counts, 0, (size_t)U * 4, s));
-            CK(emit_records(v, d_pre, ix.rec_bits, counts, ix.rec.as<uint32_t>(), shift, U, s, lo, hi,
-                            ix.rec_bound ? bound_fields(b) : BoundFields{}, first_long_prefix(c, *pre)));
+            CK(emit_records(v, d_pre, ix.low_bits, counts, ix.rec.as<uint32_t>(), shift, U, s, lo, hi, bf,
+                            first_long_prefix(c, *pre)));
             CK(order_records(counts, U, ix.rec.as<uint32_t>(), shift, s));
             ix.records = shift;
             ix.pos_bits = pb;
@@ -206,8 +210,8 @@ hyset_status build_sorted_index(hyset_ctx* ctx, hyset_coll* c, const Bounds* b, 
         uint32_t* counts = ctx->sc->counts.as<uint32_t>();
         CK(ctx->sc->gate.ensure(4, s));
         CK(cudaMemsetAsync(counts, 0, ((size_t)U + 1) * 4, s));
-        CK(emit_packed_entries(v, off, len, pb, ctx->sc->tok.as<uint32_t>(), ix.set.as<uint32_t>(), counts, s, lo,
-                               hi, 0xFFFFFFFFu, first_long_prefix(c, *pre)));
+        CK(emit_packed_entries(v, off, len, ix.low_bits, ctx->sc->tok.as<uint32_t>(), ix.set.as<uint32_t>(), counts, s,
+                               lo, hi, 0xFFFFFFFFu, first_long_prefix(c, *pre), bf));
         // the list build's path is read back once per collection and prefix
         // table (not while a batch is being captured into a graph)
         cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
@@ -226,10 +230,9 @@ hyset_status build_sorted_index(hyset_ctx* ctx, hyset_coll* c, const Bounds* b, 
         const int shift = rec_fits && E && read_back ? record_shift(ctx->h_flags[15], U) : 0;
         if (shift) {
             // this build's lists become records; later builds emit records directly
-            record_layout(c, b, kind, pb, &ix.rec_bits, &ix.rec_bound);
             CK(ix.rec.ensure(((size_t)U << shift) * 4, s));
-            CK(records_from_lists(ix.list_off.as<uint32_t>(), ix.set.as<uint32_t>(), U, ix.rec.as<uint32_t>(), shift, s,
-                                  ix.rec_bound ? bound_fields(b) : BoundFields{}, c->d_sizes, pb, ix.rec_bits));
+            CK(records_from_lists(ix.list_off.as<uint32_t>(), ix.set.as<uint32_t>(), U, ix.rec.as<uint32_t>(), shift,
+                                  s));
             ix.records = shift;
         }
         return HYSET_OK;

@@ -90,20 +90,20 @@ struct Index {
     uint32_t universe = 0;
     uint64_t entries = 0;
     uint32_t pos_bits = 0;  // > 0: packed (set << pos_bits) | position entries
-    // the records' layout: low rec_bits of an entry, the position or (rec_bound)
-    // the longest probe the entry's positional bound admits
-    uint32_t rec_bits = 0;
-    bool rec_bound = false;
+    // packed entries, in records or lists: the low low_bits of an entry hold its
+    // position or (bound) the longest probe its positional bound admits
+    uint32_t low_bits = 0;
+    bool bound = false;
     IndexView view() const {
         IndexView v;
         v.list_off = list_off.as<uint32_t>();
         v.set = records ? rec.as<uint32_t>() : set.as<uint32_t>();
         v.pos = pos_bits ? nullptr : pos.as<uint32_t>();
         v.universe = universe;
-        v.pos_bits = records ? rec_bits : pos_bits;
+        v.pos_bits = low_bits;
         v.sorted = 1;
         v.rec = records;
-        v.bound = records && rec_bound ? 1 : 0;
+        v.bound = bound ? 1 : 0;
         return v;
     }
 };

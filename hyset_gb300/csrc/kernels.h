@@ -103,12 +103,14 @@ cudaError_t emit_prefix_entries(CollView c, uint32_t lo, uint32_t hi, const uint
 // token histogram counts[token]++ of tokens below `limit` in the same pass
 // (counts may be nullptr).  Sets [lo, hi) only (hi = 0xFFFFFFFF: to the end);
 // ids stay absolute.
+// bf (optional, a self-join's midprefix index): the low pos_bits of each entry
+// hold its bound field (bound_field_of) instead of the position.
 // big_lo: sets from this id on have long prefixes and are emitted a warp
 // per set (below it, a warp per 32 sets).
 cudaError_t emit_packed_entries(CollView c, const uint32_t* entry_off, const uint32_t* len, uint32_t pos_bits,
                                 uint32_t* e_token, uint32_t* e_val, uint32_t* counts, cudaStream_t s,
                                 uint32_t lo = 0, uint32_t hi = 0xFFFFFFFFu, uint32_t limit = 0xFFFFFFFFu,
-                                uint32_t big_lo = 0xFFFFFFFFu);
+                                uint32_t big_lo = 0xFFFFFFFFu, BoundFields bf = BoundFields{});
 
 // Token records: when no list holds more than 31 (63) entries, list t is the
 // fixed record rec[2^shift t, 2^shift (t + 1)) of 32 (64) words, shift 5 (6):
@@ -150,11 +152,8 @@ constexpr uint32_t REC_OVERFLOW = 16;
 cudaError_t order_records(const uint32_t* counts, uint32_t U, uint32_t* rec, int shift, cudaStream_t s,
                           uint32_t* overflow = nullptr, uint32_t* prev = nullptr);
 // Records from index lists already built (every list at most record_entries(shift) long).
-// bf (optional): entries (set << list_bits) | position become
-// (set << rec_bits) | bound field (sizes: the indexed sets' sizes).
 cudaError_t records_from_lists(const uint32_t* list_off, const uint32_t* vals, uint32_t U, uint32_t* rec,
-                               int shift, cudaStream_t s, BoundFields bf = BoundFields{}, const uint32_t* sizes = nullptr,
-                               uint32_t list_bits = 0, uint32_t rec_bits = 0);
+                               int shift, cudaStream_t s);
 
 // Token histogram of n entries into counts[limit] (warp-aggregated atomics;
 // tokens >= limit are skipped; the counts are NOT zeroed here).

@@ -404,7 +404,7 @@ hyset_status hyset_self_join_host(hyset_ctx* ctx, const uint32_t* tokens, uint64
         const int records = assumed && lit != ctx->longest_cache.end() ? record_shift(lit->second, U) : 0;
         if (records) {
             CK(ix.rec.ensure(((size_t)U << records) * 4, s));
-            record_layout(C, b, 0, pb, &ix.rec_bits, &ix.rec_bound);
+            entry_layout(C, b, 0, pb, &ix.low_bits, &ix.bound);
         }
         const uint32_t big_lo = first_long_prefix(C, b->index_prefix);  // emitted a warp per set from here on
         bool lists_ready = false;  // prefix lengths and entry offsets computed
@@ -495,8 +495,8 @@ hyset_status hyset_self_join_host(hyset_ctx* ctx, const uint32_t* tokens, uint64
             else
                 CK(validate_collection(part, n_tokens, ctx->s_flags.as<uint32_t>(), C->meta.as<uint2>() + lo, s));
             if (records)
-                CK(emit_records(v, b->view.index_prefix, ix.rec_bits, counts, ix.rec.as<uint32_t>(), records, U, s, lo, hi,
-                                ix.rec_bound ? bound_fields(b) : BoundFields{}, big_lo));
+                CK(emit_records(v, b->view.index_prefix, ix.low_bits, counts, ix.rec.as<uint32_t>(), records, U, s, lo, hi,
+                                ix.bound ? bound_fields(b) : BoundFields{}, big_lo));
             else
                 CK(emit_packed_entries(v, off, len, pb, ctx->sc->tok.as<uint32_t>(), ix.set.as<uint32_t>(), counts, s,
                                        lo, hi, U + 1, big_lo));
@@ -589,6 +589,10 @@ hyset_status hyset_self_join_host(hyset_ctx* ctx, const uint32_t* tokens, uint64
                                ctx->sc->gate.as<uint32_t>(), key_bits_for(U), ctx->sc->scan.as<uint32_t>(), s));
             }
             ix.records = rec_now ? records : 0;
+            if (!rec_now) {  // these lists hold positions
+                ix.low_bits = pb;
+                ix.bound = false;
+            }
             ix.sim = b->sim;
             ix.tau = b->tau;
             ix.kind = 0;

@@ -311,17 +311,12 @@ __global__ void __launch_bounds__(256, REC ? HS_REC_EMIT_MINB : 1) k_emit_packed
     for (uint32_t s0 = lo + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * spw; s0 < c.n; s0 += warps * spw) {
         const uint32_t s = s0 + lane;
         const bool has = (uint32_t)lane < spw && s < c.n;
-        uint32_t l, start, o0 = 0, size = 0;
-        if constexpr (REC) {  // len is the prefix table by size; no offsets
-            const uint2 m = has ? c.meta[s] : make_uint2(0, 0);
-            l = has ? len[m.y] : 0u;
-            start = m.x;
-            size = m.y;
-        } else {
-            l = has ? len[s] : 0u;
-            start = has ? c.meta[s].x : 0u;
-            o0 = __shfl_sync(FULL, has ? off[s] : 0u, 0);
-        }
+        const uint2 m = has ? c.meta[s] : make_uint2(0, 0);
+        const uint32_t start = m.x, size = m.y;
+        // REC: len is the prefix table by size; no offsets
+        const uint32_t l = has ? (REC ? len[size] : len[s]) : 0u;
+        uint32_t o0 = 0;
+        if constexpr (!REC) o0 = __shfl_sync(FULL, has ? off[s] : 0u, 0);
         const uint32_t incl = warp_incl_scan(l, lane);
         const uint32_t total = __shfl_sync(FULL, incl, 31);
         for (uint32_t j0 = 0; j0 < total; j0 += 32 * ROUNDS) {
@@ -341,9 +336,9 @@ __global__ void __launch_bounds__(256, REC ? HS_REC_EMIT_MINB : 1) k_emit_packed
                 const uint32_t i = j - excl_k;
                 tok[u] = j < total ? __ldg(c.tokens + start_k + i) : 0u;
                 uint32_t low = i;
-                if constexpr (REC) {
+                if (bf.on()) {
                     const uint32_t size_k = __shfl_sync(FULL, size, k);
-                    if (bf.on() && j < total) low = bound_field_of(bf, size_k, i, maxf);
+                    if (j < total) low = bound_field_of(bf, size_k, i, maxf);
                 }
                 val[u] = ((s0 + (uint32_t)k) << pos_bits) | low;
             }
@@ -584,20 +579,13 @@ __global__ void __launch_bounds__(SHIFT == 5 ? 256 : 128) k_order_records(const 
 // Records from built lists: a warp per token, the record's word 0 the length,
 // word i > 0 entry i - 1 or the pad.
 __global__ void k_records_from_lists(const uint32_t* __restrict__ list_off, const uint32_t* __restrict__ vals,
-                                     uint32_t U, uint32_t* __restrict__ rec, int shift, BoundFields bf,
-                                     const uint32_t* __restrict__ sizes, uint32_t list_bits, uint32_t rec_bits) {
+                                     uint32_t U, uint32_t* __restrict__ rec, int shift) {
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     for (uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < U; t += warps) {
         const uint32_t a = list_off[t], b = list_off[t + 1];
-        for (uint32_t i = lane; i < 1u << shift; i += 32) {
-            uint32_t w = i == 0 ? b - a : (a + i - 1 < b ? vals[a + i - 1] : 0xFFFFFFFFu);
-            if (bf.on() && i > 0 && a + i - 1 < b) {  // (set, position) -> (set, bound field)
-                const uint32_t set = w >> list_bits, pos = w & ((1u << list_bits) - 1u);
-                w = (set << rec_bits) | bound_field_of(bf, sizes[set], pos, (1u << rec_bits) - 1u);
-            }
-            rec[(t << shift) + i] = w;
-        }
+        for (uint32_t i = lane; i < 1u << shift; i += 32)
+            rec[(t << shift) + i] = i == 0 ? b - a : (a + i - 1 < b ? vals[a + i - 1] : 0xFFFFFFFFu);
     }
 }
 
@@ -1020,9 +1008,8 @@ cudaError_t launch_emit(CollView c, uint32_t lo, uint32_t hi, uint32_t big_lo, c
 
 cudaError_t emit_packed_entries(CollView c, const uint32_t* entry_off, const uint32_t* len, uint32_t pos_bits,
                                 uint32_t* e_token, uint32_t* e_val, uint32_t* counts, cudaStream_t s, uint32_t lo,
-                                uint32_t hi, uint32_t limit, uint32_t big_lo) {
-    return launch_emit<false>(c, lo, hi, big_lo, entry_off, len, pos_bits, e_token, e_val, counts, limit,
-                              BoundFields{}, 0, s);
+                                uint32_t hi, uint32_t limit, uint32_t big_lo, BoundFields bf) {
+    return launch_emit<false>(c, lo, hi, big_lo, entry_off, len, pos_bits, e_token, e_val, counts, limit, bf, 0, s);
 }
 
 cudaError_t emit_records(CollView c, const uint32_t* prefix_tab, uint32_t pos_bits, uint32_t* counts, uint32_t* rec,
@@ -1043,13 +1030,11 @@ cudaError_t order_records(const uint32_t* counts, uint32_t U, uint32_t* rec, int
     return cudaGetLastError();
 }
 
-cudaError_t records_from_lists(const uint32_t* list_off, const uint32_t* vals, uint32_t U, uint32_t* rec,
-                               int shift, cudaStream_t s, BoundFields bf, const uint32_t* sizes, uint32_t list_bits,
-                               uint32_t rec_bits) {
+cudaError_t records_from_lists(const uint32_t* list_off, const uint32_t* vals, uint32_t U, uint32_t* rec, int shift,
+                               cudaStream_t s) {
     if (U == 0) return cudaSuccess;
     note_launches();
-    k_records_from_lists<<<grid_for((uint64_t)U * 32, 256), 256, 0, s>>>(list_off, vals, U, rec, shift, bf, sizes,
-                                                                         list_bits, rec_bits);
+    k_records_from_lists<<<grid_for((uint64_t)U * 32, 256), 256, 0, s>>>(list_off, vals, U, rec, shift);
     return cudaGetLastError();
 }
 
