@@ -65,8 +65,8 @@ hyset_status batch_record(hyset_ctx* ctx, BatchPlan& bp) {
                                       (int)bj.ix.pos_bits, bj.solo));
         }
         if (bj.words) {
-            CK(generate_bitmaps(bj.R->view(), bj.words, bj.bits_r.as<uint64_t>(), s));
-            if (!bj.self) CK(generate_bitmaps(bj.S->view(), bj.words, bj.bits_s.as<uint64_t>(), s));
+            CK(generate_signatures(bj.R, bj.words, bj.bits_r.as<uint64_t>(), s));
+            if (!bj.self) CK(generate_signatures(bj.S, bj.words, bj.bits_s.as<uint64_t>(), s));
         }
     }
     // the solo joins, heaviest first, each with the single-join kernel over its
@@ -195,8 +195,8 @@ hyset_status batch_prepare(hyset_ctx* ctx, const hyset_join_desc* joins, uint32_
             }
         }
         if (bj->words) {
-            CK(bj->bits_r.ensure((size_t)R->n * bj->words * 8 + 8, s));
-            if (!bj->self) CK(bj->bits_s.ensure((size_t)S->n * bj->words * 8 + 8, s));
+            CK(bj->bits_r.ensure(sig_bytes(R->n, bj->words), s));
+            if (!bj->self) CK(bj->bits_s.ensure(sig_bytes(S->n, bj->words), s));
             P.bits_R = bj->bits_r.as<uint64_t>();
             P.bits_S = bj->self ? P.bits_R : bj->bits_s.as<uint64_t>();
             P.words = bj->words;

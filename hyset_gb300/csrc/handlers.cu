@@ -47,8 +47,8 @@ hyset_status hyset_handler_create(hyset_ctx* ctx, const hyset_coll* coll, hyset_
     if (technique == HYSET_TECH_BITMAP) {
         // bitmap::handler ctor generates every signature up front (device_algorithms.hpp:144-156)
         h->words = (int)(bitmap_size / 64);
-        CK(h->bits.ensure((size_t)coll->n * h->words * 8 + 8, s));
-        CK(generate_bitmaps(coll->view(), h->words, h->bits.as<uint64_t>(), s));
+        CK(h->bits.ensure(sig_bytes(coll->n, h->words), s));
+        CK(generate_signatures(coll, h->words, h->bits.as<uint64_t>(), s));
     }
     CK(h->count.ensure(16, s));
     CK(h->work.ensure(16, s));

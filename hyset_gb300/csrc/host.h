@@ -89,6 +89,8 @@ hyset_status build_fgss_indexes(hyset_ctx* ctx, hyset_coll* R, const Bounds* b, 
                                 JoinParams& P);
 hyset_status build_groups(hyset_ctx* ctx, hyset_coll* c, const uint32_t* d_pre, const std::vector<uint32_t>& pre,
                           uint32_t U, uint64_t* entries);
+// generate_bitmaps of a whole collection into out (sig_bytes(c->n, words) bytes).
+cudaError_t generate_signatures(const hyset_coll* c, int words, uint64_t* out, cudaStream_t s, unsigned max_blocks = 0);
 hyset_status get_bitmaps(hyset_ctx* ctx, hyset_coll* c, int words, const uint64_t** out, cudaStream_t gen = nullptr);
 
 // ---- configuration, selector, autotuner (plan.cu) ---------------------------

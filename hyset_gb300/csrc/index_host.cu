@@ -301,13 +301,21 @@ hyset_status build_groups(hyset_ctx* ctx, hyset_coll* c, const uint32_t* d_pre, 
     return HYSET_OK;
 }
 
+cudaError_t generate_signatures(const hyset_coll* c, int words, uint64_t* out, cudaStream_t s, unsigned max_blocks) {
+    uint64_t long_tokens = 0;
+    for (size_t l = SIG_WARP_SIZE; l < c->size_hist.size(); ++l) long_tokens += c->size_hist[l] * l;
+    const uint32_t long_lo = c->max_size >= SIG_WARP_SIZE ? c->h_first_ge[SIG_WARP_SIZE] : c->n;
+    return generate_bitmaps(c->view(), words, out, s, long_lo,
+                            c->n_tokens ? (double)long_tokens / (double)c->n_tokens : 0.0, max_blocks);
+}
+
 // Signatures are regenerated on every join (the buffer is reused); the buffer
 // is sized on the context's stream, the generation runs on `gen` (default: the
 // same stream).
 hyset_status get_bitmaps(hyset_ctx* ctx, hyset_coll* c, int words, const uint64_t** out,
                          cudaStream_t gen) {
     DevBuf& d = c->bitmaps[words];
-    CK(d.ensure((size_t)c->n * words * 8 + 8, ctx->stream));
+    CK(d.ensure(sig_bytes(c->n, words), ctx->stream));
     if (gen && gen != ctx->stream) {
         CK(cudaEventRecord(ctx->ev_fork, ctx->stream));
         CK(cudaStreamWaitEvent(gen, ctx->ev_fork, 0));
@@ -315,7 +323,7 @@ hyset_status get_bitmaps(hyset_ctx* ctx, hyset_coll* c, int words, const uint64_
     // beside the index build the generation takes a few blocks per SM (it is
     // bandwidth-bound; the index build is latency-bound and needs the SMs)
     const unsigned cap = gen && gen != ctx->stream ? (unsigned)(ctx->sm_count * HS_SIG_BLOCKS_PER_SM) : 0u;
-    CK(generate_bitmaps(c->view(), words, d.as<uint64_t>(), gen ? gen : ctx->stream, cap));
+    CK(generate_signatures(c, words, d.as<uint64_t>(), gen ? gen : ctx->stream, cap));
     *out = d.as<uint64_t>();
     return HYSET_OK;
 }

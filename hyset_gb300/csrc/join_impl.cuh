@@ -87,15 +87,6 @@ __device__ __forceinline__ const uint32_t* stage_probe(const uint32_t* pg, uint3
     return sbuf;
 }
 
-template <int W>
-__device__ __forceinline__ uint32_t bitmap_xor_pop(const JoinParams& P, const uint64_t (&bp)[W], uint32_t c) {
-    uint32_t pop = 0;
-    const uint64_t* bc = P.bits_R + (uint64_t)c * W;
-#pragma unroll
-    for (int q = 0; q < W; ++q) pop += __popcll(bp[q] ^ __ldg(bc + q));
-    return pop;
-}
-
 // Verifies the warp's surviving items and appends the accepted pairs.
 // own_a / own_b: the item's position in the probe / candidate (ownership test)
 // or NOWN.
@@ -153,33 +144,51 @@ __device__ __forceinline__ uint32_t sig_distance(const uint64_t* __restrict__ a,
     return pop;
 }
 
-// Signatures are compared a 32-byte sector at a time: most pairs already differ
-// in more bits of the first 256 than the whole distance may be, so the wider
-// signatures' other sectors are read for the few that do not (the kernel
-// moves close to what L2 delivers: 7 TB/s of sectors on the 1M-set join).
-__host__ __device__ constexpr int sig_head(int W) { return W < 2 ? W : 2; }
-// The rest of the comparison for an item that its head left in (`pop` bits so
-// far; `most`: the largest distance that passes).
-template <int W>
-__device__ __forceinline__ bool sig_rest(const uint64_t* __restrict__ a, const uint64_t* __restrict__ b, uint32_t pop,
-                                         uint32_t most) {
-    if constexpr (W > 2) pop += sig_distance<W, 2, 4>(a, b);
-    if constexpr (W > 4) {
-        if (pop > most) return false;
-        pop += sig_distance<W, 4, 8>(a, b);
-    }
-    if constexpr (W > 8) {
-        if (pop > most) return false;
-        pop += sig_distance<W, 8, W>(a, b);
-    }
-    return pop <= most;
-}
-
 // One 32-byte load (sm_100 and later), non-coherent path: p must be 32-byte aligned.
 __device__ __forceinline__ void ldg256(const uint32_t* p, uint32_t (&w)[8]) {
     asm("ld.global.nc.v8.u32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
         : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
         : "l"(p));
+}
+
+// An item reads its candidate's and its probe's head records (start, size and
+// folded signature, one 32-byte sector each): most pairs already differ in more
+// bits of the folds than the whole distance may be, so the signatures are read
+// for the few that do not, a sector at a time.  The kernel moves close to what
+// L2 delivers (7 TB/s of sectors on the 1M-set join), where separate (start,
+// size) pairs and signatures cost an item two sectors or more.
+struct SigHead {
+    uint32_t start, size, pop;  // the candidate's; pop: bits in which the folds differ
+};
+template <int W>
+__device__ __forceinline__ SigHead sig_head(const uint32_t* __restrict__ probe, const uint32_t* __restrict__ cand) {
+    constexpr int N = 2 * W < (int)HEAD_WORDS ? 2 * W : (int)HEAD_WORDS;
+    uint32_t a[8], b[8];
+    ldg256(cand, b);
+    ldg256(probe, a);
+    SigHead h{b[0], b[1], 0};
+#pragma unroll
+    for (int w = 0; w < N; ++w) h.pop += __popc(a[2 + w] ^ b[2 + w]);
+    return h;
+}
+// The whole comparison for an item that its head left in (most: the largest
+// distance that passes); a fold of a signature no wider than itself is exact.
+template <int W>
+__device__ __forceinline__ bool sig_rest(const uint64_t* __restrict__ a, const uint64_t* __restrict__ b, uint32_t most) {
+    if constexpr (2 * W <= (int)HEAD_WORDS) {
+        return true;
+    } else {
+        uint32_t pop = sig_distance<W, 0, 4>(a, b);
+        if constexpr (W > 4) {
+            if (pop > most) return false;
+            pop += sig_distance<W, 4, 8>(a, b);
+        }
+        if constexpr (W > 8) {
+            if (pop > most) return false;
+            pop += sig_distance<W, 8, W>(a, b);
+        }
+        return pop <= most;
+    }
 }
 
 // Window [klo, khi) of a token record (length word, then ascending entries
@@ -350,20 +359,18 @@ __device__ void fgss_batch(const JoinParams& P, uint32_t i0, uint32_t k, int lan
                 if (!P.X.sorted) keep = c >= ilo && c < ihi;
                 if constexpr (BD) keep = keep && ilp <= pc;  // pc: the longest probe the entry admits
             }
-            // The first 256 signature bits are loaded with the candidate's meta (one
-            // round trip) where a pair takes no more; wider signatures only for
-            // items that pass the positional bound.
-            constexpr bool early_sig = W > 0 && W <= 4;
-            const uint64_t *sig_p = nullptr, *sig_c = nullptr;
-            if constexpr (W > 0) {
-                sig_p = P.bits_S + (uint64_t)ip * W;
-                sig_c = P.bits_R + (uint64_t)c * W;
-            }
             if (keep) {
-                const uint2 cm = P.R.meta[c];
-                if constexpr (early_sig) pop = sig_distance<W, 0, sig_head(W)>(sig_p, sig_c);
-                cstart = cm.x;
-                lc = cm.y;
+                if constexpr (W > 0) {
+                    const SigHead h = sig_head<W>(sig_heads(P.bits_S, P.S.n, W) + (uint64_t)ip * 8,
+                                                  sig_heads(P.bits_R, P.R.n, W) + (uint64_t)c * 8);
+                    cstart = h.start;
+                    lc = h.size;
+                    pop = h.pop;
+                } else {
+                    const uint2 cm = P.R.meta[c];
+                    cstart = cm.x;
+                    lc = cm.y;
+                }
                 const uint32_t big = max(ilp, lc), small = min(ilp, lc);
                 mo = minoverlap(P.B, big, small);
                 keep = BD ? ilp - jp >= mo : 1u + min(ilp - jp - 1u, lc - pc - 1u) >= mo;  // positional bound
@@ -373,8 +380,8 @@ __device__ void fgss_batch(const JoinParams& P, uint32_t i0, uint32_t k, int lan
             if constexpr (W > 0) {
                 if (keep) {
                     const uint32_t most = ilp + lc - 2u * mo;
-                    if constexpr (!early_sig) pop = sig_distance<W, 0, sig_head(W)>(sig_p, sig_c);
-                    keep = pop <= most && sig_rest<W>(sig_p, sig_c, pop, most);
+                    keep = pop <= most &&
+                           sig_rest<W>(P.bits_S + (uint64_t)ip * W, P.bits_R + (uint64_t)c * W, most);
                 }
             }
             count_stat<ST>(P, 1, keep ? 1u : 0u, lane);
@@ -433,19 +440,20 @@ __device__ __forceinline__ void run_items(const JoinParams& P, ItemLane& it, int
     const uint32_t c = keep ? it.c : 0u, pc = it.pc, jp = it.jp, ip = it.ip, ilp = it.ilp;
     uint32_t lc = 0, mo = 0, cstart = 0, pop = 0;
     count_stat<ST>(P, 0, keep ? 1u : 0u, lane);
-    // as in fgss_batch; with bound-layout entries almost every item here has
-    // passed the positional bound already, so every width's head loads early
-    constexpr bool early_sig = W > 0 && (W <= 4 || BD);
-    const uint64_t *sig_p = nullptr, *sig_c = nullptr;
-    if constexpr (W > 0) {
-        sig_p = P.bits_S + (uint64_t)ip * W;
-        sig_c = P.bits_R + (uint64_t)c * W;
-    }
+    // with signatures one record holds the candidate's start and size and the
+    // head of its signature
     if (keep) {
-        const uint2 cm = P.R.meta[c];
-        if constexpr (early_sig) pop = sig_distance<W, 0, sig_head(W)>(sig_p, sig_c);
-        cstart = cm.x;
-        lc = cm.y;
+        if constexpr (W > 0) {
+            const SigHead h = sig_head<W>(sig_heads(P.bits_S, P.S.n, W) + (uint64_t)ip * 8,
+                                          sig_heads(P.bits_R, P.R.n, W) + (uint64_t)c * 8);
+            cstart = h.start;
+            lc = h.size;
+            pop = h.pop;
+        } else {
+            const uint2 cm = P.R.meta[c];
+            cstart = cm.x;
+            lc = cm.y;
+        }
         const uint32_t big = max(ilp, lc), small = min(ilp, lc);
         mo = minoverlap(P.B, big, small);
         // positional bound; with bound-layout entries the candidate's side was
@@ -456,8 +464,8 @@ __device__ __forceinline__ void run_items(const JoinParams& P, ItemLane& it, int
     if constexpr (W > 0) {
         if (keep) {
             const uint32_t most = ilp + lc - 2u * mo;
-            if constexpr (!early_sig) pop = sig_distance<W, 0, sig_head(W)>(sig_p, sig_c);
-            keep = pop <= most && sig_rest<W>(sig_p, sig_c, pop, most);
+            keep = pop <= most &&
+                   sig_rest<W>(P.bits_S + (uint64_t)ip * W, P.bits_R + (uint64_t)c * W, most);
         }
     }
     count_stat<ST>(P, 1, keep ? 1u : 0u, lane);

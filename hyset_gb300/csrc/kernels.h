@@ -215,16 +215,21 @@ cudaError_t size_scan(const uint32_t* sizes, const uint32_t* starts, bool starts
 // The same pass writes meta[i] = (starts[i], sizes[i]).
 cudaError_t validate_collection(CollView c, uint64_t n_tokens, uint32_t* flags, uint2* meta, cudaStream_t s);
 // validate_collection and generate_bitmaps (words in {1, 2, 4, 8, 16}) in one
-// pass over the tokens; min_size (optional): no set of c is shorter (sizes are
-// ordered), parts of long sets are read a warp per set.
+// pass over the tokens, heads: the first of these sets' head records; min_size
+// (optional): no set of c is shorter (sizes are ordered), parts of long sets
+// are read a warp per set.
 cudaError_t validate_with_bitmaps(CollView c, uint64_t n_tokens, uint32_t* flags, uint2* meta, int words, uint64_t* out,
-                                  cudaStream_t s, uint32_t min_size = 0);
+                                  uint32_t* heads, cudaStream_t s, uint32_t min_size = 0);
 
 // XOR bitmap signatures, bit (token mod bits) per token
-// (include/hyset/device_algorithms.hpp:58-74), words = bits / 64 in {1,2,4,8}.
-// max_blocks > 0 caps the grid (signatures generated beside other work leave
-// it SMs).
-cudaError_t generate_bitmaps(CollView c, int words, uint64_t* out, cudaStream_t s, unsigned max_blocks = 0);
+// (include/hyset/device_algorithms.hpp:58-74), words = bits / 64 in
+// {1, 2, 4, 8, 16}, and their head records: out holds sig_bytes(c.n, words)
+// bytes.  Sets from long_lo on have at least SIG_WARP_SIZE tokens, long_share
+// of all tokens (a warp per set; c.n and 0: none).  max_blocks > 0 caps the
+// grid (signatures generated beside other work leave it SMs).
+constexpr uint32_t SIG_WARP_SIZE = 128;
+cudaError_t generate_bitmaps(CollView c, int words, uint64_t* out, cudaStream_t s, uint32_t long_lo, double long_share,
+                             unsigned max_blocks = 0);
 
 // ---- join.cu --------------------------------------------------------------
 struct IndexView {

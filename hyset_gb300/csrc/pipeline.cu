@@ -380,7 +380,7 @@ hyset_status hyset_self_join_host(hyset_ctx* ctx, const uint32_t* tokens, uint64
         CollView v = C->view();
         const int words = (int)(tn.bits / 64);
         DevBuf& bits = C->bitmaps[words];
-        if (words) CK(bits.ensure((size_t)n * words * 8 + 8, s));
+        if (words) CK(bits.ensure(sig_bytes(n, words), s));
         // A collection with the same size profile joined before: its universe
         // is assumed, so the token histogram is counted as the chunks land and
         // the checks are read after the join (one synchronisation); a larger
@@ -491,7 +491,8 @@ hyset_status hyset_self_join_host(hyset_ctx* ctx, const uint32_t* tokens, uint64
             // the checks (and the signatures, in the same pass over the tokens)
             if (words)
                 CK(validate_with_bitmaps(part, n_tokens, ctx->s_flags.as<uint32_t>(), C->meta.as<uint2>() + lo, words,
-                                         bits.as<uint64_t>() + (size_t)lo * words, s, size_at(C, lo)));
+                                         bits.as<uint64_t>() + (size_t)lo * words,
+                                         sig_heads(bits.as<uint64_t>(), n, words) + (size_t)lo * 8, s, size_at(C, lo)));
             else
                 CK(validate_collection(part, n_tokens, ctx->s_flags.as<uint32_t>(), C->meta.as<uint2>() + lo, s));
             if (records)

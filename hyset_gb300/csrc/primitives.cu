@@ -639,57 +639,92 @@ __global__ void k_iota(uint32_t* out, uint64_t n) {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) out[i] = (uint32_t)i;
 }
 
-// Eight lanes per set (four sets per warp).  The group's 2W 32-bit signature
-// words live in shared memory; every token flips its bit there with one
-// shared-memory XOR (a register fold would cost a compare and select per word
-// per token), four token loads in flight per lane; the group's lanes then
-// store the words (coalesced).  Bit b of the signature is bit b%32 of 32-bit
-// word b/32 (the popcount of a XOR of two signatures does not depend on the
-// bit layout).
+// The head record of set s (start and size m, signature words `mine` in shared
+// memory): lane g < 8 of its lanes writes word g (32 bytes, coalesced).
+template <int NW>
+__device__ __forceinline__ void store_head(uint32_t* heads, uint64_t s, uint2 m, const uint32_t* mine, int g) {
+    if (g >= 8) return;
+    uint32_t x = g == 0 ? m.x : g == 1 ? m.y : 0u;
+    if (g >= 2) {
+#pragma unroll
+        for (int w = 0; w < NW; w += (int)HEAD_WORDS)
+            if (w + g - 2 < NW) x ^= mine[w + g - 2];
+    }
+    heads[s * 8 + g] = x;
+}
+
+// XORs the bits of a set's l tokens at t into its signature words `mine` in
+// shared memory (one shared-memory XOR per token: a register fold would cost a
+// compare and select per word per token), BITMAP_UNROLL loads in flight per
+// lane; LPS lanes, g the lane's place among them.
 constexpr int BITMAP_THREADS = 256;
-constexpr int BITMAP_UNROLL = 4;
-template <int W>
-__global__ void __launch_bounds__(BITMAP_THREADS) k_bitmaps(CollView c, uint64_t* out) {
-    constexpr int NW = 2 * W;
-    __shared__ uint32_t sw[BITMAP_THREADS / 8][NW];
-    const int lane = threadIdx.x & 31, g = lane & 7;
-    uint32_t* mine = sw[threadIdx.x >> 3];
-    const uint32_t mask = 64u * W - 1u;
-    const uint32_t groups = (gridDim.x * blockDim.x) >> 3;
-    uint32_t* out32 = reinterpret_cast<uint32_t*>(out);
-    // every lane iterates the same number of times so the warp barriers match
-    const uint32_t rounds = (c.n + groups - 1) / groups;
-    uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
-    for (uint32_t r = 0; r < rounds; ++r, s += groups) {
+constexpr int BITMAP_UNROLL = 8;
+template <int LPS>
+__device__ __forceinline__ void sign_set(const uint32_t* __restrict__ t, uint32_t l, uint32_t* mine, uint32_t mask,
+                                         int g) {
+    for (uint32_t i0 = g; i0 < l; i0 += LPS * BITMAP_UNROLL) {
+        uint32_t tok[BITMAP_UNROLL];
 #pragma unroll
-        for (int q = g; q < NW; q += 8) mine[q] = 0u;
-        __syncwarp();
-        const bool live = s < c.n;
-        uint2 m = make_uint2(0, 0);
-        if (live) m = c.meta[s];
-        const uint32_t* t = c.tokens + m.x;
-        for (uint32_t i0 = g; i0 < m.y; i0 += 8 * BITMAP_UNROLL) {
-            uint32_t tok[BITMAP_UNROLL];
+        for (int u = 0; u < BITMAP_UNROLL; ++u) {
+            const uint32_t i = i0 + (uint32_t)LPS * u;
+            tok[u] = i < l ? __ldg(t + i) : 0xFFFFFFFFu;
+        }
 #pragma unroll
-            for (int u = 0; u < BITMAP_UNROLL; ++u) {
-                const uint32_t i = i0 + 8u * u;
-                tok[u] = i < m.y ? __ldg(t + i) : 0xFFFFFFFFu;
-            }
-#pragma unroll
-            for (int u = 0; u < BITMAP_UNROLL; ++u) {
-                if (i0 + 8u * u < m.y) {
-                    const uint32_t b = tok[u] & mask;
-                    atomicXor(&mine[b >> 5], 1u << (b & 31));
-                }
+        for (int u = 0; u < BITMAP_UNROLL; ++u) {
+            if (i0 + (uint32_t)LPS * u < l) {
+                const uint32_t b = tok[u] & mask;
+                atomicXor(&mine[b >> 5], 1u << (b & 31));
             }
         }
+    }
+}
+
+// The signatures and head records of sets [lo, hi), LPS lanes per set, by
+// blocks [block, block + blocks) of the grid.  Bit b of the signature is bit
+// b%32 of 32-bit word b/32 (the popcount of a XOR of two signatures does not
+// depend on the bit layout).
+template <int W, int LPS>
+__device__ __forceinline__ void sign_sets(const CollView& c, uint32_t lo, uint32_t hi, uint32_t block, uint32_t blocks,
+                                          uint32_t* out32, uint32_t* heads, uint32_t (*sw)[2 * W]) {
+    constexpr int NW = 2 * W;
+    const int g = threadIdx.x & (LPS - 1);
+    uint32_t* mine = sw[threadIdx.x / LPS];
+    const uint32_t groups = blocks * (BITMAP_THREADS / LPS);
+    // every lane iterates the same number of times so the warp barriers match
+    const uint32_t rounds = (hi - lo + groups - 1) / groups;
+    uint32_t k = block * (BITMAP_THREADS / LPS) + threadIdx.x / LPS;  // counted from the longest set
+    for (uint32_t r = 0; r < rounds; ++r, k += groups) {
+#pragma unroll
+        for (int q = g; q < NW; q += LPS) mine[q] = 0u;
+        __syncwarp();
+        const bool live = k < hi - lo;
+        const uint32_t s = live ? hi - 1 - k : 0u;
+        const uint2 m = live ? c.meta[s] : make_uint2(0, 0);
+        sign_set<LPS>(c.tokens + m.x, m.y, mine, 64u * W - 1u, g);
         __syncwarp();
         if (live) {
 #pragma unroll
-            for (int q = g; q < NW; q += 8) out32[(uint64_t)s * NW + q] = mine[q];
+            for (int q = g; q < NW; q += LPS) out32[(uint64_t)s * NW + q] = mine[q];
+            store_head<NW>(heads, s, m, mine, g);
         }
         __syncwarp();
     }
+}
+
+// Long sets a warp each, by the grid's first blocks in proportion to their
+// tokens, the others eight lanes each; either from the longest.  All at eight
+// lanes in ascending order, the longest sets' lanes (250 tokens each) ran last
+// and alone: the SMs were active 45 % of 56 us for 200,000 long sets at 256
+// bits.
+template <int W>
+__global__ void __launch_bounds__(BITMAP_THREADS) k_bitmaps(CollView c, uint64_t* out, uint32_t* heads, uint32_t long_lo,
+                                                            uint32_t long_blocks) {
+    __shared__ uint32_t sw[BITMAP_THREADS / 8][2 * W];
+    uint32_t* out32 = reinterpret_cast<uint32_t*>(out);
+    if (blockIdx.x < long_blocks)
+        sign_sets<W, 32>(c, long_lo, c.n, blockIdx.x, long_blocks, out32, heads, sw);
+    else
+        sign_sets<W, 8>(c, 0, long_lo, blockIdx.x - long_blocks, gridDim.x - long_blocks, out32, heads, sw);
 }
 
 // The checks of k_validate and the signatures of k_bitmaps in one pass over
@@ -698,9 +733,10 @@ __global__ void __launch_bounds__(BITMAP_THREADS) k_bitmaps(CollView c, uint64_t
 // the set's meta pair is written from its start and size, and its tokens are
 // read once for both (the order check reads each token's successor, an L1
 // hit).
+constexpr int VALIDATE_UNROLL = 4;
 template <int W, int LPS>
 __global__ void __launch_bounds__(BITMAP_THREADS) k_validate_bitmaps(CollView c, uint64_t n_tokens, uint32_t* flags,
-                                                                    uint2* meta, uint64_t* out) {
+                                                                    uint2* meta, uint64_t* out, uint32_t* heads) {
     static_assert(LPS == 8 || LPS == 32, "lanes per set");
     constexpr int NW = 2 * W;
     constexpr int SH = LPS == 8 ? 3 : 5;
@@ -733,16 +769,16 @@ __global__ void __launch_bounds__(BITMAP_THREADS) k_validate_bitmaps(CollView c,
             }
         }
         const uint32_t* t = c.tokens + st;
-        for (uint32_t i0 = g; i0 < l; i0 += LPS * BITMAP_UNROLL) {
-            uint32_t tok[BITMAP_UNROLL], nxt[BITMAP_UNROLL];
+        for (uint32_t i0 = g; i0 < l; i0 += LPS * VALIDATE_UNROLL) {
+            uint32_t tok[VALIDATE_UNROLL], nxt[VALIDATE_UNROLL];
 #pragma unroll
-            for (int u = 0; u < BITMAP_UNROLL; ++u) {
+            for (int u = 0; u < VALIDATE_UNROLL; ++u) {
                 const uint32_t i = i0 + (uint32_t)LPS * u;
                 tok[u] = i < l ? __ldg(t + i) : 0xFFFFFFFFu;
                 nxt[u] = i + 1 < l ? __ldg(t + i + 1) : 0xFFFFFFFFu;
             }
 #pragma unroll
-            for (int u = 0; u < BITMAP_UNROLL; ++u) {
+            for (int u = 0; u < VALIDATE_UNROLL; ++u) {
                 const uint32_t i = i0 + (uint32_t)LPS * u;
                 if (i < l) {
                     if (i + 1 < l && tok[u] >= nxt[u]) f |= 2;
@@ -755,6 +791,7 @@ __global__ void __launch_bounds__(BITMAP_THREADS) k_validate_bitmaps(CollView c,
         if (live) {
 #pragma unroll
             for (int q = g; q < NW; q += LPS) out32[(uint64_t)s * NW + q] = mine[q];
+            store_head<NW>(heads, s, make_uint2(st, c.sizes[s]), mine, g);
         }
         __syncwarp();
     }
@@ -1157,15 +1194,15 @@ cudaError_t validate_collection(CollView c, uint64_t n_tokens, uint32_t* flags, 
 namespace {
 template <int LPS>
 cudaError_t launch_validate_bitmaps(CollView c, uint64_t n_tokens, uint32_t* flags, uint2* meta, int words,
-                                    uint64_t* out, cudaStream_t s) {
+                                    uint64_t* out, uint32_t* heads, cudaStream_t s) {
     const unsigned g = grid_for((uint64_t)c.n * LPS, BITMAP_THREADS);
     note_launches();
     switch (words) {
-    case 1: k_validate_bitmaps<1, LPS><<<g, BITMAP_THREADS, 0, s>>>(c, n_tokens, flags, meta, out); break;
-    case 2: k_validate_bitmaps<2, LPS><<<g, BITMAP_THREADS, 0, s>>>(c, n_tokens, flags, meta, out); break;
-    case 4: k_validate_bitmaps<4, LPS><<<g, BITMAP_THREADS, 0, s>>>(c, n_tokens, flags, meta, out); break;
-    case 8: k_validate_bitmaps<8, LPS><<<g, BITMAP_THREADS, 0, s>>>(c, n_tokens, flags, meta, out); break;
-    case 16: k_validate_bitmaps<16, LPS><<<g, BITMAP_THREADS, 0, s>>>(c, n_tokens, flags, meta, out); break;
+    case 1: k_validate_bitmaps<1, LPS><<<g, BITMAP_THREADS, 0, s>>>(c, n_tokens, flags, meta, out, heads); break;
+    case 2: k_validate_bitmaps<2, LPS><<<g, BITMAP_THREADS, 0, s>>>(c, n_tokens, flags, meta, out, heads); break;
+    case 4: k_validate_bitmaps<4, LPS><<<g, BITMAP_THREADS, 0, s>>>(c, n_tokens, flags, meta, out, heads); break;
+    case 8: k_validate_bitmaps<8, LPS><<<g, BITMAP_THREADS, 0, s>>>(c, n_tokens, flags, meta, out, heads); break;
+    case 16: k_validate_bitmaps<16, LPS><<<g, BITMAP_THREADS, 0, s>>>(c, n_tokens, flags, meta, out, heads); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
@@ -1173,24 +1210,30 @@ cudaError_t launch_validate_bitmaps(CollView c, uint64_t n_tokens, uint32_t* fla
 }  // namespace
 
 cudaError_t validate_with_bitmaps(CollView c, uint64_t n_tokens, uint32_t* flags, uint2* meta, int words, uint64_t* out,
-                                  cudaStream_t s, uint32_t min_size) {
+                                  uint32_t* heads, cudaStream_t s, uint32_t min_size) {
     if (c.n == 0) return cudaSuccess;
-    constexpr uint32_t WARP_SET_SIZE = 128;  // sets this long (all of the part) take a warp each
-    return min_size >= WARP_SET_SIZE ? launch_validate_bitmaps<32>(c, n_tokens, flags, meta, words, out, s)
-                                     : launch_validate_bitmaps<8>(c, n_tokens, flags, meta, words, out, s);
+    return min_size >= SIG_WARP_SIZE ? launch_validate_bitmaps<32>(c, n_tokens, flags, meta, words, out, heads, s)
+                                     : launch_validate_bitmaps<8>(c, n_tokens, flags, meta, words, out, heads, s);
 }
 
-cudaError_t generate_bitmaps(CollView c, int words, uint64_t* out, cudaStream_t s, unsigned max_blocks) {
+cudaError_t generate_bitmaps(CollView c, int words, uint64_t* out, cudaStream_t s, uint32_t long_lo, double long_share,
+                             unsigned max_blocks) {
     if (c.n == 0) return cudaSuccess;
-    unsigned g = grid_for((uint64_t)c.n * 8, BITMAP_THREADS);
-    if (max_blocks && g > max_blocks) g = max_blocks;
+    if (long_lo > c.n) long_lo = c.n;
+    uint32_t* heads = sig_heads(out, c.n, words);
+    unsigned g = std::max(2u, grid_for((uint64_t)c.n * 8 + (uint64_t)(c.n - long_lo) * 24, BITMAP_THREADS));
+    if (max_blocks > 1 && g > max_blocks) g = max_blocks;
+    // each part has a block where it has sets
+    unsigned nl = (unsigned)(long_share * g + 0.5);
+    nl = std::min(std::max(nl, long_lo < c.n ? 1u : 0u), long_lo > 0 ? g - 1u : g);
+    if (long_lo == c.n) nl = 0;
     note_launches();
     switch (words) {
-    case 1: k_bitmaps<1><<<g, BITMAP_THREADS, 0, s>>>(c, out); break;
-    case 2: k_bitmaps<2><<<g, BITMAP_THREADS, 0, s>>>(c, out); break;
-    case 4: k_bitmaps<4><<<g, BITMAP_THREADS, 0, s>>>(c, out); break;
-    case 8: k_bitmaps<8><<<g, BITMAP_THREADS, 0, s>>>(c, out); break;
-    case 16: k_bitmaps<16><<<g, BITMAP_THREADS, 0, s>>>(c, out); break;
+    case 1: k_bitmaps<1><<<g, BITMAP_THREADS, 0, s>>>(c, out, heads, long_lo, nl); break;
+    case 2: k_bitmaps<2><<<g, BITMAP_THREADS, 0, s>>>(c, out, heads, long_lo, nl); break;
+    case 4: k_bitmaps<4><<<g, BITMAP_THREADS, 0, s>>>(c, out, heads, long_lo, nl); break;
+    case 8: k_bitmaps<8><<<g, BITMAP_THREADS, 0, s>>>(c, out, heads, long_lo, nl); break;
+    case 16: k_bitmaps<16><<<g, BITMAP_THREADS, 0, s>>>(c, out, heads, long_lo, nl); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
