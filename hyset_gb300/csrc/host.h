@@ -137,7 +137,7 @@ void split_heavy(const hyset_coll* S, const Bounds* b, JoinParams& P);
 // the pairs when asked (up to PAIR_SORT_MAX) and starts the copies of their
 // number (joined_count, after the stream has synchronised) and of the first
 // EARLY_PAIRS of them.
-constexpr uint64_t EARLY_PAIRS = 8192;
+constexpr uint64_t EARLY_PAIRS = 32768;  // 256 KB: under 2 us of copy
 PairSortJob pair_sort_job(const JoinParams& P);
 hyset_status enqueue_result(hyset_ctx* ctx, const JoinParams& P, const hyset_join_opts* o);
 uint64_t joined_count(const hyset_ctx* ctx);

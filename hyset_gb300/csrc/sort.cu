@@ -81,8 +81,15 @@ __global__ void __cluster_dims__(PS_CLUSTER, 1, 1) __launch_bounds__(PS_THREADS,
                 const uint32_t i = w0 + 32u * r + lane;
                 const bool valid = i < mine;
                 k[r] = valid ? sm.key[cur][i] : 0ull;
-                const uint32_t d = valid ? (uint32_t)(k[r] >> shift) & mask : 0xFFFFFFFFu;
-                const unsigned peers = __match_any_sync(FULL, d);
+                const uint32_t d = (uint32_t)(k[r] >> shift) & mask;
+                // the lanes with this digit, by a vote per bit (__match_any_sync took
+                // several times as long: 128 of them per block and pass)
+                unsigned peers = __ballot_sync(FULL, valid);
+#pragma unroll
+                for (int b = 0; b < 8; ++b) {
+                    const unsigned set = __ballot_sync(FULL, (d >> b) & 1u);
+                    peers &= (d >> b) & 1u ? set : ~set;
+                }
                 const uint32_t before = valid ? sm.whist[warp][d] : 0u;
                 __syncwarp();
                 if (valid && lane == __ffs(peers) - 1) sm.whist[warp][d] = before + __popc(peers);
