@@ -209,43 +209,63 @@ __device__ __forceinline__ bool verify_serial(const uint32_t* a, uint32_t na, co
     return ok && found >= thr;
 }
 
-// Whole warp, merge-path style: 32 tokens of b per step (one coalesced 128-byte
-// load), each lane locates its token in a by binary search, matches are counted
-// with __ballot_sync.  After each step the exact remaining upper bound
-// found + min(|b| - consumed_b, |a| - consumed_a) ends the loop as soon as the
-// pair can no longer reach thr, and the loop also ends once found >= thr.
+// Whole warp, merge-path style, in blocks of 32 tokens of either set, a token
+// per lane (one coalesced 128-byte load each, the next blocks' in flight):
+// each lane finds its token of b's block in a's by a search over the lanes,
+// matches are counted with __ballot_sync, and the block that ends first is
+// replaced.  What a step costs is that search's shuffles; a search of the rest
+// of a in memory, eleven dependent loads for 2,000 tokens, took ten times as
+// long.  After each step the exact remaining upper bound, found plus the smaller
+// number of tokens that can still match, ends the loop as soon as the pair can
+// no longer reach thr, and the loop also ends once found >= thr.
 // own_b != NOWN: a match at b[k], k < own_b, means a smaller common token
 // exists, so the pair is owned by another work item and false is returned.
-// All 32 lanes must call it with the same arguments.
-// *used (optional) receives the number of tokens of b read plus the positions
-// of a searched past (a bound on the tokens of a read).
+// All 32 lanes must call it with the same arguments; na, nb >= 1.
+// *used (optional) receives the number of tokens of both sets read.
 __device__ __forceinline__ bool verify_warp(const uint32_t* a, uint32_t na, const uint32_t* __restrict__ b,
                                             uint32_t nb, uint32_t thr, uint32_t own_b, int lane,
                                             uint32_t* used = nullptr) {
-    uint32_t found = 0, alo = 0;
-    if (used) *used = nb;
-    for (uint32_t k0 = 0; k0 < nb; k0 += 32) {
-        if (used) *used = min(nb, k0 + 32) + alo;
-        uint32_t k = k0 + lane;
-        bool valid = k < nb;
-        uint32_t y = valid ? __ldg(b + k) : 0xFFFFFFFFu;
-        uint32_t pos = valid ? lower_bound_u32(a, alo, na, y) : na;
-        bool hit = valid && pos < na && a[pos] == y;
-        unsigned m = __ballot_sync(FULL, hit);
-        if (own_b != NOWN && own_b > k0) {
-            uint32_t lim = own_b - k0;
-            unsigned early = lim >= 32 ? FULL : ((1u << lim) - 1u);
-            if (m & early) return false;
+    constexpr uint32_t PAD = 0xFFFFFFFFu;  // no token: blocks past a set's end
+    uint32_t found = 0, ia = 0, ib = 0;    // first token of either block
+    auto load_a = [&](uint32_t i) { return i + lane < na ? a[i + lane] : PAD; };
+    auto load_b = [&](uint32_t i) { return i + lane < nb ? __ldg(b + i + lane) : PAD; };
+    uint32_t x = load_a(0), y = load_b(0), xn = load_a(32), yn = load_b(32);
+    bool result = false;
+    for (;;) {
+        const uint32_t lx = __shfl_sync(FULL, x, min(31u, na - 1 - ia)), ly = __shfl_sync(FULL, y, min(31u, nb - 1 - ib));
+        uint32_t pos = 0;
+#pragma unroll
+        for (uint32_t step = 16; step >= 1; step >>= 1)
+            if (__shfl_sync(FULL, x, pos + step - 1) < y) pos += step;
+        const uint32_t at = __shfl_sync(FULL, x, pos);  // every lane shuffles, also the ones without a token
+        const bool hit = y != PAD && at == y;
+        const unsigned m = __ballot_sync(FULL, hit);
+        if (own_b != NOWN && own_b > ib) {
+            const uint32_t lim = own_b - ib;
+            if (m & (lim >= 32 ? FULL : (1u << lim) - 1u)) break;
         }
         found += __popc(m);
-        uint32_t last = min(31u, nb - 1 - k0);
-        uint32_t consumed_a = __shfl_sync(FULL, pos + (hit ? 1u : 0u), last);
-        uint32_t consumed_b = k0 + last + 1;
-        if (found >= thr) return true;
-        if (found + min(nb - consumed_b, na - consumed_a) < thr) return false;
-        alo = consumed_a;
+        if (found >= thr) {
+            result = true;
+            break;
+        }
+        // every token up to the smaller of the blocks' ends has met its match
+        const uint32_t end = min(lx, ly);
+        const uint32_t da = ia + __popc(__ballot_sync(FULL, x <= end)), db = ib + __popc(__ballot_sync(FULL, y <= end));
+        if (found + min(na - da, nb - db) < thr || da >= na || db >= nb) break;
+        if (lx <= ly) {
+            ia += 32;
+            x = xn;
+            xn = load_a(ia + 32);
+        }
+        if (ly <= lx) {
+            ib += 32;
+            y = yn;
+            yn = load_b(ib + 32);
+        }
     }
-    return found >= thr;
+    if (used) *used = min(na, ia + 32) + min(nb, ib + 32);
+    return result;
 }
 
 }  // namespace hs

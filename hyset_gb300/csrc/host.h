@@ -139,6 +139,8 @@ void split_heavy(const hyset_coll* S, const Bounds* b, JoinParams& P);
 // EARLY_PAIRS of them.
 constexpr uint64_t EARLY_PAIRS = 32768;  // 256 KB: under 2 us of copy
 PairSortJob pair_sort_job(const JoinParams& P);
+hyset_status enqueue_result(hyset_ctx* ctx, const Sink& out, const hyset_join_opts* o,
+                            const PairSortJob* sort = nullptr);
 hyset_status enqueue_result(hyset_ctx* ctx, const JoinParams& P, const hyset_join_opts* o);
 uint64_t joined_count(const hyset_ctx* ctx);
 // The signature technique's probes that are taken in small units
@@ -147,6 +149,8 @@ void split_window(const hyset_coll* R, const hyset_coll* S, const Bounds* b, int
 // The pairs of a finished join (res->count of them in the context's pair
 // buffer, enqueue_result done and the stream synchronised): sorted when asked,
 // left on the device or copied to the host.
+hyset_status deliver_pairs(hyset_ctx* ctx, const Sink& out, uint32_t n_probe, uint32_t n_indexed,
+                           const hyset_join_opts* o, hyset_result* res);
 hyset_status deliver_pairs(hyset_ctx* ctx, const JoinParams& P, const hyset_join_opts* o, hyset_result* res);
 hyset_status do_join(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const hyset_join_opts* o, hyset_result* res);
 

@@ -136,18 +136,22 @@ PairSortJob pair_sort_job(const JoinParams& P) {
                        (int)bits_for(P.out.swap ? P.S.n : P.R.n)};
 }
 
-hyset_status enqueue_result(hyset_ctx* ctx, const JoinParams& P, const hyset_join_opts* o) {
+hyset_status enqueue_result(hyset_ctx* ctx, const Sink& out, const hyset_join_opts* o, const PairSortJob* sort) {
     cudaStream_t s = ctx->stream;
-    if (!o->count_only && o->sort_pairs) CK(sort_pairs_cluster(pair_sort_job(P), s));
-    CK(cudaMemcpyAsync(ctx->h_flags + 16, P.out.count, 8, cudaMemcpyDeviceToHost, s));
+    if (sort && !o->count_only && o->sort_pairs) CK(sort_pairs_cluster(*sort, s));
+    CK(cudaMemcpyAsync(ctx->h_flags + 16, out.count, 8, cudaMemcpyDeviceToHost, s));
     if (!o->count_only && !o->device_pairs) {
-        const uint64_t early = std::min<uint64_t>(P.out.cap, EARLY_PAIRS);
+        const uint64_t early = std::min<uint64_t>(out.cap, EARLY_PAIRS);
         void* stage = nullptr;
         ST(host_stage(ctx, early * sizeof(hyset_pair), &stage));
-        if (early)
-            CK(cudaMemcpyAsync(stage, P.out.pairs, early * sizeof(hyset_pair), cudaMemcpyDeviceToHost, s));
+        if (early) CK(cudaMemcpyAsync(stage, out.pairs, early * sizeof(hyset_pair), cudaMemcpyDeviceToHost, s));
     }
     return HYSET_OK;
+}
+
+hyset_status enqueue_result(hyset_ctx* ctx, const JoinParams& P, const hyset_join_opts* o) {
+    const PairSortJob sort = pair_sort_job(P);
+    return enqueue_result(ctx, P.out, o, &sort);
 }
 
 uint64_t joined_count(const hyset_ctx* ctx) {
@@ -170,17 +174,21 @@ hyset_status read_pairs(hyset_ctx* ctx, const void* d_pairs, uint64_t count, std
 }
 
 hyset_status deliver_pairs(hyset_ctx* ctx, const JoinParams& P, const hyset_join_opts* o, hyset_result* res) {
+    return deliver_pairs(ctx, P.out, P.out.swap ? P.R.n : P.S.n, P.out.swap ? P.S.n : P.R.n, o, res);
+}
+
+hyset_status deliver_pairs(hyset_ctx* ctx, const Sink& out, uint32_t n_probe, uint32_t n_indexed,
+                           const hyset_join_opts* o, hyset_result* res) {
     if (o->count_only) return HYSET_OK;
     const bool resort = o->sort_pairs && res->count > PAIR_SORT_MAX;  // not sorted behind the join
     if (resort)
-        ST(sort_device_pairs(ctx, ctx->s_pairs.as<uint2>(), res->count, P.out.swap ? P.R.n : P.S.n,
-                             P.out.swap ? P.S.n : P.R.n));
+        ST(sort_device_pairs(ctx, ctx->s_pairs.as<uint2>(), res->count, n_probe, n_indexed));
     if (o->device_pairs) {
         if (resort) CK(cudaStreamSynchronize(ctx->stream));  // device pairs are final when the call returns
         res->device_pairs = ctx->s_pairs.p;
         return HYSET_OK;
     }
-    if (!resort && res->count <= std::min<uint64_t>(P.out.cap, EARLY_PAIRS)) {  // all of them have come with their number
+    if (!resort && res->count <= std::min<uint64_t>(out.cap, EARLY_PAIRS)) {  // all of them have come with their number
         const hyset_pair* early = static_cast<const hyset_pair*>(ctx->h_stage);
         res->pairs.assign(early, early + res->count);
     } else {

@@ -298,6 +298,8 @@ hyset_status hyset_verify_device(hyset_ctx* ctx, const hyset_coll* indexed, cons
         else ST(get_bitmaps(ctx, S, words, &sig_s));
     }
     const int count_only = opts->count_only ? 1 : 0;
+    hyset_join_opts ro = *opts;  // candidate lists' pairs are not sorted
+    ro.sort_pairs = 0;
     uint64_t cap = opts->pair_capacity ? opts->pair_capacity : (1u << 20);
     CK(ctx->s_count.ensure(16, s));
     CK(ctx->s_work.ensure(16, s));
@@ -311,9 +313,9 @@ hyset_status hyset_verify_device(hyset_ctx* ctx, const hyset_coll* indexed, cons
         CK(launch_verify_candidates(R->view(), S->view(), b->view, d_probes, d_offsets, d_candidates, n_probes, vmode,
                                     sk, ctx->s_work.as<unsigned int>(), ctx->sm_count, s, sig_r, sig_s, words));
         CK(cudaEventRecord(ctx->ek1, s));
-        unsigned long long count = 0;
-        CK(cudaMemcpyAsync(&count, ctx->s_count.p, 8, cudaMemcpyDeviceToHost, s));
+        ST(enqueue_result(ctx, sk, &ro));
         CK(cudaStreamSynchronize(s));
+        const uint64_t count = joined_count(ctx);
         float kms = 0, dms = 0;
         CK(cudaEventElapsedTime(&kms, ctx->ek0, ctx->ek1));
         CK(cudaEventElapsedTime(&dms, ctx->ev0, ctx->ek1));
@@ -326,16 +328,8 @@ hyset_status hyset_verify_device(hyset_ctx* ctx, const hyset_coll* indexed, cons
         cap = count + count / 8 + 1024;
         if (attempt == 1) return fail(ctx, HYSET_E_OVERFLOW, "pair buffer overflow after resize");
     }
-    if (!count_only && opts->device_pairs) {
-        res->device_pairs = ctx->s_pairs.p;
-    } else if (!count_only) {
-        res->pairs.resize(res->count);
-        if (res->count)
-            CK(cudaMemcpyAsync(res->pairs.data(), ctx->s_pairs.p, res->count * sizeof(hyset_pair),
-                               cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        res->has_pairs = 1;
-    }
+    ST(deliver_pairs(ctx, Sink{nullptr, nullptr, count_only ? 0ull : (unsigned long long)cap, count_only, 0}, 0, 0, &ro,
+                     res.get()));
     res->technique = words ? HYSET_TECH_BITMAP : HYSET_TECH_DIRECT;
     *out = res.release();
     return HYSET_OK;

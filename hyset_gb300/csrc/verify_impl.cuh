@@ -79,39 +79,33 @@ __device__ __forceinline__ void verify_probe_list(const CollView& R, const CollV
     const uint32_t* pg = S.tokens + pm.x;
     const uint32_t* a = pg;
     bool staged = false;
-    uint64_t ps[W > 0 ? W : 1];
-    if constexpr (W > 0) {
-#pragma unroll
-        for (int w = 0; w < W; ++w) ps[w] = __ldg(sig_S + (uint64_t)p * W + w);
-    }
     for (uint32_t k0 = 0; k0 < n; k0 += 32) {
         const uint32_t k = k0 + lane;
         bool keep = k < n;
         uint32_t c = 0, lc = 0, mo = 0, cs = 0;
         if (keep) {
             c = cand_at(k);
-            const uint2 cm = R.meta[c];
-            cs = cm.x;
-            lc = cm.y;
+            uint32_t pop = 0;
+            if constexpr (W > 0) {  // start, size and folded signature in one sector
+                const SigHead h = sig_head<W>(sig_heads(sig_S, S.n, W) + (uint64_t)p * 8,
+                                              sig_heads(sig_R, R.n, W) + (uint64_t)c * 8);
+                cs = h.start;
+                lc = h.size;
+                pop = h.pop;
+            } else {
+                const uint2 cm = R.meta[c];
+                cs = cm.x;
+                lc = cm.y;
+            }
             // hybrid_kernels.hpp:50: minoverlap(probe, candidate), for any pair
             // (an incompatible length pair gets min(lp, lc)).
             const uint32_t big = max(lp, lc), small = min(lp, lc);
             if (small >= B.minsize[big]) mo = minoverlap(B, big, small);
             else mo = small;
             if constexpr (W > 0) {
-                uint32_t pop = 0;
-                const uint64_t* bc = sig_R + (uint64_t)c * W;
-                if constexpr (W % 2 == 0) {
-#pragma unroll
-                    for (int w = 0; w < W; w += 2) {
-                        const ulonglong2 y = __ldg(reinterpret_cast<const ulonglong2*>(bc + w));
-                        pop += __popcll(ps[w] ^ y.x) + __popcll(ps[w + 1] ^ y.y);
-                    }
-                } else {
-#pragma unroll
-                    for (int w = 0; w < W; ++w) pop += __popcll(ps[w] ^ __ldg(bc + w));
-                }
-                keep = lp + lc - pop >= 2u * mo;
+                const uint32_t most = lp + lc - 2u * mo;
+                keep = pop <= most &&
+                       sig_rest<W>(sig_S + (uint64_t)p * W, sig_R + (uint64_t)c * W, most);
             }
         }
         if constexpr (W > 0) {
@@ -126,25 +120,15 @@ __device__ __forceinline__ void verify_probe_list(const CollView& R, const CollV
             staged = true;
         }
         // Long merges (both sets of at least VLONG tokens) run on the whole
-        // warp in 32-token steps: a lane-serial merge of two similar sets of
-        // 2,000 tokens holds its warp for about 4,000 dependent steps, and
-        // one such pair at the end of a launch was its tail.
-        const bool lng = VMODE != 2 && keep && min(lp, lc) >= VLONG;
-        if (VMODE != 2) {
-            unsigned ml = __ballot_sync(FULL, lng);
-            while (ml) {
-                const int src = __ffs(ml) - 1;
-                ml &= ml - 1;
-                const uint32_t cc = __shfl_sync(FULL, c, src), c2 = __shfl_sync(FULL, cs, src);
-                const uint32_t ll = __shfl_sync(FULL, lc, src), mm = __shfl_sync(FULL, mo, src);
-                const bool ok = verify_warp(a, lp, R.tokens + c2, ll, mm, NOWN, lane);
-                emit(out, ok && lane == 0, p, cc, lane);
-            }
-            keep = keep && !lng;
-        }
+        // warp: a lane-serial merge of two similar sets of 2,000 tokens holds
+        // its warp for about 4,000 dependent steps, and one such pair at the
+        // end of a launch was its tail.  (Lanes that merge up to 768 steps first
+        // and leave the rest to the warp: 302 us for 131,072 x 32 candidates
+        // against 295 with every long pair on the warp from the start.)
+        const bool whole = keep && (VMODE == 2 || min(lp, lc) >= VLONG);
+        bool ok = false;
         if constexpr (VMODE == 1) {
-            bool ok = keep && verify_serial(a, lp, R.tokens + cs, lc, mo, NOWN);
-            emit(out, ok, p, c, lane);
+            if (keep && !whole) ok = verify_serial(a, lp, R.tokens + cs, lc, mo, NOWN);
         } else if constexpr (VMODE == 3) {
             // the first VSTAGE tokens of the round's 32 candidates arrive with
             // VSTAGE coalesced loads (32 / VSTAGE candidates per load, VSTAGE
@@ -160,22 +144,18 @@ __device__ __forceinline__ void verify_probe_list(const CollView& R, const CollV
                 if (t < lj) tile[j * VSTRIDE + t] = __ldg(R.tokens + cj + t);
             }
             __syncwarp();
-            const bool ok = keep && verify_staged(a, lp, tile + lane * VSTRIDE, R.tokens + cs, lc, mo);
+            if (keep && !whole) ok = verify_staged(a, lp, tile + lane * VSTRIDE, R.tokens + cs, lc, mo);
             __syncwarp();
-            emit(out, ok, p, c, lane);
-        } else {
-            unsigned m = __ballot_sync(FULL, keep);
-            while (m) {
-                int src = __ffs(m) - 1;
-                m &= m - 1;
-                uint32_t cc = __shfl_sync(FULL, c, src);
-                uint32_t c2 = __shfl_sync(FULL, cs, src);
-                uint32_t ll = __shfl_sync(FULL, lc, src);
-                uint32_t mm = __shfl_sync(FULL, mo, src);
-                bool ok = verify_warp(a, lp, R.tokens + c2, ll, mm, NOWN, lane);
-                emit(out, ok && lane == 0, p, cc, lane);
-            }
         }
+        unsigned m = __ballot_sync(FULL, whole);
+        while (m) {
+            const int src = __ffs(m) - 1;
+            m &= m - 1;
+            const uint32_t c2 = __shfl_sync(FULL, cs, src), ll = __shfl_sync(FULL, lc, src);
+            const bool is = verify_warp(a, lp, R.tokens + c2, ll, __shfl_sync(FULL, mo, src), NOWN, lane);
+            if (lane == src) ok = is;
+        }
+        emit(out, ok, p, c, lane);
     }
     __syncwarp();
 }
