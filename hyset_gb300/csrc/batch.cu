@@ -16,22 +16,30 @@ namespace hs {
 
 namespace {
 
+// Unit u of a join: a prefix-index join's longest probes go as slot segments
+// first (JoinParams::heavy_from), then its probe batches; a window technique's
+// units are single probes.  Items are carried across a unit's slot rounds.
 template <int W>
-__device__ __forceinline__ void run_unit_words(const BatchDesc& d, uint32_t i0, uint32_t k, uint32_t* sbuf, int lane) {
+__device__ __forceinline__ void run_unit(const BatchDesc& d, uint32_t u, uint32_t* sbuf, int lane) {
+    const JoinParams& P = d.P;
+    const uint32_t nprobe = P.p_hi - P.p_lo;
     if (d.tech == TECH_FGSS) {
-        fgss_batch<1, W, false, false>(d.P, i0, k, lane);  // batches index by lists
+        const uint32_t hf = max(P.heavy_from, P.p_lo), nheavy = P.p_hi > hf ? P.p_hi - hf : 0u;
+        uint32_t i0, k, jb = 0, je = 0xFFFFFFFFu;
+        if (u < nheavy * P.segs) {
+            i0 = u / P.segs;
+            k = 1;
+            jb = (u - i0 * P.segs) * P.seg_slots;
+            je = jb + P.seg_slots;
+        } else {
+            i0 = nheavy + (u - nheavy * P.segs) * d.unit_probes;
+            k = min(d.unit_probes, nprobe - i0);
+        }
+        ItemCarry ic;
+        fgss_carry<1, W, false, false>(P, i0, k, lane, ic, jb, je);
+        flush_items<1, W, false, false>(P, ic, lane);
     } else {
-        for (uint32_t i = i0; i < i0 + k; ++i) enum_probe<1, W, false>(d.P, d.P.p_hi - 1 - i, sbuf, lane);
-    }
-}
-
-__device__ __forceinline__ void run_unit(const BatchDesc& d, uint32_t i0, uint32_t k, uint32_t* sbuf, int lane) {
-    switch (d.words) {
-    case 1: run_unit_words<1>(d, i0, k, sbuf, lane); break;
-    case 2: run_unit_words<2>(d, i0, k, sbuf, lane); break;
-    case 4: run_unit_words<4>(d, i0, k, sbuf, lane); break;
-    case 8: run_unit_words<8>(d, i0, k, sbuf, lane); break;
-    default: run_unit_words<0>(d, i0, k, sbuf, lane); break;
+        enum_probe<1, W, false>(P, P.p_hi - 1 - u, sbuf, lane);
     }
 }
 
@@ -54,10 +62,14 @@ __global__ void __launch_bounds__(JOIN_THREADS, HS_JOIN_MIN_BLOCKS) k_batch_join
             else hi = mid;
         }
         const BatchDesc& d = D[lo];
-        const uint32_t nprobe = d.P.p_hi - d.P.p_lo;
-        const uint32_t i0 = (u - unit_off[lo]) * d.unit_probes;
-        const uint32_t k = min(d.unit_probes, nprobe - i0);
-        run_unit(d, i0, k, sbuf, lane);
+        u -= unit_off[lo];
+        switch (d.words) {
+        case 1: run_unit<1>(d, u, sbuf, lane); break;
+        case 2: run_unit<2>(d, u, sbuf, lane); break;
+        case 4: run_unit<4>(d, u, sbuf, lane); break;
+        case 8: run_unit<8>(d, u, sbuf, lane); break;
+        default: run_unit<0>(d, u, sbuf, lane); break;
+        }
     }
 }
 

@@ -37,7 +37,7 @@ void release_plan(hyset_ctx* ctx, BatchPlan& bp) {
     }
     DevBuf* bufs[] = {&bp.desc, &bp.unit_off, &bp.counts, &bp.work, &bp.sorts};
     for (DevBuf* d : bufs) d->release(s);
-    bp.sc.release(s);
+    for (Scratch& sc : bp.sc) sc.release(s);
     cudaStreamSynchronize(s);
 }
 }  // namespace
@@ -49,29 +49,95 @@ void batch_release(hyset_ctx* ctx) {
 }
 
 namespace {
+// The index build and signatures of many small joins are some fifteen kernels
+// each that fill a few SMs for 5-10 us: one after the other they took as long
+// as the joins (24 joins of up to 30,000 sets: 280 kernels, 2.0 of 4.5 ms).
+// They are captured on MAX_BRANCHES parallel branches of the graph, each with
+// a scratch of its own, together at most BRANCH_BYTES (one branch for joins
+// whose scratch alone is larger: their kernels fill the GPU).  That batch with
+// 1 / 4 / 8 / 16 branches: 2.92 / 2.13 / 2.02 / 1.87 ms a call.
+constexpr uint32_t MAX_BRANCHES = 16;
+constexpr size_t BRANCH_BYTES = 2ull << 30;
+
+// While it lives, the context's stream and scratch are a branch's.
+struct OnBranch {
+    hyset_ctx* ctx;
+    cudaStream_t stream;
+    Scratch* sc;
+    OnBranch(hyset_ctx* c, cudaStream_t s, Scratch* scratch) : ctx(c), stream(c->stream), sc(c->sc) {
+        ctx->stream = s;
+        ctx->sc = scratch;
+    }
+    ~OnBranch() {
+        ctx->stream = stream;
+        ctx->sc = sc;
+    }
+};
+
+hyset_status side_streams(hyset_ctx* ctx, size_t n) {
+    while (ctx->side.size() < n) {
+        cudaStream_t b = nullptr;
+        CK(cudaStreamCreateWithFlags(&b, cudaStreamNonBlocking));
+        ctx->side.push_back(b);
+    }
+    while (ctx->side_ev.size() < n) {
+        cudaEvent_t e = nullptr;
+        CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        ctx->side_ev.push_back(e);
+    }
+    return HYSET_OK;
+}
+
+// A join's index and signatures on the context's stream; a signature-technique
+// join runs there too (k_window over its own launch: in the shared launch each
+// of its probes was a unit that one warp walked).
+hyset_status build_batch_join(hyset_ctx* ctx, BatchPlan& bp, uint32_t k) {
+    BatchJoin& bj = *bp.joins[bp.order[k]];
+    if (bj.ktech == TECH_FGSS) {
+        ST(build_sorted_index(ctx, bj.R, bj.b, bj.self ? 0 : 1, bj.ix, nullptr, nullptr, -1, bj.solo));
+        if (use_bands(bj.b, bj.self))
+            ST(build_sorted_index(ctx, bj.R, bj.b, 2, bj.ix_mid, &bj.b->mid_prefix, bj.b->view.mid_prefix,
+                                  (int)bj.ix.pos_bits, bj.solo));
+    }
+    if (bj.words) {
+        CK(generate_signatures(bj.R, bj.words, bj.bits_r.as<uint64_t>(), ctx->stream));
+        if (!bj.self) CK(generate_signatures(bj.S, bj.words, bj.bits_s.as<uint64_t>(), ctx->stream));
+    }
+    if (bj.window) {
+        JoinParams P = bp.host_desc[k].P;
+        P.work = bp.work.as<unsigned int>() + 4 + 4 * k;
+        split_window(bj.R, bj.S, bj.b, bj.words, P);
+        CK(launch_join(P, TECH_BITMAP, 1, ctx->sm_count, ctx->stream));
+    }
+    return HYSET_OK;
+}
+
 // The device work of a batch: per join its index build and signatures, then
 // one persistent launch over the units of every join.  Asynchronous only.
 hyset_status batch_record(hyset_ctx* ctx, BatchPlan& bp) {
     cudaStream_t s = ctx->stream;
     const uint32_t n = (uint32_t)bp.joins.size();
     CK(cudaMemsetAsync(bp.counts.p, 0, n * sizeof(unsigned long long), s));
-    CK(cudaMemsetAsync(bp.work.p, 0, 16 + 8 * (size_t)n, s));
-    for (auto& bjp : bp.joins) {
-        BatchJoin& bj = *bjp;
-        if (bj.ktech == TECH_FGSS) {
-            ST(build_sorted_index(ctx, bj.R, bj.b, bj.self ? 0 : 1, bj.ix, nullptr, nullptr, -1, bj.solo));
-            if (use_bands(bj.b, bj.self))
-                ST(build_sorted_index(ctx, bj.R, bj.b, 2, bj.ix_mid, &bj.b->mid_prefix, bj.b->view.mid_prefix,
-                                      (int)bj.ix.pos_bits, bj.solo));
-        }
-        if (bj.words) {
-            CK(generate_signatures(bj.R, bj.words, bj.bits_r.as<uint64_t>(), s));
-            if (!bj.self) CK(generate_signatures(bj.S, bj.words, bj.bits_s.as<uint64_t>(), s));
+    CK(cudaMemsetAsync(bp.work.p, 0, 16 + 16 * (size_t)n, s));
+    const uint32_t branches = (uint32_t)bp.sc.size();
+    if (branches == 1) {
+        OnBranch on(ctx, s, &bp.sc[0]);
+        for (uint32_t k = 0; k < n; ++k) ST(build_batch_join(ctx, bp, k));
+    } else {
+        CK(cudaEventRecord(ctx->ev_fork, s));
+        for (uint32_t k = 0; k < branches; ++k) {
+            CK(cudaStreamWaitEvent(ctx->side[k], ctx->ev_fork, 0));
+            {
+                OnBranch on(ctx, ctx->side[k], &bp.sc[k]);
+                for (uint32_t q = 0; q < n; ++q)
+                    if (bp.branch[bp.order[q]] == k) ST(build_batch_join(ctx, bp, q));
+            }
+            CK(cudaEventRecord(ctx->side_ev[k], ctx->side[k]));
+            CK(cudaStreamWaitEvent(s, ctx->side_ev[k], 0));
         }
     }
     // the solo joins, heaviest first, each with the single-join kernel over its
     // own index (token records when its lists fit them), then the shared launch
-    uint32_t q = 0;
     for (uint32_t k = 0; k < n; ++k) {
         BatchJoin& bj = *bp.joins[bp.order[k]];
         if (!bj.solo) continue;
@@ -80,7 +146,7 @@ hyset_status batch_record(hyset_ctx* ctx, BatchPlan& bp) {
         if (use_bands(bj.b, bj.self)) P.X2 = bj.ix_mid.view();
         P.grab = std::min<uint32_t>(bj.batch, P.X2.set ? 16u : 32u);
         split_heavy(bj.S, bj.b, P);
-        P.work = bp.work.as<unsigned int>() + 4 + 2 * q++;
+        P.work = bp.work.as<unsigned int>() + 4 + 4 * k;
         CK(launch_join(P, TECH_FGSS, bj.vmode, ctx->sm_count, s));
     }
     CK(launch_batch_join(bp.desc.as<BatchDesc>(), bp.unit_off.as<uint32_t>(), n, bp.work.as<unsigned int>(),
@@ -99,17 +165,11 @@ hyset_status batch_prepare(hyset_ctx* ctx, const hyset_join_desc* joins, uint32_
         if (plan) release_plan(ctx, *plan);
     });
     plan->sig = sig;
-    // index builds of the batch use the plan's own scratch, so later joins that
-    // grow the context's scratch cannot free memory the graph still addresses
-    struct ScratchSwitch {
-        hyset_ctx* c;
-        ~ScratchSwitch() { c->sc = &c->own; }
-    } sw{ctx};
-    ctx->sc = &plan->sc;
     cudaStream_t s = ctx->stream;
     std::vector<BatchDesc> desc(n);
     std::vector<double> cost(n);
     uint64_t maxE = 1, maxU = 1, maxN = 1;
+    std::vector<double> build(n, 0.0);  // entries to index and tokens to sign
     for (uint32_t j = 0; j < n; ++j) {
         const hyset_join_desc& d = joins[j];
         if (!d.indexed) return fail(ctx, HYSET_E_INVALID, "batch join without an indexed collection");
@@ -172,6 +232,7 @@ hyset_status batch_prepare(hyset_ctx* ctx, const hyset_join_desc* joins, uint32_
             const uint64_t E = prefix_entries(R, bj->b->index_prefix);
             if (E >= (1ull << 32)) return fail(ctx, HYSET_E_UNSUPPORTED, "more than 2^32 prefix entries");
             maxE = std::max<uint64_t>(maxE, E);
+            build[j] = 4.0 * (double)E;
             maxU = std::max<uint64_t>(maxU, (uint64_t)R->universe + 1);
             maxN = std::max<uint64_t>(maxN, R->n);
             CK(bj->ix.list_off.ensure(((size_t)R->universe + 1) * 4, s));
@@ -209,31 +270,57 @@ hyset_status batch_prepare(hyset_ctx* ctx, const hyset_join_desc* joins, uint32_
         bj->unit_probes = bj->ktech == TECH_FGSS ? desc[j].unit_probes : 0;
         bj->batch = desc[j].unit_probes;
         const uint32_t np = P.p_hi - P.p_lo;
-        bj->units = bj->solo ? 0u : (np + desc[j].unit_probes - 1) / desc[j].unit_probes;
+        uint32_t nheavy = 0;  // probes taken as slot segments
+        if (bj->ktech == TECH_FGSS) {
+            split_heavy(S, bj->b, P);
+            const uint32_t hf = std::max(P.heavy_from, P.p_lo);
+            nheavy = P.p_hi > hf ? P.p_hi - hf : 0u;
+        }
+        bj->window = bj->ktech == TECH_BITMAP && bj->words > 0;
+        bj->units = bj->solo || bj->window ? 0u : nheavy * P.segs + (np - nheavy + desc[j].unit_probes - 1) / desc[j].unit_probes;
+        if (bj->ktech == TECH_BITMAP) build[j] += (double)np * (double)R->n / 64.0;  // its pairs, at a token's cost each 64
+        if (bj->words) build[j] += (double)R->n_tokens + (bj->self ? 0.0 : (double)S->n_tokens);
         cost[j] = (double)np * (double)(R->n_tokens / std::max<uint32_t>(R->n, 1) + 1) *
                   (bj->ktech == TECH_FGSS ? 1.0 : (double)R->n);
     }
-    // scratch for the largest index build, sized before capture
-    CK(ctx->sc->len.ensure((size_t)maxN * 4 + 4, s));
-    CK(ctx->sc->off.ensure((size_t)maxN * 4 + 4, s));
+    // index builds of the batch use the plan's own scratch, so later joins that
+    // grow the context's scratch cannot free memory the graph still addresses;
+    // every branch's holds the largest index build, sized before the capture
     const size_t e4 = (size_t)maxE * 4;
-    CK(ctx->sc->tok.ensure(e4, s));
-    CK(ctx->sc->set.ensure(e4, s));
-    CK(ctx->sc->pos.ensure(e4, s));
-    CK(ctx->sc->order.ensure(e4, s));
-    CK(ctx->sc->altk.ensure(e4, s));
-    CK(ctx->sc->altv.ensure(e4, s));
-    CK(ctx->sc->gate.ensure(4, s));
-    CK(ctx->sc->counts.ensure((size_t)maxU * 4, s));
     const size_t scan_words = std::max(std::max(scan_scratch_words(maxN), scan_scratch_words(maxU)),
                                        radix_scratch_words(maxE));
-    CK(ctx->sc->scan.ensure(scan_words * 4, s));
+    const size_t per_branch = 8 * (size_t)maxN + 6 * e4 + 4 * ((size_t)maxU + scan_words);
+    const uint32_t branches =
+        std::max<uint32_t>(1, (uint32_t)std::min<uint64_t>({MAX_BRANCHES, n, (uint64_t)(BRANCH_BYTES / per_branch)}));
+    ST(side_streams(ctx, branches));
+    plan->sc.resize(branches);
+    for (Scratch& sc : plan->sc) {
+        CK(sc.len.ensure((size_t)maxN * 4 + 4, s));
+        CK(sc.off.ensure((size_t)maxN * 4 + 4, s));
+        for (DevBuf* d : {&sc.tok, &sc.set, &sc.pos, &sc.order, &sc.altk, &sc.altv}) CK(d->ensure(e4, s));
+        CK(sc.gate.ensure(4, s));
+        CK(sc.counts.ensure((size_t)maxU * 4, s));
+        CK(sc.scan.ensure(scan_words * 4, s));
+    }
+    // each join to the branch with the least to build, the largest first
+    plan->branch.assign(n, 0);
+    {
+        std::vector<uint32_t> by(n);
+        for (uint32_t j = 0; j < n; ++j) by[j] = j;
+        std::stable_sort(by.begin(), by.end(), [&](uint32_t a, uint32_t b) { return build[a] > build[b]; });
+        std::vector<double> load(branches, 0.0);
+        for (uint32_t j : by) {
+            const uint32_t k = (uint32_t)(std::min_element(load.begin(), load.end()) - load.begin());
+            plan->branch[j] = k;
+            load[k] += build[j] + 2e5;  // its launches, whatever its size
+        }
+    }
     // heaviest joins first, so the tail of the launch is light
     plan->order.resize(n);
     for (uint32_t j = 0; j < n; ++j) plan->order[j] = j;
     std::stable_sort(plan->order.begin(), plan->order.end(), [&](uint32_t a, uint32_t b) { return cost[a] > cost[b]; });
     CK(plan->counts.ensure(n * sizeof(unsigned long long), s));
-    CK(plan->work.ensure(16 + 8 * (size_t)n, s));  // the shared launch's counter, then two per solo join
+    CK(plan->work.ensure(16 + 16 * (size_t)n, s));  // the shared launch's counter, then four for every join's own
     std::vector<BatchDesc> ordered(n);
     std::vector<uint32_t> unit_off(n + 1, 0);
     std::vector<PairSortJob> sorts;
@@ -263,6 +350,7 @@ hyset_status batch_prepare(hyset_ctx* ctx, const hyset_join_desc* joins, uint32_
     // indexes whose list path is not known yet are built once here, outside
     // the capture, so that the path is read back and remembered: the graph then
     // holds only the kernels of the path each index takes
+    OnBranch first(ctx, s, &bp.sc[0]);
     for (auto& bjp : bp.joins) {
         BatchJoin& bj = *bjp;
         if (bj.ktech != TECH_FGSS) continue;

@@ -125,6 +125,11 @@ void hyset_destroy(hyset_ctx* ctx) {
         cudaStreamSynchronize(ctx->aux);
         cudaStreamDestroy(ctx->aux);
     }
+    for (cudaStream_t b : ctx->side) {
+        cudaStreamSynchronize(b);
+        cudaStreamDestroy(b);
+    }
+    for (cudaEvent_t e : ctx->side_ev) cudaEventDestroy(e);
     if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
     for (cudaEvent_t e : ctx->pipe_ev) cudaEventDestroy(e);
     if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);

@@ -130,6 +130,7 @@ struct BatchJoin {
     // graph (the single-join kernel: token records, carried items), not in the
     // shared launch
     bool solo = false;
+    bool window = false;  // a signature-technique join: a launch of its own on its branch of the graph
     int vmode = 1;
     uint32_t batch = 3;
 };
@@ -148,7 +149,8 @@ struct Scratch {
 // device descriptors, and the instantiated graph of its device work.
 struct BatchPlan {
     std::vector<std::string> sig;
-    Scratch sc;  // owned by the plan: its graph holds these addresses
+    std::vector<Scratch> sc;  // a branch each; owned by the plan: its graph holds these addresses
+    std::vector<uint32_t> branch;  // joins[j] builds its index and signatures on this branch
     std::vector<std::unique_ptr<BatchJoin>> joins;
     std::vector<uint32_t> order;  // joins[order[k]] is descriptor k (heaviest first)
     DevBuf desc, unit_off, counts, work, sorts;
@@ -167,6 +169,8 @@ struct hyset_ctx {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ek0 = nullptr, ek1 = nullptr;
     cudaStream_t aux = nullptr;                         // work that overlaps the index build
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;  // fork to / join from aux
+    std::vector<cudaStream_t> side;                     // branches of a batch's graph, created on demand
+    std::vector<cudaEvent_t> side_ev;                   // one per branch: its end
     std::vector<cudaEvent_t> pipe_ev;                   // one per copy chunk of a host-input join
     std::string err;
     std::map<std::tuple<int, double, uint32_t, int>, std::unique_ptr<hs::Bounds>> bounds;

@@ -26,10 +26,6 @@
 #include "join_impl.cuh"
 #include "verify_impl.cuh"
 
-#ifndef HS_ITEM_CARRY
-#define HS_ITEM_CARRY 1  // probe-major FGSS: items carried until a round of 32 is full (fgss_carry)
-#endif
-
 namespace hs {
 
 namespace {
@@ -44,11 +40,11 @@ __global__ void __launch_bounds__(JOIN_THREADS, HS_JOIN_MIN_BLOCKS) k_join(JoinP
     const uint32_t nprobe = P.p_hi - P.p_lo;
     const uint32_t grab = P.grab ? P.grab : 1;
     uint32_t i = 0, i_end = 0;
-    ItemCarry ic;  // FGSS with HS_ITEM_CARRY: items pending across slot rounds and batches
+    ItemCarry ic;  // FGSS: items pending across slot rounds and batches
     ic.q = sbuf;   // its queue for bound-layout indexes (QSLOTS * QF_N <= MAXP words)
     static_assert(QSLOTS * QF_N <= MAXP, "item queue exceeds the warp's shared-memory slot");
     uint32_t nheavy = 0;  // the longest probes (the first from the top) go as slot segments, one per steal
-    if constexpr (TECH == TECH_FGSS && HS_ITEM_CARRY) {
+    if constexpr (TECH == TECH_FGSS) {
         const uint32_t hf = max(P.heavy_from, P.p_lo);
         nheavy = P.p_hi > hf ? P.p_hi - hf : 0u;
         const uint32_t units = nheavy * P.segs;
@@ -72,14 +68,13 @@ __global__ void __launch_bounds__(JOIN_THREADS, HS_JOIN_MIN_BLOCKS) k_join(JoinP
         const uint32_t end = min(i_end, i + grab);
         // largest sets first: the heaviest probes start early, the tail is light
         if constexpr (TECH == TECH_FGSS) {
-            if constexpr (HS_ITEM_CARRY) fgss_carry<VMODE, W, ST, BD>(P, i, end - i, lane, ic);
-            else fgss_batch<VMODE, W, ST, true, BD>(P, i, end - i, lane);
+            fgss_carry<VMODE, W, ST, BD>(P, i, end - i, lane, ic);
         } else {
             for (uint32_t q = i; q < end; ++q) enum_probe<VMODE, W, ST>(P, P.p_hi - 1 - q, sbuf, lane);
         }
         i = end;
     }
-    if constexpr (TECH == TECH_FGSS && HS_ITEM_CARRY) flush_items<VMODE, W, ST, BD>(P, ic, lane);
+    if constexpr (TECH == TECH_FGSS) flush_items<VMODE, W, ST, BD>(P, ic, lane);
 }
 
 #ifndef HS_VREVERSE
