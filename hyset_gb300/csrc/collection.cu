@@ -31,6 +31,8 @@ hyset_status host_stage(hyset_ctx* ctx, size_t bytes, void** out) {
     return HYSET_OK;
 }
 
+constexpr uint32_t SIZE_RUNS = 8192;  // distinct sizes whose runs are read back (64 KB)
+
 // Enqueues the checks of a new collection (one pass over the tokens, which also
 // writes the meta pairs) and the read-back of their flags (and of the sizes,
 // when they are only on the device).  With host sizes the histogram work runs
@@ -38,9 +40,15 @@ hyset_status host_stage(hyset_ctx* ctx, size_t bytes, void** out) {
 hyset_status enqueue_collection_checks(hyset_ctx* ctx, hyset_coll* c, const uint32_t* h_sizes_or_null) {
     cudaStream_t s = ctx->stream;
     if (!h_sizes_or_null && c->n) {
+        // sizes on the device: their runs of equal values come back, not the sizes
+        // (a host pass over a million of them takes 1.4 ms on a Grace core)
+        constexpr size_t BYTES = 8 + (size_t)SIZE_RUNS * 8;
         void* stage = nullptr;
-        ST(host_stage(ctx, (size_t)c->n * 4, &stage));
-        CK(cudaMemcpyAsync(stage, c->d_sizes, (size_t)c->n * 4, cudaMemcpyDeviceToHost, s));
+        ST(host_stage(ctx, BYTES, &stage));
+        CK(ctx->s_runs.ensure(BYTES, s));
+        CK(cudaMemsetAsync(ctx->s_runs.p, 0, 8, s));
+        CK(size_runs(c->d_sizes, c->n, ctx->s_runs.as<uint32_t>(), SIZE_RUNS, s));
+        CK(cudaMemcpyAsync(stage, ctx->s_runs.p, BYTES, cudaMemcpyDeviceToHost, s));
     }
     CK(ctx->s_flags.ensure(16, s));
     CK(cudaMemsetAsync(ctx->s_flags.p, 0, 16, s));
@@ -63,9 +71,16 @@ hyset_status finish_collection_checks(hyset_ctx* ctx, hyset_coll* c, const uint3
     if (f[0] & 4) return fail(ctx, HYSET_E_INVALID, "sets must be ordered by non-decreasing size");
     if (f[1] == 0xFFFFFFFFu) return fail(ctx, HYSET_E_INVALID, "token 0xFFFFFFFF is reserved");
     c->universe = c->n ? f[1] + 1 : 1;
-    if (!h_sizes_or_null || !c->n)
-        ST(build_size_meta(ctx, c, c->n ? static_cast<const uint32_t*>(ctx->h_stage) : nullptr));
-    return HYSET_OK;
+    if (!c->n) return build_size_meta(ctx, c, nullptr);
+    if (h_sizes_or_null) return HYSET_OK;
+    const uint32_t* runs = static_cast<const uint32_t*>(ctx->h_stage);
+    if (runs[0] <= SIZE_RUNS) return build_size_meta_runs(ctx, c, runs + 2, runs[0]);
+    // more sizes than the runs' buffer holds: the host goes through all of them
+    void* stage = nullptr;
+    ST(host_stage(ctx, (size_t)c->n * 4, &stage));
+    CK(cudaMemcpyAsync(stage, c->d_sizes, (size_t)c->n * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    return build_size_meta(ctx, c, static_cast<const uint32_t*>(stage));
 }
 
 hyset_status make_collection(hyset_ctx* ctx, hyset_coll* c, const uint32_t* h_sizes_or_null) {

@@ -60,6 +60,8 @@ hyset_status make_collection(hyset_ctx* ctx, hyset_coll* c, const uint32_t* h_si
 
 // ---- index builds and size statistics (index_host.cu) ------------------------
 hyset_status build_size_meta(hyset_ctx* ctx, hyset_coll* c, const uint32_t* sizes);
+// The same from the n_runs runs of equal sizes: (size, first set) pairs in any order.
+hyset_status build_size_meta_runs(hyset_ctx* ctx, hyset_coll* c, const uint32_t* runs, uint32_t n_runs);
 // The host side of the size metadata (max_size, size_hist, h_first_ge) from a
 // first_ge table computed on the device (c->first_ge holds it already).
 void size_meta_from_first_ge(hyset_coll* c, const uint32_t* first_ge, uint32_t L);

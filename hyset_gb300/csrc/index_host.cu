@@ -18,6 +18,24 @@ namespace hs {
 // enqueued on the stream (the host array is a member, so no synchronisation is
 // needed here).  The collection keeps no per-set host array: sizes of single
 // sets and of id ranges come from first_ge.
+namespace {
+// first_ge (and its device copy) and the largest size from the histogram.
+hyset_status finish_size_meta(hyset_ctx* ctx, hyset_coll* c) {
+    const uint32_t L = (uint32_t)c->size_hist.size() - 1;
+    c->max_size = L;
+    std::vector<uint32_t>& f = c->h_first_ge;
+    f.resize((size_t)L + 2);
+    uint64_t run = 0;
+    for (uint32_t l = 0; l <= L + 1; ++l) {
+        f[l] = (uint32_t)run;
+        if (l <= L) run += c->size_hist[l];
+    }
+    CK(c->first_ge.ensure(f.size() * 4, ctx->stream));
+    CK(cudaMemcpyAsync(c->first_ge.p, f.data(), f.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
+    return HYSET_OK;
+}
+}  // namespace
+
 hyset_status build_size_meta(hyset_ctx* ctx, hyset_coll* c, const uint32_t* sizes) {
     std::vector<uint64_t>& hist = c->size_hist;
     hist.assign(c->n ? (size_t)sizes[c->n - 1] + 1 : 1, 0);
@@ -31,18 +49,17 @@ hyset_status build_size_meta(hyset_ctx* ctx, hyset_coll* c, const uint32_t* size
         hist[v] += j - i;
         i = j;
     }
-    const uint32_t L = (uint32_t)hist.size() - 1;
-    c->max_size = L;
-    std::vector<uint32_t>& f = c->h_first_ge;
-    f.resize((size_t)L + 2);
-    uint64_t run = 0;
-    for (uint32_t l = 0; l <= L + 1; ++l) {
-        f[l] = (uint32_t)run;
-        if (l <= L) run += c->size_hist[l];
-    }
-    CK(c->first_ge.ensure(f.size() * 4, ctx->stream));
-    CK(cudaMemcpyAsync(c->first_ge.p, f.data(), f.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
-    return HYSET_OK;
+    return finish_size_meta(ctx, c);
+}
+
+hyset_status build_size_meta_runs(hyset_ctx* ctx, hyset_coll* c, const uint32_t* runs, uint32_t n_runs) {
+    std::vector<std::pair<uint32_t, uint32_t>> by(n_runs);  // (first set, size): sizes are non-decreasing
+    for (uint32_t k = 0; k < n_runs; ++k) by[k] = {runs[2 * k + 1], runs[2 * k]};
+    std::sort(by.begin(), by.end());
+    c->size_hist.assign(n_runs ? (size_t)by.back().second + 1 : 1, 0);
+    for (uint32_t k = 0; k < n_runs; ++k)
+        c->size_hist[by[k].second] += (k + 1 < n_runs ? by[k + 1].first : c->n) - by[k].first;
+    return finish_size_meta(ctx, c);
 }
 
 void size_meta_from_first_ge(hyset_coll* c, const uint32_t* first_ge, uint32_t L) {

@@ -177,6 +177,7 @@ struct hyset_ctx {
     // scratch reused across joins; a batch being prepared points sc at its own
     hs::Scratch own;
     hs::Scratch* sc = &own;
+    hs::DevBuf s_runs;  // the runs of a new collection's sizes
     hs::DevBuf s_pairs, s_count, s_work, s_stats, s_flags;
     uint32_t* h_flags = nullptr;  // pinned host words for small device-to-host reads ([16..17]: a join's count)
     void* h_stage = nullptr;      // pinned staging for larger reads (grows)

@@ -212,6 +212,10 @@ cudaError_t size_scan(const uint32_t* sizes, const uint32_t* starts, bool starts
                       uint64_t n_tokens, uint32_t* out, uint32_t* first_ge, uint32_t* chunk_hi, cudaStream_t s);
 
 
+// The runs of equal sizes, in any order: out[0] their number (zeroed by the
+// caller), then from out[2] (size, first set) of the first cap of them.
+cudaError_t size_runs(const uint32_t* sizes, uint32_t n, uint32_t* out, uint32_t cap, cudaStream_t s);
+
 // The same pass writes meta[i] = (starts[i], sizes[i]).
 cudaError_t validate_collection(CollView c, uint64_t n_tokens, uint32_t* flags, uint2* meta, cudaStream_t s);
 // validate_collection and generate_bitmaps (words in {1, 2, 4, 8, 16}) in one

@@ -38,6 +38,22 @@ std::vector<uint64_t> chunk_ends(uint64_t n_tokens) {
     }
     return ends;
 }
+
+// Chunks of a text of `tiles` parser tiles copied from the host: 16 MB (32 MB
+// from pageable memory, whose copies each cost the host some work), then a third
+// of what is left, down to 4 MB (8 MB), in tiles before the end of each.
+constexpr uint64_t PARSE_TILE_BYTES = 4096;
+std::vector<uint64_t> parse_chunk_ends(uint64_t tiles, bool pinned) {
+    const uint64_t MOST = (pinned ? 16ull << 20 : 32ull << 20) / PARSE_TILE_BYTES;
+    const uint64_t LEAST = (pinned ? 4ull << 20 : 8ull << 20) / PARSE_TILE_BYTES;
+    std::vector<uint64_t> ends;
+    for (uint64_t t = 0; t < tiles;) {
+        const uint64_t left = tiles - t;
+        t += std::min(left, std::min(MOST, std::max(LEAST, left / 3)));
+        ends.push_back(t);
+    }
+    return ends;
+}
 }  // namespace
 
 cudaEvent_t pipe_event(hyset_ctx* ctx, size_t k) { return nth_event(ctx->pipe_ev, k); }
@@ -66,28 +82,39 @@ hyset_status hyset_collection_parse(hyset_ctx* ctx, const char* text, uint64_t n
     } rel{{&staged, &counts, &err}, s};
     cudaPointerAttributes attr{};
     if (cudaPointerGetAttributes(&attr, text) != cudaSuccess) cudaGetLastError();
-    // host text travels in 64 MB chunks on the auxiliary stream; the tiles of a
-    // chunk are counted once it and the next chunk (a tile reads one byte past
-    // its end) have landed, so counting overlaps the copy
-    constexpr uint64_t PARSE_CHUNK = 64ull << 20;  // a multiple of the 4 KiB tile
-    uint64_t n_chunks = 0;
-    if (n_bytes && attr.type != cudaMemoryTypeDevice && attr.type != cudaMemoryTypeManaged) {
+    // host text travels in chunks on the auxiliary stream; the tiles of a chunk
+    // are counted once it and the next chunk (a tile reads one byte past its
+    // end) have landed, so counting overlaps the copy.  The chunks are small and
+    // the last ones smaller, as the work of the last two is what the copy leaves
+    // behind: 155 MB in 64 MB chunks took 1.27 ms from pinned memory, 0.52 ms past
+    // its copy.  Copies from pageable memory may hold the host, so each of them is
+    // issued a chunk ahead of the work on the chunk before.
+    std::vector<uint64_t> ends;  // tiles before the end of each chunk
+    const bool on_host = n_bytes && attr.type != cudaMemoryTypeDevice && attr.type != cudaMemoryTypeManaged;
+    const bool pinned = attr.type == cudaMemoryTypeHost;
+    if (on_host) {
         CK(staged.ensure(n_bytes + 16, s));
         CK(cudaEventRecord(ctx->ev_fork, s));
         CK(cudaStreamWaitEvent(ctx->aux, ctx->ev_fork, 0));
-        n_chunks = (n_bytes + PARSE_CHUNK - 1) / PARSE_CHUNK;
-        for (uint64_t k = 0; k < n_chunks; ++k) {
-            const uint64_t b0 = k * PARSE_CHUNK, b1 = std::min(n_bytes, b0 + PARSE_CHUNK);
-            CK(cudaMemcpyAsync(staged.as<uint8_t>() + b0, text + b0, b1 - b0, cudaMemcpyHostToDevice, ctx->aux));
-            cudaEvent_t e = pipe_event(ctx, k);
-            if (!e) {
-                cudaStreamSynchronize(ctx->aux);
-                return fail(ctx, HYSET_E_CUDA, "event creation");
-            }
-            CK(cudaEventRecord(e, ctx->aux));
-        }
+        ends = parse_chunk_ends(parse_tiles(n_bytes), pinned);
         d_text = staged.as<uint8_t>();
     }
+    const uint64_t n_chunks = ends.size();
+    uint64_t copied = 0;  // chunks whose copy has been issued
+    auto copy_chunks = [&](uint64_t upto) -> hyset_status {
+        for (; copied < std::min(upto, n_chunks); ++copied) {
+            const uint64_t b0 = (copied ? ends[copied - 1] : 0) * PARSE_TILE_BYTES;
+            const uint64_t b1 = std::min(n_bytes, ends[copied] * PARSE_TILE_BYTES);
+            CK(cudaMemcpyAsync(staged.as<uint8_t>() + b0, text + b0, b1 - b0, cudaMemcpyHostToDevice, ctx->aux));
+            cudaEvent_t e = pipe_event(ctx, copied);
+            if (!e) return fail(ctx, HYSET_E_CUDA, "event creation");
+            CK(cudaEventRecord(e, ctx->aux));
+        }
+        return HYSET_OK;
+    };
+    auto landed = on_exit([&] {  // no return while a copy may still write the staged text
+        if (copied) cudaStreamSynchronize(ctx->aux);
+    });
     if (n_bytes && (reinterpret_cast<uintptr_t>(d_text) & 15u)) {  // tiles load 16-byte words
         DevBuf aligned;
         CK(aligned.ensure(n_bytes + 16, s));
@@ -134,16 +161,17 @@ hyset_status hyset_collection_parse(hyset_ctx* ctx, const char* text, uint64_t n
         // whole parse overlaps the copy.  The output is sized from the first
         // chunk's density (one wait); a text denser further on overflows that
         // estimate and is emitted again at its exact size.
-        const uint64_t per = PARSE_CHUNK / 4096;  // tiles per chunk
         uint32_t tok_cap = 0, line_cap = 0;
         for (uint64_t k = 0; k < n_chunks; ++k) {
+            const uint64_t t0 = k ? ends[k - 1] : 0, t1 = ends[k];
+            ST(copy_chunks(pinned ? n_chunks : k + 2));
             CK(cudaStreamWaitEvent(s, pipe_event(ctx, std::min(k + 1, n_chunks - 1)), 0));
-            CK(parse_count(d_text, n_bytes, tile_toks, tile_lines, flags, first_bad, s, k * per, (k + 1) * per));
-            CK(parse_chunk_scan(tile_toks, tile_lines, k * per, std::min(tiles, (k + 1) * per), carry, k, s));
+            CK(parse_count(d_text, n_bytes, tile_toks, tile_lines, flags, first_bad, s, t0, t1));
+            CK(parse_chunk_scan(tile_toks, tile_lines, t0, t1, carry, k, s));
             if (k == 0) {
                 CK(cudaMemcpyAsync(h + 4, carry + 2, 8, cudaMemcpyDeviceToHost, s));
                 CK(cudaStreamSynchronize(s));
-                const double scale = (double)n_bytes / (double)std::min<uint64_t>(n_bytes, PARSE_CHUNK);
+                const double scale = (double)n_bytes / (double)std::min<uint64_t>(n_bytes, t1 * PARSE_TILE_BYTES);
                 const double bound = (double)(n_bytes / 2 + 2);  // a token or a line takes two bytes
                 tok_cap = (uint32_t)std::min({bound, 1.25 * scale * h[4] + 4096.0, 4294967295.0});
                 line_cap = (uint32_t)std::min({bound, 1.25 * scale * h[5] + 4096.0, 4294967295.0});
@@ -151,7 +179,7 @@ hyset_status hyset_collection_parse(hyset_ctx* ctx, const char* text, uint64_t n
                 CK(c->starts.ensure((size_t)line_cap * 4 + 4, s));
             }
             CK(parse_emit(d_text, n_bytes, tile_toks, tile_lines, c->tokens.as<uint32_t>(), c->starts.as<uint32_t>(),
-                          flags, first_bad, s, k * per, (k + 1) * per, tok_cap, line_cap));
+                          flags, first_bad, s, t0, t1, tok_cap, line_cap));
         }
         CK(cudaMemcpyAsync(h, err.p, 16, cudaMemcpyDeviceToHost, s));
         CK(cudaMemcpyAsync(h + 4, carry + 2 * n_chunks, 8, cudaMemcpyDeviceToHost, s));
