@@ -46,10 +46,26 @@ Tuned tune(const hyset_coll* R, const hyset_coll* S, const hyset_join_opts* o, h
     t.probe_major = (o->technique == HYSET_TECH_FGSS && !o->probe_major) ? 0 : 1;
     t.batch = o->fgss_batch ? o->fgss_batch : DEFAULT_PROBE_BATCH;
     t.bits = o->bitmap_bits;
-    if (o->technique == HYSET_TECH_AUTO && t.bits == 0) t.bits = avg <= 48.0 ? 128 : 256;
+    // Signature width without timed samples: head records let the prefix filter
+    // read a wide signature only for the few pairs their folds leave in, so above
+    // a mean size of 48 its width costs nothing and 512 bits reject what 256 pass
+    // (10,000 long sets, cosine 0.8: kernel 0.57 -> 0.21 ms; means of 60 within
+    // 2 %); below, 128 bits are as good.  A window technique pays for every word
+    // of every pair.
+    if (o->technique == HYSET_TECH_AUTO && t.bits == 0) t.bits = avg <= 48.0 ? 128 : t.tech == HYSET_TECH_FGSS ? 512 : 256;
     if (t.tech == HYSET_TECH_BITMAP && t.bits == 0) t.bits = 64;
     if (t.tech == HYSET_TECH_DIRECT) t.bits = 0;
-    t.vmode = o->verify_mode ? (int)o->verify_mode : 1;
+    // Verification without timed samples: a lane per candidate, unless there are
+    // sets so long that one lane's merge of two of them outlasts a small join (a
+    // step per token, 250 cycles under load): with sets of 2,000 tokens, 512 bits,
+    // 2,000 / 10,000 / 40,000 sets at Jaccard 0.8 took 0.116 / 0.149 / 0.298 ms of
+    // kernel with lanes and 0.075 / 0.131 / 0.141 with warps (0.6: 0.174 / 0.321 /
+    // 0.399 and 0.121 / 0.266 / 0.399); with sets of up to 640 tokens lanes are as
+    // good or better.
+    constexpr uint32_t WARP_MERGE_SIZE = 1000;
+    const bool long_sets = o->technique == HYSET_TECH_AUTO && t.tech == HYSET_TECH_FGSS && t.bits >= 512 &&
+                           std::min(R->max_size, S->max_size) >= WARP_MERGE_SIZE;
+    t.vmode = o->verify_mode ? (int)o->verify_mode : long_sets ? 2 : 1;
     if (t.vmode == 3) t.vmode = 1;  // the staged mode exists for explicit candidate lists only
     return t;
 }

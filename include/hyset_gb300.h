@@ -70,11 +70,13 @@ typedef struct {
                                   window techniques, the token-major kernel and the candidate
                                   verifier use 512 for it); 0 = chosen by the library with technique
                                   AUTO (timed samples for joins of 60,000 probes or more, else
-                                  128 bits for mean set sizes <= 48 and 256 above), no signature
+                                  128 bits for mean set sizes <= 48 and 512 above, 256 for the window
+                                  techniques), no signature
                                   filter with an explicit technique */
     uint32_t count_only;       /* 1 = count result pairs, do not materialise them */
     uint32_t verify_mode;      /* 0 = auto (a lane per candidate, or a warp per candidate where
-                                  the samples that choose the signature width show it faster),
+                                  the samples that choose the signature width show it faster or,
+                                  without samples, where both sides have sets of 1,000 tokens),
                                   1 = one lane per candidate, 2 = one warp per candidate,
                                   3 = one lane per candidate from staged prefixes (explicit candidate
                                   lists; joins treat it as 1) */
