@@ -138,10 +138,12 @@ void split_heavy(const hyset_coll* S, const Bounds* b, JoinParams& P);
 // Behind a join's launch, before the host knows its number of pairs: orders
 // the pairs when asked (up to PAIR_SORT_MAX) and starts the copies of their
 // number (joined_count, after the stream has synchronised) and of the first
-// EARLY_PAIRS of them.
-constexpr uint64_t EARLY_PAIRS = 32768;  // 256 KB: under 2 us of copy
+// early_pairs of them: a sixteenth of the probes (most joins find fewer), 2,048
+// to 32,768 (256 KB cost a 70 us call 5 us).
+constexpr uint64_t EARLY_PAIRS = 32768;
+uint64_t early_pairs(uint64_t cap, uint32_t n_probe);
 PairSortJob pair_sort_job(const JoinParams& P);
-hyset_status enqueue_result(hyset_ctx* ctx, const Sink& out, const hyset_join_opts* o,
+hyset_status enqueue_result(hyset_ctx* ctx, const Sink& out, uint32_t n_probe, const hyset_join_opts* o,
                             const PairSortJob* sort = nullptr);
 hyset_status enqueue_result(hyset_ctx* ctx, const JoinParams& P, const hyset_join_opts* o);
 uint64_t joined_count(const hyset_ctx* ctx);

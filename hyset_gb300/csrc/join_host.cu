@@ -136,12 +136,17 @@ PairSortJob pair_sort_job(const JoinParams& P) {
                        (int)bits_for(P.out.swap ? P.S.n : P.R.n)};
 }
 
-hyset_status enqueue_result(hyset_ctx* ctx, const Sink& out, const hyset_join_opts* o, const PairSortJob* sort) {
+uint64_t early_pairs(uint64_t cap, uint32_t n_probe) {
+    return std::min(cap, std::min<uint64_t>(EARLY_PAIRS, std::max<uint64_t>(2048, n_probe / 16)));
+}
+
+hyset_status enqueue_result(hyset_ctx* ctx, const Sink& out, uint32_t n_probe, const hyset_join_opts* o,
+                            const PairSortJob* sort) {
     cudaStream_t s = ctx->stream;
     if (sort && !o->count_only && o->sort_pairs) CK(sort_pairs_cluster(*sort, s));
     CK(cudaMemcpyAsync(ctx->h_flags + 16, out.count, 8, cudaMemcpyDeviceToHost, s));
     if (!o->count_only && !o->device_pairs) {
-        const uint64_t early = std::min<uint64_t>(out.cap, EARLY_PAIRS);
+        const uint64_t early = early_pairs(out.cap, n_probe);
         void* stage = nullptr;
         ST(host_stage(ctx, early * sizeof(hyset_pair), &stage));
         if (early) CK(cudaMemcpyAsync(stage, out.pairs, early * sizeof(hyset_pair), cudaMemcpyDeviceToHost, s));
@@ -151,7 +156,7 @@ hyset_status enqueue_result(hyset_ctx* ctx, const Sink& out, const hyset_join_op
 
 hyset_status enqueue_result(hyset_ctx* ctx, const JoinParams& P, const hyset_join_opts* o) {
     const PairSortJob sort = pair_sort_job(P);
-    return enqueue_result(ctx, P.out, o, &sort);
+    return enqueue_result(ctx, P.out, P.out.swap ? P.R.n : P.S.n, o, &sort);
 }
 
 uint64_t joined_count(const hyset_ctx* ctx) {
@@ -188,7 +193,7 @@ hyset_status deliver_pairs(hyset_ctx* ctx, const Sink& out, uint32_t n_probe, ui
         res->device_pairs = ctx->s_pairs.p;
         return HYSET_OK;
     }
-    if (!resort && res->count <= std::min<uint64_t>(out.cap, EARLY_PAIRS)) {  // all of them have come with their number
+    if (!resort && res->count <= early_pairs(out.cap, n_probe)) {  // all of them have come with their number
         const hyset_pair* early = static_cast<const hyset_pair*>(ctx->h_stage);
         res->pairs.assign(early, early + res->count);
     } else {
