@@ -281,8 +281,11 @@ cudaError_t launch_window_w(const JoinParams& P, int sm_count, cudaStream_t s) {
     const uint64_t hcand = P.r_hi > std::max(P.r_lo, P.heavy_lo) ? P.r_hi - std::max(P.r_lo, P.heavy_lo) : 1;
     while (units(np, ncand, rest.tile, rest.seg) < 8ull * blocks && rest.seg > 1024) rest.seg /= 2;
     while (units(np, ncand, rest.tile, rest.seg) < 8ull * blocks && rest.tile > 16) rest.tile /= 2;
-    // the heavy ones' pairs are mostly verified: down to one probe (8,000 long sets
-    // at 128 bits: a thousand of them in 63 units of 16 took 0.6 ms)
+    // the heavy ones' pairs are mostly verified: down to four probes for a tail of
+    // a thirtieth of the launch, to one when there are fewer units than blocks take
+    // (8,000 long sets at 128 bits: a thousand heavy probes in 63 units of 16 took
+    // 0.6 ms; 30,000 at 64 bits, cosine 0.9: 1.08 ms at 16 to a unit, 0.71 at four)
+    while (nh && units(nh, hcand, heavy.tile, heavy.seg) < 32ull * blocks && heavy.tile > 4) heavy.tile /= 2;
     while (nh && units(nh, hcand, heavy.tile, heavy.seg) < 8ull * blocks && heavy.tile > 1) heavy.tile /= 2;
     while (units(np, ncand, rest.tile, rest.seg) > 0x7FFF0000ull) rest.seg *= 2;  // the steal counter has 32 bits
     while (units(nh, hcand, heavy.tile, heavy.seg) > 0x7FFF0000ull) heavy.seg *= 2;
