@@ -110,7 +110,7 @@ Tuned tune(const hyset_coll* R, const hyset_coll* S, const hyset_join_opts* o,
            hyset_technique selected = HYSET_TECH_AUTO);
 hyset_status compute_features(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const hyset_join_opts* o, float* f,
                               double* base);
-std::string coll_signature(const hyset_coll* c);
+const std::string& coll_signature(const hyset_coll* c);
 std::string join_key(const hyset_coll* R, const hyset_coll* S, const hyset_join_opts* o);
 hyset_status select_technique(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const hyset_join_opts* o,
                               hyset_technique* out, int* selector);

@@ -221,6 +221,7 @@ struct hyset_coll {
     uint32_t max_size = 0;
     uint32_t universe = 0;  // max token + 1
     std::vector<uint64_t> size_hist;  // sets per size, [max_size+1]
+    mutable std::string signature;    // of the statistics, once asked for (coll_signature)
     hs::DevBuf first_ge;              // [max_size+2] first id with size >= l
     std::vector<uint32_t> h_first_ge; // host copy (source of the device copy)
     hs::Index index;

@@ -51,8 +51,7 @@ hyset_status run_join(hyset_ctx* ctx, JoinParams P, int tech, int vmode, const h
     const int count_only = o->count_only ? 1 : 0;
     uint64_t cap = o->pair_capacity ? o->pair_capacity : std::max<uint64_t>(1u << 20, 4ull * P.S.n);
     if (count_only) cap = 0;
-    CK(ctx->s_count.ensure(16, s));
-    CK(ctx->s_work.ensure(16, s));
+    CK(ctx->s_count.ensure(32, s));  // the count, then the launch's counters: one clear
     CK(ctx->s_stats.ensure(64, s));
     P.stats = o->collect_stats ? ctx->s_stats.as<unsigned long long>() : nullptr;
     for (int attempt = 0; attempt < 2; ++attempt) {
@@ -61,10 +60,9 @@ hyset_status run_join(hyset_ctx* ctx, JoinParams P, int tech, int vmode, const h
         P.out.count = ctx->s_count.as<unsigned long long>();
         P.out.cap = cap;
         P.out.count_only = count_only;
-        P.work = ctx->s_work.as<unsigned int>();
+        P.work = ctx->s_count.as<unsigned int>() + 4;
         if (!timed_from_ev0 || attempt > 0) CK(cudaEventRecord(ctx->ev0, s));
-        CK(cudaMemsetAsync(ctx->s_count.p, 0, 16, s));
-        CK(cudaMemsetAsync(ctx->s_work.p, 0, 16, s));
+        CK(cudaMemsetAsync(ctx->s_count.p, 0, 32, s));
         if (P.stats) CK(cudaMemsetAsync(P.stats, 0, 64, s));
         CK(cudaEventRecord(ctx->ek0, s));
         if (T) {

@@ -466,7 +466,7 @@ hyset_status hyset_self_join_host(hyset_ctx* ctx, const uint32_t* tokens, uint64
             ix.pos_bits = pb;
             const bool count_only = o->count_only != 0;
             cap = count_only ? 0 : (o->pair_capacity ? o->pair_capacity : std::max<uint64_t>(1u << 20, 4ull * n));
-            CK(ctx->s_count.ensure(16, s));
+            CK(ctx->s_count.ensure(32, s));
             CK(ctx->s_work.ensure((2 * n_chunks + 4) * 4, s));
             CK(ctx->s_stats.ensure(64, s));
             if (!count_only) CK(ctx->s_pairs.ensure(std::max<uint64_t>(cap, 1) * sizeof(uint2), s));

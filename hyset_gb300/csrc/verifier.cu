@@ -301,17 +301,15 @@ hyset_status hyset_verify_device(hyset_ctx* ctx, const hyset_coll* indexed, cons
     hyset_join_opts ro = *opts;  // candidate lists' pairs are not sorted
     ro.sort_pairs = 0;
     uint64_t cap = opts->pair_capacity ? opts->pair_capacity : (1u << 20);
-    CK(ctx->s_count.ensure(16, s));
-    CK(ctx->s_work.ensure(16, s));
+    CK(ctx->s_count.ensure(32, s));
     for (int attempt = 0; attempt < 2; ++attempt) {
         if (!count_only) CK(ctx->s_pairs.ensure(std::max<uint64_t>(cap, 1) * sizeof(uint2), s));
         Sink sk{count_only ? nullptr : ctx->s_pairs.as<uint2>(), ctx->s_count.as<unsigned long long>(),
                 count_only ? 0ull : (unsigned long long)cap, count_only};
-        CK(cudaMemsetAsync(ctx->s_count.p, 0, 16, s));
-        CK(cudaMemsetAsync(ctx->s_work.p, 0, 16, s));
+        CK(cudaMemsetAsync(ctx->s_count.p, 0, 32, s));
         CK(cudaEventRecord(ctx->ek0, s));
         CK(launch_verify_candidates(R->view(), S->view(), b->view, d_probes, d_offsets, d_candidates, n_probes, vmode,
-                                    sk, ctx->s_work.as<unsigned int>(), ctx->sm_count, s, sig_r, sig_s, words));
+                                    sk, ctx->s_count.as<unsigned int>() + 4, ctx->sm_count, s, sig_r, sig_s, words));
         CK(cudaEventRecord(ctx->ek1, s));
         ST(enqueue_result(ctx, sk, n_probes, &ro));
         CK(cudaStreamSynchronize(s));
