@@ -207,7 +207,34 @@ hyset_status build_sorted_index(hyset_ctx* ctx, hyset_coll* c, const Bounds* b, 
     if (packed && records_ok) entry_layout(c, b, kind, pb, &ix.low_bits, &ix.bound);
     const BoundFields bf = ix.bound ? bound_fields(b) : BoundFields{};
     if (rec_fits) {
-        const auto lk = c->list_longest.find(d_pre);
+        auto lk = c->list_longest.find(d_pre);
+        // The first build with this prefix table does not know its longest list.
+        // Where the average is short enough that it may fit, the entries go into
+        // wide records at once and their counts are read back; lists, an offset
+        // scan, a scatter, a ranking and a conversion took 90 us longer for 200,000
+        // long sets.  Longer lists than a record holds are built again below.
+        constexpr uint64_t MAY_FIT = 16;  // entries per token: a longest list of 63 is four times this
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        CK(cudaStreamIsCapturing(s, &cap));
+        if (lk == c->list_longest.end() && whole && E && E <= MAY_FIT * U && record_shift(record_entries(6), U) == 6 &&
+            cap == cudaStreamCaptureStatusNone) {
+            uint32_t* counts = ctx->sc->counts.as<uint32_t>();
+            CK(ix.rec.ensure(((size_t)U << 6) * 4, s));
+            CK(ctx->sc->gate.ensure(4, s));
+            CK(cudaMemsetAsync(counts, 0, (size_t)U * 4, s));
+            CK(emit_records(v, d_pre, ix.low_bits, counts, ix.rec.as<uint32_t>(), 6, U, s, lo, hi, bf,
+                            first_long_prefix(c, *pre)));
+            int& path = c->list_path[d_pre];
+            CK(longest_list(counts, U, ctx->sc->gate.as<uint32_t>(), s, ctx->h_flags + 15, &path));
+            c->list_longest[d_pre] = ctx->h_flags[15];
+            lk = c->list_longest.find(d_pre);
+            if (record_shift(lk->second, U)) {
+                CK(order_records(counts, U, ix.rec.as<uint32_t>(), 6, s));
+                ix.records = 6;
+                ix.pos_bits = pb;
+                return HYSET_OK;
+            }
+        }
         const int shift = lk != c->list_longest.end() ? record_shift(lk->second, U) : 0;
         if (shift) {
             uint32_t* counts = ctx->sc->counts.as<uint32_t>();

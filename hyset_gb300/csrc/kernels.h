@@ -91,6 +91,10 @@ cudaError_t index_lists(uint32_t* e_token, uint32_t* e_val, uint64_t n, uint32_t
                         uint32_t* list_off, uint32_t* alt_keys, uint32_t* alt_vals, uint32_t* gate, int key_bits,
                         uint32_t* scratch, cudaStream_t s, int* path = nullptr, uint32_t* h_gate = nullptr);
 
+// The longest of U lists from their counts, read back to *h_gate (pinned; a
+// synchronisation), and the path their build takes (index_lists).
+cudaError_t longest_list(const uint32_t* counts, uint32_t U, uint32_t* gate, cudaStream_t s, uint32_t* h_gate, int* path);
+
 // Prefix entries of sets [lo, hi): the first prefix_len(size) tokens of every
 // set (include/hyset/collection.hpp:128-135).  entry_off must hold the
 // exclusive scan of the per-set prefix lengths over [lo, hi) (relative to lo).

@@ -1127,6 +1127,18 @@ cudaError_t records_from_lists(const uint32_t* list_off, const uint32_t* vals, u
     return cudaGetLastError();
 }
 
+cudaError_t longest_list(const uint32_t* counts, uint32_t U, uint32_t* gate, cudaStream_t s, uint32_t* h_gate,
+                         int* path) {
+    cudaError_t e = cudaMemsetAsync(gate, 0, 4, s);
+    if (e != cudaSuccess) return e;
+    note_launches();
+    k_list_max<<<grid_for(U, 256, 4 * 152), 256, 0, s>>>(counts, U, gate);
+    e = cudaMemcpyAsync(h_gate, gate, 4, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) *path = *h_gate <= LIST_SHORT ? 1 : 2;
+    return e;
+}
+
 cudaError_t index_lists(uint32_t* e_token, uint32_t* e_val, uint64_t n, uint32_t U, uint32_t* counts,
                         uint32_t* list_off, uint32_t* alt_keys, uint32_t* alt_vals, uint32_t* gate, int key_bits,
                         uint32_t* scratch, cudaStream_t s, int* path, uint32_t* h_gate) {
@@ -1136,17 +1148,15 @@ cudaError_t index_lists(uint32_t* e_token, uint32_t* e_val, uint64_t n, uint32_t
     int p = path ? *path : 0;
     const uint32_t* g = nullptr;  // the kernels' device-side choice (p == 0 only)
     if (p == 0) {
-        e = cudaMemsetAsync(gate, 0, 4, s);
-        if (e != cudaSuccess) return e;
-        note_launches();
-        k_list_max<<<grid_for(U, 256, 4 * 152), 256, 0, s>>>(counts, U, gate);
         if (h_gate) {  // one host read settles the path for later builds
-            e = cudaMemcpyAsync(h_gate, gate, 4, cudaMemcpyDeviceToHost, s);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+            e = longest_list(counts, U, gate, s, h_gate, &p);
             if (e != cudaSuccess) return e;
-            p = *h_gate <= LIST_SHORT ? 1 : 2;
             if (path) *path = p;
         } else {
+            e = cudaMemsetAsync(gate, 0, 4, s);
+            if (e != cudaSuccess) return e;
+            note_launches();
+            k_list_max<<<grid_for(U, 256, 4 * 152), 256, 0, s>>>(counts, U, gate);
             g = gate;
         }
     }
