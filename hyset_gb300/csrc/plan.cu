@@ -397,6 +397,20 @@ hyset_status autotune_bits(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const h
         }
         return HYSET_OK;
     };
+    // the kernel time of the whole probe range with verification mode m and g probes per batch
+    auto whole = [&](int m, uint32_t g, float* out) -> hyset_status {
+        P.grab = g;
+        P.p_lo = p_lo;
+        P.p_hi = p_hi;
+        CK(cudaMemsetAsync(ctx->s_count.p, 0, 16, s));
+        CK(cudaMemsetAsync(ctx->s_work.p, 0, 16, s));
+        CK(cudaEventRecord(ctx->ek0, s));
+        CK(launch_join(P, TECH_FGSS, m, ctx->sm_count, s));
+        CK(cudaEventRecord(ctx->ek1, s));
+        CK(cudaEventSynchronize(ctx->ek1));
+        CK(cudaEventElapsedTime(out, ctx->ek0, ctx->ek1));
+        return HYSET_OK;
+    };
     if (learned) {
         float f[MLP_IN], x[MLP_IN], y[MLP_OUT] = {0, 0, 0};
         ST(compute_features(ctx, R, S, o, f, nullptr));
@@ -431,6 +445,9 @@ hyset_status autotune_bits(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const h
             P.bits_R = br;
             P.bits_S = bs;
         }
+        // the first launch of a kernel in a process also loads it (milliseconds,
+        // scaled up like the sample: 512 bits lost to 1024 by it): not kept
+        ST(sample(1, &kern_est[k]));
         ST(sample(1, &kern_est[k]));
         est[k] = kern_est[k] + gen_ms;
         return HYSET_OK;
@@ -459,26 +476,13 @@ hyset_status autotune_bits(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const h
         // 512 against 1024 bits again over the whole probe range when that is
         // cheap: the samples weigh the heaviest probes (the largest sets, where
         // the wider signature pays) like the light ones and can misjudge it
-        auto whole_at = [&](uint32_t width, float* out) -> hyset_status {
-            ST(use_width(width));
-            P.p_lo = p_lo;
-            P.p_hi = p_hi;
-            float ms = 0;
-            for (int rep = 0; rep < 2; ++rep) {  // the first run warms the caches
-                CK(cudaMemsetAsync(ctx->s_count.p, 0, 16, s));
-                CK(cudaMemsetAsync(ctx->s_work.p, 0, 16, s));
-                CK(cudaEventRecord(ctx->ek0, s));
-                CK(launch_join(P, TECH_FGSS, 1, ctx->sm_count, s));
-                CK(cudaEventRecord(ctx->ek1, s));
-                CK(cudaEventSynchronize(ctx->ek1));
-                CK(cudaEventElapsedTime(&ms, ctx->ek0, ctx->ek1));
-            }
-            *out = ms;
-            return HYSET_OK;
-        };
         float ms512 = 0, ms1024 = 0;
-        ST(whole_at(512, &ms512));
-        ST(whole_at(1024, &ms1024));
+        ST(use_width(512));
+        ST(whole(1, base_batch, &ms512));  // the first run warms the caches
+        ST(whole(1, base_batch, &ms512));
+        ST(use_width(1024));
+        ST(whole(1, base_batch, &ms1024));
+        ST(whole(1, base_batch, &ms1024));
         best = ms1024 < TUNE_MARGIN * ms512 ? 1024u : 512u;
         kern_est[3] = ms512;
         kern_est[4] = ms1024;
@@ -496,7 +500,17 @@ hyset_status autotune_bits(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const h
     }
     if (vmode) {
         float warp_ms = 0;
+        ST(sample(2, &warp_ms));  // not kept, as above
         ST(sample(2, &warp_ms));
+        if (warp_ms < TUNE_VMODE_MARGIN * cur_ms && cur_ms <= TUNE_BATCH_FULL_MS) {
+            // again over the whole probe range when that is cheap: a sample ends
+            // on one lane's longest merge, which a full launch hides behind its
+            // other warps (a million long sets, Jaccard 0.8: the samples prefer
+            // the warp, the whole range takes 0.67 ms with a lane, 0.72 with a warp)
+            ST(whole(2, base_batch, &warp_ms));  // warms the caches
+            ST(whole(1, base_batch, &cur_ms));
+            ST(whole(2, base_batch, &warp_ms));
+        }
         if (warp_ms < TUNE_VMODE_MARGIN * cur_ms) {
             vm = 2;
             cur_ms = warp_ms;
@@ -513,28 +527,15 @@ hyset_status autotune_bits(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const h
     uint32_t tb = base_batch;
     if (batch) {
         if (cur_ms <= TUNE_BATCH_FULL_MS) {
-            auto whole = [&](uint32_t g, float* out) -> hyset_status {
-                P.grab = g;
-                P.p_lo = p_lo;
-                P.p_hi = p_hi;
-                CK(cudaMemsetAsync(ctx->s_count.p, 0, 16, s));
-                CK(cudaMemsetAsync(ctx->s_work.p, 0, 16, s));
-                CK(cudaEventRecord(ctx->ek0, s));
-                CK(launch_join(P, TECH_FGSS, vm, ctx->sm_count, s));
-                CK(cudaEventRecord(ctx->ek1, s));
-                CK(cudaEventSynchronize(ctx->ek1));
-                CK(cudaEventElapsedTime(out, ctx->ek0, ctx->ek1));
-                return HYSET_OK;
-            };
             float base_ms = 0;
-            ST(whole(base_batch, &base_ms));  // warms the caches the other runs find warm too
-            ST(whole(base_batch, &base_ms));
+            ST(whole(vm, base_batch, &base_ms));  // warms the caches the other runs find warm too
+            ST(whole(vm, base_batch, &base_ms));
             float tb_ms = base_ms;
             for (uint32_t cand_b : TUNE_BATCHES) {
                 const uint32_t g = std::min(cand_b, grab_cap);
                 if (g == base_batch) continue;
                 float ms = 0;
-                ST(whole(g, &ms));
+                ST(whole(vm, g, &ms));
                 if (ms < TUNE_BATCH_MARGIN * base_ms && ms < tb_ms) {
                     tb = g;
                     tb_ms = ms;
