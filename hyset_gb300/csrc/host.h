@@ -130,7 +130,8 @@ hyset_status read_pairs(hyset_ctx* ctx, const void* d_pairs, uint64_t count, std
 hyset_status sort_device_pairs(hyset_ctx* ctx, uint2* pairs, uint64_t n, uint32_t n_probe, uint32_t n_indexed);
 bool swap_sides(const hyset_coll* R, const hyset_coll* S, const hyset_join_opts* o);
 hyset_status run_join(hyset_ctx* ctx, JoinParams P, int tech, int vmode, const hyset_join_opts* o, hyset_result* res,
-                      bool timed_from_ev0, TokenJoinParams* T = nullptr);
+                      bool timed_from_ev0, TokenJoinParams* T = nullptr,
+                      const std::vector<JoinParams>* parts = nullptr);
 // The probe-major prefix filter's split of the longest probes of S into slot
 // segments (JoinParams::heavy_from, segs, seg_slots).
 // The launch's work buffer then needs two zeroed counters.
@@ -150,6 +151,11 @@ uint64_t joined_count(const hyset_ctx* ctx);
 // The signature technique's probes that are taken in small units
 // (JoinParams::heavy_from, heavy_lo); words: 64-bit words per signature.
 void split_window(const hyset_coll* R, const hyset_coll* S, const Bounds* b, int words, JoinParams& P);
+// A signature join whose probes of full signatures are taken by wider ones:
+// one launch's parameters per width, the widest first (empty: P alone).  The
+// wider signatures are generated on `gen`.
+hyset_status widen_window(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const Bounds* b, const JoinParams& P,
+                          cudaStream_t gen, std::vector<JoinParams>& parts);
 // The pairs of a finished join (res->count of them in the context's pair
 // buffer, enqueue_result done and the stream synchronised): sorted when asked,
 // left on the device or copied to the host.

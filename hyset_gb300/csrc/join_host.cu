@@ -46,7 +46,8 @@ bool swap_sides(const hyset_coll* R, const hyset_coll* S, const hyset_join_opts*
 // Runs one configured join launch into the context's pair buffer, growing the
 // buffer and re-running when the first pass overflowed.
 hyset_status run_join(hyset_ctx* ctx, JoinParams P, int tech, int vmode, const hyset_join_opts* o,
-                      hyset_result* res, bool timed_from_ev0, TokenJoinParams* T) {
+                      hyset_result* res, bool timed_from_ev0, TokenJoinParams* T,
+                      const std::vector<JoinParams>* parts) {
     cudaStream_t s = ctx->stream;
     const int count_only = o->count_only ? 1 : 0;
     uint64_t cap = o->pair_capacity ? o->pair_capacity : std::max<uint64_t>(1u << 20, 4ull * P.S.n);
@@ -70,6 +71,13 @@ hyset_status run_join(hyset_ctx* ctx, JoinParams P, int tech, int vmode, const h
             T->work = P.work;
             T->stats = P.stats;
             CK(launch_join_tm(*T, ctx->sm_count, s));
+        } else if (parts && !parts->empty()) {  // up to three launches, a counter each
+            for (size_t k = 0; k < parts->size(); ++k) {
+                JoinParams Q = (*parts)[k];
+                Q.out = P.out;
+                Q.work = P.work + k;
+                CK(launch_join(Q, tech, vmode, ctx->sm_count, s));
+            }
         } else {
             CK(launch_join(P, tech, vmode, ctx->sm_count, s));
         }
@@ -127,6 +135,64 @@ void split_window(const hyset_coll* R, const hyset_coll* S, const Bounds* b, int
         P.heavy_lo = R->h_first_ge[ms];
         return;
     }
+}
+
+// The first set of S from whose size on unrelated pairs of one size pass
+// signatures of `words` words: two sets of l tokens differ in about E = bits / 2
+// (1 - exp(-4 l / bits)) bits, and from an admissible distance of E less two
+// deviations on more than a few percent pass.
+static uint32_t filled_from(const hyset_coll* S, const Bounds* b, int words) {
+    const double bits = 64.0 * words;
+    uint32_t l = std::min(S->max_size, b->L) + 1;
+    for (; l > 1; --l) {
+        const double e = 0.5 * bits * (1.0 - std::exp(-4.0 * (l - 1) / bits));
+        const uint32_t most = 2 * (l - 1) - 2 * minoverlap_of(b->sim, l - 1, l - 1, b->tau);
+        if ((double)most < e - 2.0 * std::sqrt(e * (1.0 - e / bits))) break;
+    }
+    return l > S->max_size ? S->n : S->h_first_ge[l];
+}
+
+// Pairs that pass a full signature are all verified, 5 ps each and more for
+// long sets (200,000 short sets at 64 bits, Jaccard 0.5: 1.2e10 pairs in 61 ms),
+// where a signature that still rejects costs a pair 0.3 ps (64 bits) to 1.2
+// (512).  So the probes that fill their signatures take 256 bits, and those that
+// fill these 512; WIDE_PAIRS pairs cost their verification about what a width's
+// generation and launch cost (at half as many, joins of 8,000 long sets lost
+// 10 to 20 us; with 128 bits between 64 and 256, 100,000 long sets took 3.3 ms
+// instead of 2.8 at cosine 0.75).
+hyset_status widen_window(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const Bounds* b, const JoinParams& P,
+                          cudaStream_t gen, std::vector<JoinParams>& parts) {
+    constexpr uint64_t WIDE_PAIRS = 16ull << 20;
+    parts.assign(1, P);
+    for (int words = std::max(4, 2 * P.words); words <= 8; words *= 2) {
+        const uint32_t from = std::max(P.p_lo, std::min(P.p_hi, filled_from(S, b, parts.back().words)));
+        if (from >= P.p_hi) break;
+        const uint32_t least = std::min(b->minsize[size_at(S, from)], R->max_size + 1);
+        if ((uint64_t)(P.p_hi - from) * (R->n - R->h_first_ge[least]) < WIDE_PAIRS) break;
+        // without room for them the narrow ones do
+        if (R->bitmaps[words].ensure(sig_bytes(R->n, words), ctx->stream) != cudaSuccess ||
+            (S != R && S->bitmaps[words].ensure(sig_bytes(S->n, words), ctx->stream) != cudaSuccess)) {
+            (void)cudaGetLastError();
+            break;
+        }
+        JoinParams W = P;
+        const uint64_t *br = nullptr, *bs = nullptr;
+        ST(get_bitmaps(ctx, R, words, &br, gen));
+        if (S == R) bs = br;
+        else ST(get_bitmaps(ctx, S, words, &bs, gen));
+        W.bits_R = br;
+        W.bits_S = bs;
+        W.words = words;
+        W.p_lo = from;
+        split_window(R, S, b, words, W);
+        parts.back().p_hi = from;
+        parts.push_back(W);
+    }
+    if (parts.size() == 1) parts.clear();
+    std::reverse(parts.begin(), parts.end());  // the longest sets first
+    parts.erase(std::remove_if(parts.begin(), parts.end(), [](const JoinParams& q) { return q.p_lo >= q.p_hi; }),
+                parts.end());
+    return HYSET_OK;
 }
 
 PairSortJob pair_sort_job(const JoinParams& P) {
@@ -304,23 +370,27 @@ hyset_status do_join(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const hyset_j
     // auxiliary stream while the index builds on the context's stream
     // 1024-bit signatures serve the probe-major prefix filter; the window
     // techniques and the token-major kernel take 512 at most
+    std::vector<JoinParams> parts;
     const int words = (int)(tn.bits / 64) > 8 && !(tech == HYSET_TECH_FGSS && tn.probe_major) ? 8 : (int)(tn.bits / 64);
     if (words) {
         const uint64_t *br = nullptr, *bs = nullptr;
         ST(get_bitmaps(ctx, R, words, &br, ctx->aux));
         if (self) bs = br;
         else ST(get_bitmaps(ctx, S, words, &bs, ctx->aux));
-        CK(cudaEventRecord(ctx->ev_join, ctx->aux));
         P.bits_R = br;
         P.bits_S = bs;
         P.words = words;
+        if (tech == HYSET_TECH_BITMAP) {
+            split_window(R, S, b, words, P);
+            if (!o->collect_stats) ST(widen_window(ctx, R, S, b, P, ctx->aux, parts));
+        }
+        CK(cudaEventRecord(ctx->ev_join, ctx->aux));
     }
     if (!token_major && tech == HYSET_TECH_FGSS) {
         ST(build_fgss_indexes(ctx, R, b, self, R->index, R->index_mid, P));
         if (P.X2.set) P.grab = std::min<uint32_t>(P.grab, 16);  // two bands per probe share a warp batch
         split_heavy(S, b, P);
     }
-    if (tech == HYSET_TECH_BITMAP && words) split_window(R, S, b, words, P);
     if (words) CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_join, 0));
     int ktech = tech == HYSET_TECH_FGSS ? TECH_FGSS : (tech == HYSET_TECH_DIRECT ? TECH_DIRECT : TECH_BITMAP);
     if (token_major) {
@@ -332,7 +402,7 @@ hyset_status do_join(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const hyset_j
         ST(run_join(ctx, P, ktech, vmode, o, res, true, &T));
         res->stats[3] = group_entries;
     } else {
-        ST(run_join(ctx, P, ktech, vmode, o, res, true));
+        ST(run_join(ctx, P, ktech, vmode, o, res, true, nullptr, &parts));
     }
     if (P.X.set && o->collect_stats && !token_major) {
         res->stats[3] = R->index.entries;
