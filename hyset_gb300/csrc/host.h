@@ -97,6 +97,7 @@ hyset_status get_bitmaps(hyset_ctx* ctx, hyset_coll* c, int words, const uint64_
 
 // ---- configuration, selector, autotuner (plan.cu) ---------------------------
 constexpr uint32_t TUNE_MIN_PROBES = 60000;  // joins this large time samples to pick their configuration
+constexpr uint32_t WARP_MERGE_SIZE = 1000;   // launches of few probes verify sets this long a warp per candidate, untuned
 constexpr uint32_t DEFAULT_PROBE_BATCH = 3;  // probes per warp batch of the probe-major kernel, untuned
 hyset_status check_opts(hyset_ctx* ctx, const hyset_join_opts* o);
 struct Tuned {

@@ -540,11 +540,17 @@ hyset_status hyset_self_join_host(hyset_ctx* ctx, const uint32_t* tokens, uint64
                 Q.p_hi = hi;
                 // the pieces of the longest sets hold few probes: with fewer than
                 // four probe batches per warp the launch ends on its slowest
-                // warps, so their batches are halved (down to 3)
-                while (Q.grab > 3 && (uint64_t)(hi - join_lo) < 4ull * Q.grab * join_resident_warps(ctx->sm_count))
-                    Q.grab = std::max(3u, (Q.grab + 1) / 2);
+                // warps, so their batches are halved (down to 1), and on its
+                // longest merge, so those of the longest sets verify a warp per
+                // candidate (the tuned mode is the whole range's).  A call at
+                // Jaccard 0.8 / 0.9, a million long sets: 2.70 / 2.50 ms with
+                // lanes and batches down to 3, 2.67 / 2.41 with warps, 2.60 /
+                // 2.39 with both; from sets of 500 tokens on the same
+                while (Q.grab > 1 && (uint64_t)(hi - join_lo) < 4ull * Q.grab * join_resident_warps(ctx->sm_count))
+                    Q.grab = (Q.grab + 1) / 2;
+                const int vm = !o->verify_mode && size_at(C, hi - 1) >= WARP_MERGE_SIZE ? 2 : tn.vmode;
                 Q.work = ctx->s_work.as<unsigned int>() + 2 * join_launches;  // probe batches, split probes
-                CK(launch_join(Q, TECH_FGSS, tn.vmode, ctx->sm_count, s));
+                CK(launch_join(Q, TECH_FGSS, vm, ctx->sm_count, s));
                 ++join_launches;
                 join_lo = hi;
                 joined_to = ends[k];

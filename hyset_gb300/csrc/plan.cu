@@ -62,7 +62,6 @@ Tuned tune(const hyset_coll* R, const hyset_coll* S, const hyset_join_opts* o, h
     // kernel with lanes and 0.075 / 0.131 / 0.141 with warps (0.6: 0.174 / 0.321 /
     // 0.399 and 0.121 / 0.266 / 0.399); with sets of up to 640 tokens lanes are as
     // good or better.
-    constexpr uint32_t WARP_MERGE_SIZE = 1000;
     const bool long_sets = o->technique == HYSET_TECH_AUTO && t.tech == HYSET_TECH_FGSS && t.bits >= 512 &&
                            std::min(R->max_size, S->max_size) >= WARP_MERGE_SIZE;
     t.vmode = o->verify_mode ? (int)o->verify_mode : long_sets ? 2 : 1;
