@@ -382,6 +382,15 @@ hyset_status autotune_bits(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const h
         *out = total * (float)(p_hi - p_lo) / (float)(sampled ? sampled : 1);
         return HYSET_OK;
     };
+    // the first launch of a kernel in a process also loads it (milliseconds,
+    // scaled up with a sample: 512 bits lost to 1024 by it): one probe, not timed
+    auto load = [&](int vm) -> hyset_status {
+        P.p_lo = p_lo;
+        P.p_hi = p_lo + 1;
+        CK(cudaMemsetAsync(ctx->s_work.p, 0, 16, s));
+        CK(launch_join(P, TECH_FGSS, vm, ctx->sm_count, s));
+        return HYSET_OK;
+    };
     auto use_width = [&](uint32_t width) -> hyset_status {
         const int words = (int)(width / 64);
         P.words = words;
@@ -444,9 +453,7 @@ hyset_status autotune_bits(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const h
             P.bits_R = br;
             P.bits_S = bs;
         }
-        // the first launch of a kernel in a process also loads it (milliseconds,
-        // scaled up like the sample: 512 bits lost to 1024 by it): not kept
-        ST(sample(1, &kern_est[k]));
+        ST(load(1));
         ST(sample(1, &kern_est[k]));
         est[k] = kern_est[k] + gen_ms;
         return HYSET_OK;
@@ -470,6 +477,7 @@ hyset_status autotune_bits(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const h
         ST(time_width(4));
         if (est[4] < TUNE_MARGIN * est[3]) best = 1024;
     }
+    float whole_ms = 0;  // the chosen width's whole range with mode vm and the base batch (0: not measured)
     if (best >= 512 && std::max(kern_est[3], kern_est[4]) > 0 &&
         std::max(kern_est[3], kern_est[4]) <= TUNE_BATCH_FULL_MS) {
         // 512 against 1024 bits again over the whole probe range when that is
@@ -485,38 +493,46 @@ hyset_status autotune_bits(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const h
         best = ms1024 < TUNE_MARGIN * ms512 ? 1024u : 512u;
         kern_est[3] = ms512;
         kern_est[4] = ms1024;
+        whole_ms = best == 512 ? ms512 : ms1024;
     }
     const int kc = best == 0 ? 0 : best == 128 ? 1 : best == 256 ? 2 : best == 512 ? 3 : 4;
     float cur_ms = kern_est[kc];  // the chosen configuration's estimated kernel time
-    // verification: a lane per surviving item, or the warp per item when the
-    // samples show it faster at the chosen width (long merges: low thresholds,
-    // cosine); an explicit mode is kept
+    // verification: a lane per surviving item, or the warp per item where that
+    // is faster at the chosen width (long merges: low thresholds, cosine); an
+    // explicit mode is kept.  Over the whole probe range where that is cheap: a
+    // sample ends on one lane's longest merge, which a full launch hides behind
+    // its other warps (a million long sets, Jaccard 0.8: the samples prefer the
+    // warp, the whole range takes 0.67 ms with a lane, 0.72 with a warp)
     int vm = o->verify_mode == 2 ? 2 : 1;
     ST(use_width(best));
-    if (learned) {  // the predicted width's own estimate (the base of the comparisons below)
+    if (whole_ms > 0) {
+        cur_ms = whole_ms;
+    } else if (learned) {  // the predicted width's own estimate (the base of the comparisons below)
         ST(sample(1, &cur_ms));  // the first run after the generation warms the caches: not kept
         ST(sample(1, &cur_ms));
     }
     if (vmode) {
         float warp_ms = 0;
-        ST(sample(2, &warp_ms));  // not kept, as above
-        ST(sample(2, &warp_ms));
-        if (warp_ms < TUNE_VMODE_MARGIN * cur_ms && cur_ms <= TUNE_BATCH_FULL_MS) {
-            // again over the whole probe range when that is cheap: a sample ends
-            // on one lane's longest merge, which a full launch hides behind its
-            // other warps (a million long sets, Jaccard 0.8: the samples prefer
-            // the warp, the whole range takes 0.67 ms with a lane, 0.72 with a warp)
-            ST(whole(2, base_batch, &warp_ms));  // warms the caches
-            ST(whole(1, base_batch, &cur_ms));
+        ST(load(2));
+        if (whole_ms > 0) {
             ST(whole(2, base_batch, &warp_ms));
+        } else {
+            ST(sample(2, &warp_ms));
+            if (warp_ms < TUNE_VMODE_MARGIN * cur_ms && cur_ms <= TUNE_BATCH_FULL_MS) {
+                ST(whole(1, base_batch, &whole_ms));
+                cur_ms = whole_ms;
+                ST(whole(2, base_batch, &warp_ms));
+            }
         }
         if (warp_ms < TUNE_VMODE_MARGIN * cur_ms) {
             vm = 2;
             cur_ms = warp_ms;
+            if (whole_ms > 0) whole_ms = warp_ms;
         }
         *vmode = vm;
     } else if (vm == 2) {
         ST(sample(2, &cur_ms));
+        whole_ms = 0;
     }
     // probe batch: it trades loads in flight per warp against balance across
     // warps, which samples of a few thousand batches cannot show (they do not
@@ -526,9 +542,11 @@ hyset_status autotune_bits(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const h
     uint32_t tb = base_batch;
     if (batch) {
         if (cur_ms <= TUNE_BATCH_FULL_MS) {
-            float base_ms = 0;
-            ST(whole(vm, base_batch, &base_ms));  // warms the caches the other runs find warm too
-            ST(whole(vm, base_batch, &base_ms));
+            float base_ms = whole_ms;
+            if (whole_ms == 0) {
+                ST(whole(vm, base_batch, &base_ms));  // warms the caches the other runs find warm too
+                ST(whole(vm, base_batch, &base_ms));
+            }
             float tb_ms = base_ms;
             for (uint32_t cand_b : TUNE_BATCHES) {
                 const uint32_t g = std::min(cand_b, grab_cap);
