@@ -142,12 +142,12 @@ def algorithmic_bytes(st, count, words, n_probes):
     counters: per probe its (start, size) record (8); per prefix token the token
     and its list bounds (12); per index entry in a window the packed entry (4);
     per entry that passes the entry's side of the positional bound (all of
-    them unless the records carry that bound) the candidate's (start, size)
-    (8); per signature check both signatures (16 W); per token read by
-    verification 4; per result pair 8."""
-    prefix_tokens, items, bitmap_checks, verify_tokens = st[4], st[0], st[5], st[6]
+    them unless the index carries that bound) the candidate's head record (32;
+    without signatures its (start, size), 8); per item that reaches verification
+    both signatures (16 W); per token read by verification 4; per result pair 8."""
+    prefix_tokens, items, verified, verify_tokens = st[4], st[0], st[1], st[6]
     entries = st[7] or items
-    return (8 * n_probes + 12 * prefix_tokens + 4 * entries + 8 * items + 16 * words * bitmap_checks
+    return (8 * n_probes + 12 * prefix_tokens + 4 * entries + (32 if words else 8) * items + 16 * words * verified
             + 4 * verify_tokens + 8 * count)
 
 
@@ -228,6 +228,7 @@ def run_ours(args, ws, rank, local):
     import numpy as np
     import torch
     import hyset_gb300 as hs
+    from hyset_gb300 import similarity
     from hyset_gb300.handlers import FgssHandler
 
     torch.cuda.set_device(local)
@@ -344,7 +345,10 @@ def run_ours(args, ws, rank, local):
             h.set_output_handler(ph)
             torch.cuda.synchronize()
             t0 = time.perf_counter()
-            h.join(hs.Partition(0, hc.blocks), hs.Partition(0, hc.blocks))
+            for first in hc.blocks:  # the reference's length filter per block pair
+                for second in hc.blocks[first.id:]:
+                    if c.sizes[first.end_id] >= similarity.minsize("jaccard", int(c.sizes[second.start_id]), THRESHOLD):
+                        h.join(first, second)
             plain.append(time.perf_counter() - t0)
             h.close()
         plain_ms = 1000.0 * min(plain) if plain else None
