@@ -23,9 +23,11 @@
 //     (window, distance over all words) and queued, and 32 queued pairs are
 //     verified at a time, a lane or the warp each.
 // 200,000 short sets (lognormal, mean 29), Jaccard 0.7, 64 bits on GB300: a
-// call 13.76 ms before, 2.40 ms now; one block fewer per SM for W <= 2 2.52,
-// heavy probes (see WinCut) 4 / 8 to a unit 2.70 / 2.52, segments of 4,096
-// 2.58, one group up to a distance of 14 or 18 instead of 16 within 1 %.
+// call 13.76 ms before, 2.40 ms with this kernel alone, 1.93 with its longest
+// probes in launches of wider signatures (widen_window, join_host.cu).  Alone:
+// one block fewer per SM for W <= 2 2.52, heavy probes (see WinCut) 4 / 8 to a
+// unit 2.70 / 2.52, segments of 4,096 2.58, one group up to a distance of 14 or
+// 18 instead of 16 within 1 %.
 #include "join_impl.cuh"
 
 namespace hs {
