@@ -68,7 +68,8 @@ typedef struct {
     hyset_technique technique;
     uint32_t bitmap_bits;      /* 64, 128, 256, 512 or 1024 (the probe-major prefix filter only; the
                                   window techniques, the token-major kernel and the candidate
-                                  verifier use 512 for it); 0 = chosen by the library with technique
+                                  verifier use 512 for it; a signature join's probes that fill
+                                  narrower ones may take 256 or 512); 0 = chosen by the library with technique
                                   AUTO (timed samples for joins of 60,000 probes or more, else
                                   128 bits for mean set sizes <= 48 and 512 above, 256 for the window
                                   techniques), no signature
