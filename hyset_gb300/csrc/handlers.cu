@@ -12,6 +12,21 @@
 
 using namespace hs;
 
+namespace {
+
+// Room for `cap` pairs.  h->cap follows the buffer: a failed allocation leaves
+// it at what the handler still holds (nothing, when the old buffer was given
+// back for the new one), never at what was asked for.
+cudaError_t pair_room(hyset_handler* h, uint64_t cap) {
+    const cudaError_t e = h->pairs.ensure(cap * sizeof(uint2), h->ctx->stream);
+    h->cap = e == cudaSuccess ? cap : std::min<uint64_t>(h->cap, h->pairs.bytes / sizeof(uint2));
+    return e;
+}
+
+uint64_t least_pair_room(const hyset_handler* h) { return std::max<uint64_t>(1u << 16, (uint64_t)h->block_size * 4); }
+
+}  // namespace
+
 extern "C" {
 
 hyset_status hyset_handler_create(hyset_ctx* ctx, const hyset_coll* coll, hyset_technique technique, hyset_sim sim,
@@ -52,8 +67,7 @@ hyset_status hyset_handler_create(hyset_ctx* ctx, const hyset_coll* coll, hyset_
     }
     CK(h->count.ensure(16, s));
     CK(h->work.ensure(16, s));
-    h->cap = aggregate ? 0 : std::max<uint64_t>(1u << 16, (uint64_t)block_size * 4);
-    if (!aggregate) CK(h->pairs.ensure(h->cap * sizeof(uint2), s));
+    if (!h->aggregate) CK(pair_room(h.get(), least_pair_room(h.get())));
     CK(cudaStreamSynchronize(s));
     *out = h.release();
     return HYSET_OK;
@@ -105,6 +119,7 @@ hyset_status build_block_index(hyset_handler* h, const hyset_block& blk) {
 hyset_status run_handler_join(hyset_handler* h, JoinParams P) {
     hyset_ctx* ctx = h->ctx;
     cudaStream_t s = ctx->stream;
+    if (!h->aggregate && h->cap == 0) CK(pair_room(h, least_pair_room(h)));  // lost to a failed allocation
     const int tech = h->technique == HYSET_TECH_FGSS ? TECH_FGSS : TECH_BITMAP;
     const int vmode = 1;
     hyset_join_opts o;
@@ -138,8 +153,7 @@ hyset_status run_handler_join(hyset_handler* h, JoinParams P) {
             h->out_count += count;
             return HYSET_OK;
         }
-        h->cap = count + count / 4 + 1024;
-        CK(h->pairs.ensure(h->cap * sizeof(uint2), s));
+        CK(pair_room(h, count + count / 4 + 1024));
     }
     return fail(ctx, HYSET_E_OVERFLOW, "handler pair buffer overflow after resize");
 }
@@ -193,10 +207,10 @@ hyset_status join_ranges(hyset_handler* h, uint32_t r_lo, uint32_t r_hi, uint32_
     P.p_hi = p_hi;
     P.r_lo = r_lo;
     P.r_hi = r_hi;
-    if (!h->aggregate) {  // room for a few pairs of every probe, as a whole join has
-        h->cap = std::max(h->cap, std::min<uint64_t>(4ull * (p_hi - p_lo), 1u << 24));
-        CK(h->pairs.ensure(h->cap * sizeof(uint2), ctx->stream));
-    }
+    // room for a few pairs of every probe, as a whole join has (without it a
+    // result that overflows is run again)
+    const uint64_t room = std::min<uint64_t>(4ull * (p_hi - p_lo), 1u << 24);
+    if (!h->aggregate && room > h->cap && pair_room(h, room) != cudaSuccess) (void)cudaGetLastError();
     if (h->technique == HYSET_TECH_FGSS) {
         P.grab = DEFAULT_PROBE_BATCH;
         ST(build_sorted_index(ctx, c, h->bounds, 0, h->part, nullptr, nullptr, -1, true, r_lo, r_hi));
