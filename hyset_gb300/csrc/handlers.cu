@@ -87,6 +87,7 @@ hyset_status build_block_index(hyset_handler* h, const hyset_block& blk) {
     const std::vector<uint64_t> bh = range_hist(c, lo, hi);
     for (size_t l = 0; l < bh.size(); ++l) E += bh[l] * h->bounds->index_prefix[l];
     const uint64_t E1 = E ? E : 1;
+    h->indexed_block = -1;  // until the build is through: a failed one leaves no block's index
     CK(h->counts.ensure(((size_t)U + 1) * 4, s));
     CK(h->list_off.ensure(((size_t)U + 1) * 4, s));
     CK(h->e_len.ensure((size_t)nb * 4 + 4, s));

@@ -263,7 +263,7 @@ struct hyset_handler {
     hs::Bounds* bounds = nullptr;
     // per-indexed-block inverted index (reference layout: unsorted lists)
     hs::DevBuf counts, list_off, e_len, e_off, e_tok, e_set, e_pos, idx_set, idx_pos, scan;
-    uint32_t indexed_block = 0xFFFFFFFFu;
+    int64_t indexed_block = -1;  // the block the arrays above hold (-1: none)
     hs::Index part;  // the index of an indexed partition joined as a whole
     hs::DevBuf bits, pairs, count, work;
     uint64_t cap = 0;

@@ -3,6 +3,7 @@ made to fail (as in test_gpu_faults.py, before CUDA is asked), and the call
 either goes on with less or reports HYSET_E_NOMEM and leaves its objects fit
 for the next call."""
 import contextlib
+import dataclasses
 import itertools
 import os
 
@@ -81,3 +82,42 @@ def test_handler_pairs_that_outgrow_their_buffer(ctx, tech, form):
         np.testing.assert_array_equal(_sorted(out.pairs), want)
 
     assert not all(outcomes(op, 60))
+
+
+def test_block_index_that_was_not_finished(ctx):
+    """A failed build leaves no block's index behind, and no block id stands for "none"."""
+    c = synth.generate(synth.C2, n_sets=4000, universe=2500, dup_frac=0.2, seed=9)
+    hc = hs.from_arrays(c.tokens, c.sizes, 1000, 0.7)
+    coll = ctx.upload(c.tokens, c.sizes, c.starts)
+    pairs = oracle.as_set(oracle.join(c.tokens, c.starts, c.sizes, 0.7))
+    b = list(hc.blocks)
+
+    def between(f, s):
+        return {(p, q) for p, q in pairs if s.start_id <= p <= s.end_id and f.start_id <= q <= f.end_id}
+
+    def op(k):
+        h = FgssHandler(ctx, hc, coll, 1000, False, 0.7)
+        out = hs.PairsHandler()
+        h.set_output_handler(out)
+        h.join(b[0], b[2])
+        try:
+            h.join(b[3], b[3])  # longer sets: a larger index
+        except hs.HysetError:
+            h.join(b[0], b[1])
+            assert oracle.as_set(out.pairs) == between(b[0], b[2]) | between(b[0], b[1])
+            raise
+        assert oracle.as_set(out.pairs) == between(b[0], b[2]) | between(b[3], b[3])
+
+    assert not all(outcomes(op, 60))
+
+
+def test_every_block_id_is_indexed(ctx):
+    c = synth.generate(synth.C2, n_sets=2000, universe=2500, dup_frac=0.2, seed=9)
+    hc = hs.from_arrays(c.tokens, c.sizes, 2000, 0.7)
+    coll = ctx.upload(c.tokens, c.sizes, c.starts)
+    last = dataclasses.replace(hc.blocks[0], id=0xFFFFFFFF)
+    h = FgssHandler(ctx, hc, coll, 2000, False, 0.7)
+    out = hs.PairsHandler()
+    h.set_output_handler(out)
+    h.join(last, last)
+    assert oracle.as_set(out.pairs) == oracle.as_set(oracle.join(c.tokens, c.starts, c.sizes, 0.7))
