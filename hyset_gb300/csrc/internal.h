@@ -41,6 +41,7 @@ struct DevBuf {
             add_device_bytes((long long)bytes);
         } else {
             p = nullptr;
+            (void)cudaGetLastError();  // reported here, not by the next launch
         }
         return e;
     }
