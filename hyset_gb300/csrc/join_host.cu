@@ -106,9 +106,16 @@ hyset_status run_join(hyset_ctx* ctx, JoinParams P, int tech, int vmode, const h
 // one probe, 1.04 at three; 0.47 split).  Above 64 / 96 / 128 slots, a call of
 // that join: 0.865 / 0.789 / 0.776 ms; units of 32 / 64 / 128 slots 0.809 /
 // 0.776 / 0.801.
+// The units are a grid, split probes x segments of the longest prefix, counted
+// in 32 bits, and most of it is empty where one set is far longer than the
+// others: a set of 4,200,000 tokens beside 131,200 of 260 made 2^32 + 10^7 units
+// of 64 slots at Jaccard 0.5, and the probes of the first 2^32 were left out.  So
+// the segments grow until the grid is at most four times what the probes' own
+// slots fill (32 million units, whatever they are; a million always pass).
 void split_heavy(const hyset_coll* S, const Bounds* b, JoinParams& P) {
     constexpr uint32_t HEAVY_SLOTS = 128;  // probes with longer prefixes are split
     constexpr uint32_t SEG_SLOTS = 64;     // prefix slots per unit of a split probe
+    constexpr uint64_t MANY_UNITS = 1ull << 20, MOST_UNITS = 1ull << 25;  // 2^32 tokens hold 2^24 split probes at most
     P.heavy_from = 0xFFFFFFFFu;
     P.segs = 0;
     P.seg_slots = SEG_SLOTS;
@@ -117,6 +124,15 @@ void split_heavy(const hyset_coll* S, const Bounds* b, JoinParams& P) {
         if (b->probe_prefix[l] > HEAVY_SLOTS) {
             P.heavy_from = S->h_first_ge[l];
             P.segs = (b->probe_prefix[L] + SEG_SLOTS - 1) / SEG_SLOTS;
+            const uint64_t heavy = S->n - P.heavy_from;
+            if (heavy * P.segs <= MANY_UNITS) return;
+            uint64_t filled = heavy;
+            for (uint32_t k = l; k <= L; ++k) filled += S->size_hist[k] * (uint64_t)b->probe_prefix[k] / SEG_SLOTS;
+            const uint64_t most = std::min(std::max(4 * filled, MANY_UNITS), MOST_UNITS);
+            while (heavy * P.segs > most) {
+                P.seg_slots *= 2;
+                P.segs = (b->probe_prefix[L] + P.seg_slots - 1) / P.seg_slots;
+            }
             return;
         }
 }
