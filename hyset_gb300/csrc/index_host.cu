@@ -142,10 +142,10 @@ int key_bits_for(uint32_t universe) {
 // force_pb >= 0 fixes the layout (0 = unpacked, > 0 = packed with that many
 // position bits) so that two indexes of one join share it.
 // records_ok: the caller's kernel reads token records (record_shift); they are
-// built once the longest list of this prefix table is known to fit (it is
-// read back on the collection's first build with the table; that build's
-// lists are converted), afterwards directly from the prefix entries: one emit
-// pass and one ordering pass, no offsets, no scan.
+// built where the longest list of this prefix table fits (it is read back on
+// the collection's first build with the table, which guesses the width) and
+// there is room for them, directly from the prefix entries: one emit pass and
+// one ordering pass, no offsets, no scan.
 // [lo, hi): only these sets are indexed (set ids stay absolute).
 hyset_status build_sorted_index(hyset_ctx* ctx, hyset_coll* c, const Bounds* b, int kind, Index& ix,
                                 const std::vector<uint32_t>* pre, const uint32_t* d_pre,
@@ -206,46 +206,60 @@ hyset_status build_sorted_index(hyset_ctx* ctx, hyset_coll* c, const Bounds* b, 
     // the kernel that reads records reads bound fields, in records or lists
     if (packed && records_ok) entry_layout(c, b, kind, pb, &ix.low_bits, &ix.bound);
     const BoundFields bf = ix.bound ? bound_fields(b) : BoundFields{};
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(s, &capture));
+    const bool capturing = capture != cudaStreamCaptureStatusNone;
+    // Room for records of this shift; without it the lists do.  (A capture
+    // allocates nothing: its buffers were sized before it.)
+    auto room = [&](int shift) {
+        const size_t need = ((size_t)U << shift) * 4;
+        if (capturing) return ix.rec.p && ix.rec.bytes >= need;
+        if (ix.rec_guessed && ix.rec.bytes > need) ix.rec.release(s);  // wider than its lists turned out to need
+        ix.rec_guessed = false;
+        return ix.rec.ensure(need, s) == cudaSuccess;
+    };
+    auto emit_in_records = [&](int shift) -> hyset_status {
+        CK(cudaMemsetAsync(ctx->sc->counts.p, 0, (size_t)U * 4, s));
+        CK(emit_records(v, d_pre, ix.low_bits, ctx->sc->counts.as<uint32_t>(), ix.rec.as<uint32_t>(), shift, U, s, lo,
+                        hi, bf, first_long_prefix(c, *pre)));
+        return HYSET_OK;
+    };
+    auto finish_records = [&](int shift) -> hyset_status {
+        CK(order_records(ctx->sc->counts.as<uint32_t>(), U, ix.rec.as<uint32_t>(), shift, s));
+        ix.records = shift;
+        ix.pos_bits = pb;
+        return HYSET_OK;
+    };
     if (rec_fits) {
         auto lk = c->list_longest.find(d_pre);
         // The first build with this prefix table does not know its longest list.
         // Where the average is short enough that it may fit, the entries go into
-        // wide records at once and their counts are read back; lists, an offset
-        // scan, a scatter, a ranking and a conversion took 90 us longer for 200,000
+        // records at once and their counts are read back; lists, an offset scan,
+        // a scatter, a ranking and a conversion took 90 us longer for 200,000
         // long sets.  Longer lists than a record holds are built again below.
+        // Narrow records up to one entry per token on average: the first join of
+        // 1,024 sets over 2^24 tokens takes 0.60 ms and 2.2 GB with them, 0.80 and
+        // 4.4 with the wide ones, 1.36 and 2.2 by way of lists.
         constexpr uint64_t MAY_FIT = 16;  // entries per token: a longest list of 63 is four times this
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        CK(cudaStreamIsCapturing(s, &cap));
-        if (lk == c->list_longest.end() && whole && E && E <= MAY_FIT * U && record_shift(record_entries(6), U) == 6 &&
-            cap == cudaStreamCaptureStatusNone) {
-            uint32_t* counts = ctx->sc->counts.as<uint32_t>();
-            CK(ix.rec.ensure(((size_t)U << 6) * 4, s));
+        const int guess = E <= U ? 5 : E <= MAY_FIT * U ? 6 : 0;
+        if (lk == c->list_longest.end() && whole && E && guess && record_shift(record_entries(guess), U) == guess &&
+            !capturing && room(guess)) {
             CK(ctx->sc->gate.ensure(4, s));
-            CK(cudaMemsetAsync(counts, 0, (size_t)U * 4, s));
-            CK(emit_records(v, d_pre, ix.low_bits, counts, ix.rec.as<uint32_t>(), 6, U, s, lo, hi, bf,
-                            first_long_prefix(c, *pre)));
+            ST(emit_in_records(guess));
             int& path = c->list_path[d_pre];
-            CK(longest_list(counts, U, ctx->sc->gate.as<uint32_t>(), s, ctx->h_flags + 15, &path));
-            c->list_longest[d_pre] = ctx->h_flags[15];
-            lk = c->list_longest.find(d_pre);
-            if (record_shift(lk->second, U)) {
-                CK(order_records(counts, U, ix.rec.as<uint32_t>(), 6, s));
-                ix.records = 6;
-                ix.pos_bits = pb;
-                return HYSET_OK;
+            CK(longest_list(ctx->sc->counts.as<uint32_t>(), U, ctx->sc->gate.as<uint32_t>(), s, ctx->h_flags + 15, &path));
+            lk = c->list_longest.emplace(d_pre, ctx->h_flags[15]).first;
+            const int needs = record_shift(lk->second, U);
+            if (needs && needs <= guess) {
+                ix.rec_guessed = needs < guess;
+                return finish_records(guess);
             }
+            if (!needs) ix.rec.release(s);
         }
         const int shift = lk != c->list_longest.end() ? record_shift(lk->second, U) : 0;
-        if (shift) {
-            uint32_t* counts = ctx->sc->counts.as<uint32_t>();
-            CK(ix.rec.ensure(((size_t)U << shift) * 4, s));
-            CK(cudaMemsetAsync(counts, 0, (size_t)U * 4, s));
-            CK(emit_records(v, d_pre, ix.low_bits, counts, ix.rec.as<uint32_t>(), shift, U, s, lo, hi, bf,
-                            first_long_prefix(c, *pre)));
-            CK(order_records(counts, U, ix.rec.as<uint32_t>(), shift, s));
-            ix.records = shift;
-            ix.pos_bits = pb;
-            return HYSET_OK;
+        if (shift && room(shift)) {
+            ST(emit_in_records(shift));
+            return finish_records(shift);
         }
     }
     CK(set_prefix_lengths(v, d_pre, lo, hi, len + lo, s));  // len and off by absolute set id
@@ -258,23 +272,20 @@ hyset_status build_sorted_index(hyset_ctx* ctx, hyset_coll* c, const Bounds* b, 
                                lo, hi, 0xFFFFFFFFu, first_long_prefix(c, *pre), bf));
         // the list build's path is read back once per collection and prefix
         // table (not while a batch is being captured into a graph)
-        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-        CK(cudaStreamIsCapturing(s, &capturing));
         // (a part of the collection has no longer lists than the whole, but says
         // nothing about it: its own path is not remembered)
         const auto known = c->list_path.find(d_pre);
         int part_path = known == c->list_path.end() ? 0 : known->second;
         int& path = whole ? c->list_path[d_pre] : part_path;
-        const bool read_back = path == 0 && capturing == cudaStreamCaptureStatusNone;
+        const bool read_back = path == 0 && !capturing;
         CK(index_lists(ctx->sc->tok.as<uint32_t>(), ix.set.as<uint32_t>(), E, U, counts, ix.list_off.as<uint32_t>(),
                        ctx->sc->altk.as<uint32_t>(), ctx->sc->altv.as<uint32_t>(), ctx->sc->gate.as<uint32_t>(),
                        key_bits_for(U), scr, s, &path, read_back ? ctx->h_flags + 15 : nullptr));
         if (read_back && E && whole) c->list_longest[d_pre] = ctx->h_flags[15];
         ix.pos_bits = pb;
         const int shift = rec_fits && E && read_back ? record_shift(ctx->h_flags[15], U) : 0;
-        if (shift) {
+        if (shift && room(shift)) {
             // this build's lists become records; later builds emit records directly
-            CK(ix.rec.ensure(((size_t)U << shift) * 4, s));
             CK(records_from_lists(ix.list_off.as<uint32_t>(), ix.set.as<uint32_t>(), U, ix.rec.as<uint32_t>(), shift,
                                   s));
             ix.records = shift;

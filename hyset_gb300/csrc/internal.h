@@ -88,6 +88,7 @@ struct Index {
     DevBuf list_off, set, pos;
     DevBuf rec;             // token records (2^records words per token) when records is set
     int records = 0;        // their shift (see record_shift); 0: lists
+    bool rec_guessed = false;  // rec was sized before the longest list was known, and is wider than that needs
     uint32_t universe = 0;
     uint64_t entries = 0;
     uint32_t pos_bits = 0;  // > 0: packed (set << pos_bits) | position entries

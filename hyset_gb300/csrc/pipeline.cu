@@ -429,9 +429,9 @@ hyset_status hyset_self_join_host(hyset_ctx* ctx, const uint32_t* tokens, uint64
         // (this collection's tokens differ), and the join is then run again
         // over lists.
         auto lit = ctx->longest_cache.find(key);
-        const int records = assumed && lit != ctx->longest_cache.end() ? record_shift(lit->second, U) : 0;
+        int records = assumed && lit != ctx->longest_cache.end() ? record_shift(lit->second, U) : 0;
+        if (records && ix.rec.ensure(((size_t)U << records) * 4, s) != cudaSuccess) records = 0;  // no room: lists
         if (records) {
-            CK(ix.rec.ensure(((size_t)U << records) * 4, s));
             entry_layout(C, b, 0, pb, &ix.low_bits, &ix.bound);
         }
         const uint32_t big_lo = first_long_prefix(C, b->index_prefix);  // emitted a warp per set from here on

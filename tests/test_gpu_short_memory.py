@@ -14,6 +14,7 @@ import hyset_gb300 as hs
 import oracle
 from hyset_gb300 import synth
 from hyset_gb300.handlers import BitmapHandler, FgssHandler
+from test_gpu_index_lists import _plant
 
 pytestmark = pytest.mark.gpu
 
@@ -40,14 +41,15 @@ def keep(ctx):
         x.close() if hasattr(x, "close") else x.free()
 
 
-def outcomes(op, most):
-    """op(n) with the n-th allocation failing, until twelve in a row come to no
-    harm: for each n, whether the call went through."""
+def outcomes(op, most, ready=lambda: None):
+    """op(ready()) with the n-th allocation of op failing, n from 1 until twelve
+    in a row come to no harm: for each n, whether the call went through."""
     went = []
     while len(went) < most and not (len(went) >= 12 and all(went[-12:])):
+        x = ready()
         with failing(len(went) + 1):
             try:
-                op(len(went) + 1)
+                op(x)
                 went.append(True)
             except hs.HysetError as e:
                 assert e.status == E_NOMEM, str(e)
@@ -76,7 +78,7 @@ def test_handler_pairs_that_outgrow_their_buffer(ctx, keep, tech, form):
         whole = hs.Partition(0, hc.blocks)
         h.join(*((whole, whole) if form == "partition" else (hc.blocks[0], hc.blocks[0])))
 
-    def op(k):
+    def op(_):
         h = keep(BitmapHandler(ctx, hc, coll, 64, 100, False, 0.8) if tech == "bitmap"
                  else FgssHandler(ctx, hc, coll, 100, False, 0.8))
         out = hs.PairsHandler()
@@ -104,7 +106,7 @@ def test_block_index_that_was_not_finished(ctx, keep):
     def between(f, s):
         return {(p, q) for p, q in pairs if s.start_id <= p <= s.end_id and f.start_id <= q <= f.end_id}
 
-    def op(k):
+    def op(_):
         h = keep(FgssHandler(ctx, hc, coll, 1000, False, 0.7))
         out = hs.PairsHandler()
         h.set_output_handler(out)
@@ -142,3 +144,100 @@ def test_a_refused_allocation_is_reported_once(ctx, keep):
             ctx.self_join(coll, threshold=0.7, pair_capacity=1 << 45, **kw)
         assert e.value.status == E_NOMEM
         assert oracle.as_set(ctx.self_join(coll, threshold=0.7, **kw).pairs) == want
+
+
+def _uniform(n, spread, size=30, seed=1):
+    """n sets whose prefix tokens (four of 30 at Jaccard 0.8) spread evenly over
+    `spread` tokens; near-copies among them."""
+    rng = np.random.default_rng(seed)
+    low = np.arange(4) * (spread // 4) + rng.integers(0, spread // 4, (n, 4))
+    high = spread + np.arange(size - 4) * 64 + rng.integers(0, 64, (n, size - 4))
+    rows = np.concatenate([low, high], axis=1).astype(np.uint32)
+    rows[n // 2:n // 2 + n // 8] = rows[:n // 8]
+    rows[n // 2:n // 2 + n // 8, 9] = spread + 5 * 64 + rng.integers(0, 64, n // 8)
+    return rows.reshape(-1), np.full(n, size, np.uint32)
+
+
+PREFIX = dict(threshold=0.8, technique="fgss", probe_major=True, bitmap=128, sort_pairs=True)  # midprefix of 30: 4
+
+
+# (sets, universe, the record width in words after the first and after later builds; 0: lists)
+@pytest.mark.parametrize("n,spread,first,later", [
+    (2_000, 1 << 20, 32, 32),    # few sets over many tokens
+    (40_000, 1 << 15, 64, 32),   # five entries to a token, none with 32
+    (60_000, 1 << 14, 64, 64),   # fifteen, and some with more than 31
+    (100_000, 1 << 14, 64, 64),  # twenty-four: lists first, then their records
+    (200_000, 1 << 14, 0, 0),    # fifty: lists
+])
+def test_records_no_wider_than_the_lists_need(ctx, keep, n, spread, first, later):
+    tokens, sizes = _uniform(n, spread)
+    entries = np.concatenate([tokens[k::30] for k in range(4)])
+    longest = np.bincount(entries).max()
+    assert (later == 32) == (longest <= 31) and (later == 0) == (longest > 63)
+    universe = int(tokens.max()) + 1
+    coll = keep(ctx.upload(tokens, sizes))
+    keep(ctx.upload(tokens, sizes))
+    bytes_now = hs._lib.load().hyset_device_bytes
+    other = keep(ctx.upload(tokens, sizes))
+    ctx.self_join(other, **PREFIX)  # the context's own buffers
+    before = bytes_now()
+    got = ctx.self_join(coll, **PREFIX)
+    lists = (universe + 1) * 4 + entries.size * 8  # list offsets, entries and their positions
+    signatures = n * (16 + 32) + 8 + 32
+    assert bytes_now() - before <= lists + signatures + universe * first * 4 + 64
+    again = ctx.self_join(coll, **PREFIX)
+    assert bytes_now() - before <= lists + signatures + universe * later * 4 + 64
+    want = oracle.as_set(oracle.join(tokens, np.arange(n, dtype=np.uint32) * 30, sizes, 0.8))
+    assert oracle.as_set(got.pairs) == want and oracle.as_set(again.pairs) == want and len(want) >= n // 8
+
+
+def test_lists_that_outgrow_the_guessed_records(ctx, keep):
+    c = _plant(synth.generate(synth.C2, n_sets=20000, seed=64), 90, seed=2)
+    bytes_now = hs._lib.load().hyset_device_bytes
+    ctx.self_join(keep(ctx.upload(c.tokens, c.sizes, c.starts)), **PREFIX)
+    coll = keep(ctx.upload(c.tokens, c.sizes, c.starts))
+    before = bytes_now()
+    got = ctx.self_join(coll, **PREFIX)
+    assert bytes_now() - before < (int(c.tokens.max()) + 1) * 128  # no record buffer is kept
+    assert oracle.as_set(got.pairs) == oracle.as_set(oracle.join(c.tokens, c.starts, c.sizes, 0.8))
+
+
+@pytest.mark.parametrize("builds", [0, 1, 2])
+def test_join_without_room_for_records(ctx, keep, builds):
+    """A first build, and one after `builds` others; R-S joins have two indexes."""
+    c = synth.generate(synth.C2, n_sets=12000, universe=9000, dup_frac=0.1, seed=31)
+    s = synth.generate(synth.C2, n_sets=13000, universe=9000, dup_frac=0.1, seed=32)
+    want = oracle.as_set(oracle.join(c.tokens, c.starts, c.sizes, 0.8))
+    want_rs = oracle.as_set(oracle.brute_rs((c.tokens, c.starts, c.sizes), (s.tokens, s.starts, s.sizes), 0.8))
+    S = keep(ctx.upload(s.tokens, s.sizes, s.starts))
+    ctx.rs_join(keep(ctx.upload(c.tokens, c.sizes, c.starts)), S, **PREFIX)
+    for join, exp in ((lambda x: ctx.self_join(x, **PREFIX), want), (lambda x: ctx.rs_join(x, S, **PREFIX), want_rs)):
+        def ready():
+            coll = keep(ctx.upload(c.tokens, c.sizes, c.starts))
+            for _ in range(builds):
+                join(coll)
+            return coll
+
+        def op(coll):
+            assert oracle.as_set(join(coll).pairs) == exp
+
+        went = outcomes(op, 60, ready)
+        if builds == 0:  # list offsets, entries, positions, signatures: records come after them
+            assert not went[0] and sum(not w for w in went) <= (4 if exp is want else 7)
+
+
+def test_host_join_without_room_for_records(ctx):
+    c = synth.generate(synth.C2, n_sets=12000, universe=9000, dup_frac=0.1, seed=31)
+    want = oracle.as_set(oracle.join(c.tokens, c.starts, c.sizes, 0.8))
+
+    def join():
+        return ctx.self_join_host(c.tokens, c.sizes, c.starts, **PREFIX)
+
+    for _ in range(3):
+        join()
+
+    def op(_):
+        assert oracle.as_set(join().pairs) == want
+
+    went = outcomes(op, 60)
+    assert False in went and True in went[:len(went) - 1 - went[::-1].index(False)]  # records are not the last buffer
