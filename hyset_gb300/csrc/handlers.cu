@@ -172,7 +172,8 @@ hyset_status check_block(hyset_ctx* ctx, const hyset_coll* c, const hyset_block*
 // id rule leaves out (probe block id below the indexed block's) hold no pair of
 // a candidate before its probe; its length filter leaves out no pair of the
 // result.  Blocks in another order, with gaps or with such ids go pair by pair,
-// as do ranges of so many prefix entries that one index would take gigabytes.
+// as do ranges of so many prefix entries that one index would take gigabytes,
+// and ranges for whose index the device has no room.
 bool joins_as_one(const hyset_handler* h, const hyset_block* first, uint32_t n_first, const hyset_block* second,
                   uint32_t n_second) {
     if (n_first == 0 || n_second == 0 || (uint64_t)n_first * n_second < 2) return false;
@@ -265,10 +266,15 @@ hyset_status hyset_handler_join_blocks(hyset_handler* h, const hyset_block* firs
 hyset_status hyset_handler_join_partitions(hyset_handler* h, const hyset_block* first, uint32_t n_first,
                                            const hyset_block* second, uint32_t n_second) {
     if (!h || (n_first && !first) || (n_second && !second)) return HYSET_E_INVALID;
-    if (joins_as_one(h, first, n_first, second, n_second)) return join_ranges(h, first[0].start_id,
-                                                                              first[n_first - 1].end_id + 1,
-                                                                              second[0].start_id,
-                                                                              second[n_second - 1].end_id + 1);
+    if (joins_as_one(h, first, n_first, second, n_second)) {
+        const hyset_status st = join_ranges(h, first[0].start_id, first[n_first - 1].end_id + 1, second[0].start_id,
+                                            second[n_second - 1].end_id + 1);
+        if (st != HYSET_E_NOMEM) return st;
+        // nothing has come out yet: what the range's index took goes back, and one
+        // block's index at a time does
+        for (DevBuf* b : {&h->part.list_off, &h->part.set, &h->part.pos, &h->part.rec}) b->release(h->ctx->stream);
+        h->ctx->sc->release(h->ctx->stream);
+    }
     // device::length_filter (device_algorithms.hpp:21-53): probe block id >= indexed
     // block id and size[last indexed] >= minsize(size[first probe]).
     for (uint32_t i = 0; i < n_first; ++i) {

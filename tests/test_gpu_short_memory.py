@@ -241,3 +241,24 @@ def test_host_join_without_room_for_records(ctx):
 
     went = outcomes(op, 60)
     assert False in went and True in went[:len(went) - 1 - went[::-1].index(False)]  # records are not the last buffer
+
+
+@pytest.mark.parametrize("tech,aggregate", [("fgss", False), ("fgss", True), ("bitmap", False)])
+def test_partitions_without_room_for_their_index(ctx, keep, tech, aggregate):
+    """Any one allocation may fail: the blocks are then joined pair by pair."""
+    c = synth.generate(synth.C2, n_sets=20_000, universe=15_000, dup_frac=0.1, seed=33)
+    want = oracle.as_set(oracle.join(c.tokens, c.starts, c.sizes, 0.8))
+    hc = hs.from_arrays(c.tokens, c.sizes, 5_000, 0.8)
+    coll = keep(ctx.upload(c.tokens, c.sizes, c.starts))
+    whole = hs.Partition(0, hc.blocks)
+    for n in range(1, 40):
+        own = keep(hs.Context(0)) if n < 25 else ctx  # with and without a context's scratch from earlier calls
+        mine = keep(own.upload(c.tokens, c.sizes, c.starts)) if own is not ctx else coll
+        h = keep(BitmapHandler(own, hc, mine, 64, 5_000, aggregate, 0.8) if tech == "bitmap"
+                 else FgssHandler(own, hc, mine, 5_000, aggregate, 0.8))
+        out = hs.CountHandler() if aggregate else hs.PairsHandler()
+        h.set_output_handler(out)
+        with failing(n if own is not ctx else n - 24):
+            h.join(whole, whole)
+        assert out.get_count() == len(want)
+        assert aggregate or oracle.as_set(out.pairs) == want
