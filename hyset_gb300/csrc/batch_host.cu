@@ -54,8 +54,9 @@ namespace {
 // as the joins (24 joins of up to 30,000 sets: 280 kernels, 2.0 of 4.5 ms).
 // They are captured on MAX_BRANCHES parallel branches of the graph, each with
 // a scratch of its own, together at most BRANCH_BYTES (one branch for joins
-// whose scratch alone is larger: their kernels fill the GPU).  That batch with
-// 1 / 4 / 8 / 16 branches: 2.92 / 2.13 / 2.02 / 1.87 ms a call.
+// whose scratch alone is larger: their kernels fill the GPU), and fewer where
+// the device has no room.  That batch with 1 / 4 / 8 / 16 branches: 2.92 / 2.13 /
+// 2.02 / 1.87 ms a call.
 constexpr uint32_t MAX_BRANCHES = 16;
 constexpr size_t BRANCH_BYTES = 2ull << 30;
 
@@ -290,18 +291,26 @@ hyset_status batch_prepare(hyset_ctx* ctx, const hyset_join_desc* joins, uint32_
     const size_t scan_words = std::max(std::max(scan_scratch_words(maxN), scan_scratch_words(maxU)),
                                        radix_scratch_words(maxE));
     const size_t per_branch = 8 * (size_t)maxN + 6 * e4 + 4 * ((size_t)maxU + scan_words);
-    const uint32_t branches =
+    const uint32_t wanted =
         std::max<uint32_t>(1, (uint32_t)std::min<uint64_t>({MAX_BRANCHES, n, (uint64_t)(BRANCH_BYTES / per_branch)}));
-    ST(side_streams(ctx, branches));
-    plan->sc.resize(branches);
-    for (Scratch& sc : plan->sc) {
+    auto scratch = [&](Scratch& sc) -> hyset_status {
         CK(sc.len.ensure((size_t)maxN * 4 + 4, s));
         CK(sc.off.ensure((size_t)maxN * 4 + 4, s));
         for (DevBuf* d : {&sc.tok, &sc.set, &sc.pos, &sc.order, &sc.altk, &sc.altv}) CK(d->ensure(e4, s));
         CK(sc.gate.ensure(4, s));
         CK(sc.counts.ensure((size_t)maxU * 4, s));
         CK(sc.scan.ensure(scan_words * 4, s));
-    }
+        return HYSET_OK;
+    };
+    plan->sc.resize(wanted);
+    ST(scratch(plan->sc[0]));
+    for (uint32_t k = 1; k < plan->sc.size(); ++k)
+        if (scratch(plan->sc[k]) != HYSET_OK) {  // as many branches as have room
+            plan->sc[k].release(s);
+            plan->sc.resize(k);
+        }
+    const uint32_t branches = (uint32_t)plan->sc.size();
+    ST(side_streams(ctx, branches));
     // each join to the branch with the least to build, the largest first
     plan->branch.assign(n, 0);
     {

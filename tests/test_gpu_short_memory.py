@@ -262,3 +262,32 @@ def test_partitions_without_room_for_their_index(ctx, keep, tech, aggregate):
             h.join(whole, whole)
         assert out.get_count() == len(want)
         assert aggregate or oracle.as_set(out.pairs) == want
+
+
+def test_batch_with_room_for_fewer_branches(ctx, keep):
+    """Five joins: five scratches, the first of which is needed."""
+    c = synth.generate(synth.C2, n_sets=3000, universe=2000, dup_frac=0.05, seed=77)
+    coll = keep(ctx.upload(c.tokens, c.sizes, c.starts))
+    taus = (0.6, 0.65, 0.7, 0.8, 0.9)
+    joins = [(coll, None, dict(threshold=t, technique="fgss", probe_major=True, bitmap=64)) for t in taus]
+    want = [oracle.as_set(oracle.join(c.tokens, c.starts, c.sizes, t)) for t in taus]
+    bytes_now = hs._lib.load().hyset_device_bytes
+    ctx.batch_join(joins)  # the bound tables, and the plan's whole size
+    held = bytes_now()
+    plain = keep(ctx.upload(c.tokens, c.sizes, c.starts))
+    less, failed = 0, 0
+    for n in range(1, 90):
+        ctx.batch_join([(plain, None, dict(threshold=0.95))])  # another batch: the plan is made again
+        with failing(n):
+            try:
+                got = ctx.batch_join(joins)
+            except hs.HysetError as e:
+                assert e.status == E_NOMEM
+                failed += 1
+                continue
+        assert [oracle.as_set(r.pairs) for r in got] == want
+        less = max(less, held - bytes_now())
+    # each join's lists, positions, entries, signatures and pairs, eleven arrays of the
+    # first scratch, and the plan's counts, counters, descriptors and units
+    assert failed == 5 * 5 + 11 + 4
+    assert less > 4 * 6 * 3000 * 4 // 2  # four scratches fewer, six arrays of the longest index's entries each
