@@ -143,7 +143,7 @@ hyset_status run_handler_join(hyset_handler* h, JoinParams P) {
             return HYSET_OK;
         }
         if (count <= h->cap) {
-            if (count <= early_pairs(h->cap, P.S.n)) {
+            if (count <= early_pairs(P)) {
                 const hyset_pair* early = static_cast<const hyset_pair*>(ctx->h_stage);
                 h->out_pairs.insert(h->out_pairs.end(), early, early + count);
             } else {

@@ -140,12 +140,13 @@ void split_heavy(const hyset_coll* S, const Bounds* b, JoinParams& P);
 // Behind a join's launch, before the host knows its number of pairs: orders
 // the pairs when asked (up to PAIR_SORT_MAX) and starts the copies of their
 // number (joined_count, after the stream has synchronised) and of the first
-// early_pairs of them: a sixteenth of the probes (most joins find fewer), 2,048
-// to 32,768 (256 KB cost a 70 us call 5 us).
+// `early` of them.  early_pairs: a sixteenth of the sets probed (most joins find
+// fewer), 2,048 to 32,768 (256 KB cost a 70 us call 5 us).
 constexpr uint64_t EARLY_PAIRS = 32768;
-uint64_t early_pairs(uint64_t cap, uint32_t n_probe);
+uint64_t early_pairs(uint64_t cap, uint32_t probed);
+uint64_t early_pairs(const JoinParams& P);
 PairSortJob pair_sort_job(const JoinParams& P);
-hyset_status enqueue_result(hyset_ctx* ctx, const Sink& out, uint32_t n_probe, const hyset_join_opts* o,
+hyset_status enqueue_result(hyset_ctx* ctx, const Sink& out, uint64_t early, const hyset_join_opts* o,
                             const PairSortJob* sort = nullptr);
 hyset_status enqueue_result(hyset_ctx* ctx, const JoinParams& P, const hyset_join_opts* o);
 uint64_t joined_count(const hyset_ctx* ctx);
@@ -160,7 +161,7 @@ hyset_status widen_window(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const Bo
 // The pairs of a finished join (res->count of them in the context's pair
 // buffer, enqueue_result done and the stream synchronised): sorted when asked,
 // left on the device or copied to the host.
-hyset_status deliver_pairs(hyset_ctx* ctx, const Sink& out, uint32_t n_probe, uint32_t n_indexed,
+hyset_status deliver_pairs(hyset_ctx* ctx, uint64_t early, uint32_t n_probe, uint32_t n_indexed,
                            const hyset_join_opts* o, hyset_result* res);
 hyset_status deliver_pairs(hyset_ctx* ctx, const JoinParams& P, const hyset_join_opts* o, hyset_result* res);
 hyset_status do_join(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const hyset_join_opts* o, hyset_result* res);

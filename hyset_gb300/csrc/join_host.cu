@@ -216,17 +216,20 @@ PairSortJob pair_sort_job(const JoinParams& P) {
                        (int)bits_for(P.out.swap ? P.S.n : P.R.n)};
 }
 
-uint64_t early_pairs(uint64_t cap, uint32_t n_probe) {
-    return std::min(cap, std::min<uint64_t>(EARLY_PAIRS, std::max<uint64_t>(2048, n_probe / 16)));
+uint64_t early_pairs(uint64_t cap, uint32_t probed) {
+    return std::min(cap, std::min<uint64_t>(EARLY_PAIRS, std::max<uint64_t>(2048, probed / 16)));
 }
 
-hyset_status enqueue_result(hyset_ctx* ctx, const Sink& out, uint32_t n_probe, const hyset_join_opts* o,
+uint64_t early_pairs(const JoinParams& P) {  // (a join of exchanged roles has no probe range)
+    return early_pairs(P.out.cap, P.out.swap ? P.R.n : P.p_hi - P.p_lo);
+}
+
+hyset_status enqueue_result(hyset_ctx* ctx, const Sink& out, uint64_t early, const hyset_join_opts* o,
                             const PairSortJob* sort) {
     cudaStream_t s = ctx->stream;
     if (sort && !o->count_only && o->sort_pairs) CK(sort_pairs_cluster(*sort, s));
     CK(cudaMemcpyAsync(ctx->h_flags + 16, out.count, 8, cudaMemcpyDeviceToHost, s));
     if (!o->count_only && !o->device_pairs) {
-        const uint64_t early = early_pairs(out.cap, n_probe);
         void* stage = nullptr;
         ST(host_stage(ctx, early * sizeof(hyset_pair), &stage));
         if (early) CK(cudaMemcpyAsync(stage, out.pairs, early * sizeof(hyset_pair), cudaMemcpyDeviceToHost, s));
@@ -236,7 +239,7 @@ hyset_status enqueue_result(hyset_ctx* ctx, const Sink& out, uint32_t n_probe, c
 
 hyset_status enqueue_result(hyset_ctx* ctx, const JoinParams& P, const hyset_join_opts* o) {
     const PairSortJob sort = pair_sort_job(P);
-    return enqueue_result(ctx, P.out, P.out.swap ? P.R.n : P.S.n, o, &sort);
+    return enqueue_result(ctx, P.out, early_pairs(P), o, &sort);
 }
 
 uint64_t joined_count(const hyset_ctx* ctx) {
@@ -259,10 +262,10 @@ hyset_status read_pairs(hyset_ctx* ctx, const void* d_pairs, uint64_t count, std
 }
 
 hyset_status deliver_pairs(hyset_ctx* ctx, const JoinParams& P, const hyset_join_opts* o, hyset_result* res) {
-    return deliver_pairs(ctx, P.out, P.out.swap ? P.R.n : P.S.n, P.out.swap ? P.S.n : P.R.n, o, res);
+    return deliver_pairs(ctx, early_pairs(P), P.out.swap ? P.R.n : P.S.n, P.out.swap ? P.S.n : P.R.n, o, res);
 }
 
-hyset_status deliver_pairs(hyset_ctx* ctx, const Sink& out, uint32_t n_probe, uint32_t n_indexed,
+hyset_status deliver_pairs(hyset_ctx* ctx, uint64_t early, uint32_t n_probe, uint32_t n_indexed,
                            const hyset_join_opts* o, hyset_result* res) {
     if (o->count_only) return HYSET_OK;
     const bool resort = o->sort_pairs && res->count > PAIR_SORT_MAX;  // not sorted behind the join
@@ -273,9 +276,9 @@ hyset_status deliver_pairs(hyset_ctx* ctx, const Sink& out, uint32_t n_probe, ui
         res->device_pairs = ctx->s_pairs.p;
         return HYSET_OK;
     }
-    if (!resort && res->count <= early_pairs(out.cap, n_probe)) {  // all of them have come with their number
-        const hyset_pair* early = static_cast<const hyset_pair*>(ctx->h_stage);
-        res->pairs.assign(early, early + res->count);
+    if (!resort && res->count <= early) {  // all of them have come with their number
+        const hyset_pair* staged = static_cast<const hyset_pair*>(ctx->h_stage);
+        res->pairs.assign(staged, staged + res->count);
     } else {
         ST(read_pairs(ctx, ctx->s_pairs.p, res->count, res->pairs));
     }

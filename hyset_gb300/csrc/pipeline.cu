@@ -488,6 +488,7 @@ hyset_status hyset_self_join_host(hyset_ctx* ctx, const uint32_t* tokens, uint64
             SP.R_L = C->max_size;
             SP.self = 1;
             SP.grab = std::min<uint32_t>(tn.batch, 32);
+            SP.p_hi = n;
             SP.r_lo = 0;
             SP.r_hi = n;
             SP.X = ix.view();

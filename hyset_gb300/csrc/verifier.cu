@@ -311,7 +311,7 @@ hyset_status hyset_verify_device(hyset_ctx* ctx, const hyset_coll* indexed, cons
         CK(launch_verify_candidates(R->view(), S->view(), b->view, d_probes, d_offsets, d_candidates, n_probes, vmode,
                                     sk, ctx->s_count.as<unsigned int>() + 4, ctx->sm_count, s, sig_r, sig_s, words));
         CK(cudaEventRecord(ctx->ek1, s));
-        ST(enqueue_result(ctx, sk, n_probes, &ro));
+        ST(enqueue_result(ctx, sk, early_pairs(sk.cap, n_probes), &ro));
         CK(cudaStreamSynchronize(s));
         const uint64_t count = joined_count(ctx);
         float kms = 0, dms = 0;
@@ -326,8 +326,7 @@ hyset_status hyset_verify_device(hyset_ctx* ctx, const hyset_coll* indexed, cons
         cap = count + count / 8 + 1024;
         if (attempt == 1) return fail(ctx, HYSET_E_OVERFLOW, "pair buffer overflow after resize");
     }
-    ST(deliver_pairs(ctx, Sink{nullptr, nullptr, count_only ? 0ull : (unsigned long long)cap, count_only, 0}, n_probes, 0, &ro,
-                     res.get()));
+    ST(deliver_pairs(ctx, early_pairs(count_only ? 0 : cap, n_probes), n_probes, 0, &ro, res.get()));
     res->technique = words ? HYSET_TECH_BITMAP : HYSET_TECH_DIRECT;
     *out = res.release();
     return HYSET_OK;
