@@ -69,6 +69,9 @@ struct Bounds {
     // positional bound admits (the bound layout of token records)
     std::vector<uint32_t> lp_row, lp_tab;
     bool mo_monotone = false;  // minoverlap non-decreasing in each length (R-S bands are valid)
+    // sizes from which signatures of 1, 2, 4 and 8 words are split finer and are
+    // filled (split_window, widen_window; L + 1: none, 0: not looked for yet)
+    mutable uint32_t split_size[4] = {0, 0, 0, 0}, filled_size[4] = {0, 0, 0, 0};
     std::vector<uint64_t> mo_row;
     DevBuf dev;
     BoundsView view{};
