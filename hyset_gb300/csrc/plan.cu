@@ -519,6 +519,7 @@ hyset_status autotune_bits(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const h
         } else {
             ST(sample(2, &warp_ms));
             if (warp_ms < TUNE_VMODE_MARGIN * cur_ms && cur_ms <= TUNE_BATCH_FULL_MS) {
+                ST(whole(1, base_batch, &whole_ms));  // the range's first run warms the caches: not kept
                 ST(whole(1, base_batch, &whole_ms));
                 cur_ms = whole_ms;
                 ST(whole(2, base_batch, &warp_ms));
