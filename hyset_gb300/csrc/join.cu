@@ -188,6 +188,21 @@ cudaError_t dispatch_words(const JoinParams& P, int sm_count, cudaStream_t s) {
 
 }  // namespace
 
+// A tile's probes of different sizes are compared one after the other and its
+// survivors merged by the few warps that found them, so a launch of few tiles
+// lasts as long as one of them; a warp per probe fills the GPU sooner.  Kernel of
+// k_window / enumeration in us, by probes x candidates (250 x 250 short sets,
+// cosine 0.6, 64 bits: 87 / 24; 500 plain sets, Jaccard 0.95: 15 / 11), and as the
+// mean ratio over three shapes of set and seven thresholds:
+//   64 to 256 bits: self-joins 0.64M 1.11, 1.2M 1.00, 1.7M 0.97, 3.2M 0.84,
+//                   R-S joins 0.64M 1.24, 1.7M 1.08, 2.6M 1.02, 4.8M 0.94;
+//   512 bits:       self-joins 0.36M 1.28, 0.64M 1.12, 1.2M 0.95,
+//                   R-S joins 0.42M 1.13, 0.56M 1.04, 0.81M 0.91.
+static bool small_window(const JoinParams& P) {
+    const uint64_t pairs = (uint64_t)(P.p_hi - P.p_lo) * (P.r_hi > P.r_lo ? P.r_hi - P.r_lo : 0u);
+    return pairs < (P.words > 4 ? 3ull << 18 : P.self ? 5ull << 18 : 3ull << 20);
+}
+
 uint32_t join_resident_warps(int sm_count) { return (uint32_t)sm_count * HS_JOIN_MIN_BLOCKS * JOIN_WARPS; }
 
 cudaError_t launch_join(const JoinParams& P, int technique, int vmode, int sm_count, cudaStream_t s) {
@@ -196,8 +211,9 @@ cudaError_t launch_join(const JoinParams& P, int technique, int vmode, int sm_co
         return vmode == 2 ? dispatch_words<TECH_FGSS, 2>(P, sm_count, s) : dispatch_words<TECH_FGSS, 1>(P, sm_count, s);
     // signatures over the windows: tiles of probes (window.cu), whose lanes do
     // not count their work; the enumeration kernel serves a launch with work
-    // counters and DIRECT, which has no signatures
-    if (technique == TECH_BITMAP && P.bits_R && P.words && !P.stats) return launch_window(P, vmode, sm_count, s);
+    // counters, DIRECT, which has no signatures, and small joins
+    if (technique == TECH_BITMAP && P.bits_R && P.words && !P.stats && !small_window(P))
+        return launch_window(P, vmode, sm_count, s);
     JoinParams Q = P;
     if (technique == TECH_DIRECT) Q.bits_R = Q.bits_S = nullptr;
     return vmode == 2 ? dispatch_words<TECH_BITMAP, 2>(Q, sm_count, s) : dispatch_words<TECH_BITMAP, 1>(Q, sm_count, s);

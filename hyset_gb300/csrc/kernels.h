@@ -293,7 +293,8 @@ uint32_t join_resident_warps(int sm_count);
 
 // ---- window.cu ---------------------------------------------------------------
 // The signature technique over the length windows (P.words in {1, 2, 4, 8},
-// signatures set, no work counters): one launch.
+// signatures set, no work counters): one launch.  launch_join takes it for all
+// but small joins.
 cudaError_t launch_window(const JoinParams& P, int vmode, int sm_count, cudaStream_t s);
 
 // ---- join_tm.cu ------------------------------------------------------------

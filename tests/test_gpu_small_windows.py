@@ -1,0 +1,61 @@
+"""Signature joins on both sides of the number of pairs from which on the tiled
+kernel takes them, by probe ranges of one collection: ranges that leave every
+remainder of a tile, one probe more and one less than the bound."""
+import numpy as np
+import pytest
+
+import oracle
+from hyset_gb300 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _set(p):
+    s = oracle.as_set(p)
+    assert len(s) == len(p), "duplicate pairs"
+    return s
+
+
+@pytest.mark.parametrize("bits", [64, 128, 256, 512])
+@pytest.mark.parametrize("sim,tau", [("jaccard", 0.6), ("cosine", 0.8)])
+def test_self_join_ranges(ctx, bits, sim, tau):
+    c = synth.generate(synth.C2, n_sets=16_384, universe=9_000, dup_frac=0.2, seed=bits)
+    coll = ctx.upload(c.tokens, c.sizes, c.starts)
+    want = np.array(sorted(oracle.as_set(oracle.join(c.tokens, c.starts, c.sizes, tau, sim=sim))))
+    bound = (3 << 18 if bits == 512 else 5 << 18) // c.n  # 48 or 80 probes
+    for lo in (0, 5_001, 12_000):
+        for np_ in (1, 15, 17, bound - 1, bound, bound + 1, 2 * bound + 5, 4 * bound - 1):
+            for mode in (1, 2):
+                got = ctx.self_join(coll, threshold=tau, sim=sim, technique="bitmap", bitmap=bits, verify_mode=mode,
+                                    probe_range=(lo, lo + np_))
+                rows = want[(want[:, 0] >= lo) & (want[:, 0] < lo + np_)]
+                assert _set(got.pairs) == set(map(tuple, rows.tolist()))
+    hi = c.n  # the longest sets
+    for np_ in (bound - 1, bound, bound + 9):
+        got = ctx.self_join(coll, threshold=tau, sim=sim, technique="bitmap", bitmap=bits, probe_range=(hi - np_, hi))
+        assert _set(got.pairs) == set(map(tuple, want[want[:, 0] >= hi - np_].tolist()))
+    coll.free()
+
+
+@pytest.mark.parametrize("bits", [64, 512])
+def test_rs_join_ranges(ctx, bits):
+    c = synth.generate(synth.C2, n_sets=11_192, universe=5_000, dup_frac=0.3, seed=3)
+    side = np.zeros(c.n, bool)
+    side[np.random.default_rng(1).choice(c.n, 8_192, replace=False)] = True
+    at = np.where(side, np.cumsum(side) - 1, np.cumsum(~side) - 1)  # in the halves' own numbers
+    want = np.array(sorted((int(at[b]), int(at[a])) if side[a] else (int(at[a]), int(at[b]))
+                           for a, b in oracle.as_set(oracle.join(c.tokens, c.starts, c.sizes, 0.6)) if side[a] != side[b]))
+    colls = []
+    for ids in (np.nonzero(side)[0], np.nonzero(~side)[0]):
+        colls.append(ctx.upload(np.concatenate([c.set(i) for i in ids]), c.sizes[ids]))
+    R, S = colls
+    bound = (3 << 18 if bits == 512 else 3 << 20) // 8_192  # 96 or 384 probes
+    assert len(want) > 500
+    for lo in (0, 1_001, 2_000):
+        for np_ in (1, bound - 1, bound, bound + 1, 2 * bound + 3):
+            got = ctx.rs_join(R, S, threshold=0.6, technique="bitmap", bitmap=bits, probe_range=(lo, lo + np_),
+                              orientation="as_given")
+            rows = want[(want[:, 0] >= lo) & (want[:, 0] < lo + np_)]
+            assert _set(got.pairs) == set(map(tuple, rows.tolist()))
+    R.free()
+    S.free()
