@@ -3,8 +3,7 @@
 // The device-resident form of the reference's block-pair work queue
 // (src/queue.cu:142-281, moodycamel ConcurrentQueue + one GPU consumer thread):
 // every join of a batch is split into work units (a batch of probes for the
-// prefix-index technique, one probe for the exhaustive one; signature joins are
-// launches of their own, window.cu);
+// prefix-index technique, one probe for the window-enumeration techniques);
 // the units of all joins form one flat range, and the warps of a single launch
 // steal units from it with one atomic each.  A unit finds its join by bisection
 // over the units' prefix offsets and runs that join's filter + verify with the
@@ -18,9 +17,8 @@ namespace hs {
 namespace {
 
 // Unit u of a join: a prefix-index join's longest probes go as slot segments
-// first (JoinParams::heavy_from), then its probe batches; the exhaustive
-// technique's units are single probes and have no signatures.  Items are
-// carried across a unit's slot rounds.
+// first (JoinParams::heavy_from), then its probe batches; a window technique's
+// units are single probes.  Items are carried across a unit's slot rounds.
 template <int W>
 __device__ __forceinline__ void run_unit(const BatchDesc& d, uint32_t u, uint32_t* sbuf, int lane) {
     const JoinParams& P = d.P;
@@ -40,8 +38,8 @@ __device__ __forceinline__ void run_unit(const BatchDesc& d, uint32_t u, uint32_
         ItemCarry ic;
         fgss_carry<1, W, false, false>(P, i0, k, lane, ic, jb, je);
         flush_items<1, W, false, false>(P, ic, lane);
-    } else if constexpr (W == 0) {
-        enum_probe<1, 0, false>(P, P.p_hi - 1 - u, sbuf, lane);
+    } else {
+        enum_probe<1, W, false>(P, P.p_hi - 1 - u, sbuf, lane);
     }
 }
 
