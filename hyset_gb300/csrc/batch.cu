@@ -3,7 +3,8 @@
 // The device-resident form of the reference's block-pair work queue
 // (src/queue.cu:142-281, moodycamel ConcurrentQueue + one GPU consumer thread):
 // every join of a batch is split into work units (a batch of probes for the
-// prefix-index technique, one probe for the window-enumeration techniques);
+// prefix-index technique, one probe for the exhaustive one and for small
+// signature joins; large ones are launches of their own, window.cu);
 // the units of all joins form one flat range, and the warps of a single launch
 // steal units from it with one atomic each.  A unit finds its join by bisection
 // over the units' prefix offsets and runs that join's filter + verify with the
@@ -17,8 +18,9 @@ namespace hs {
 namespace {
 
 // Unit u of a join: a prefix-index join's longest probes go as slot segments
-// first (JoinParams::heavy_from), then its probe batches; a window technique's
-// units are single probes.  Items are carried across a unit's slot rounds.
+// first (JoinParams::heavy_from), then its probe batches; the window
+// techniques' units are single probes.  Items are carried across a unit's slot
+// rounds.
 template <int W>
 __device__ __forceinline__ void run_unit(const BatchDesc& d, uint32_t u, uint32_t* sbuf, int lane) {
     const JoinParams& P = d.P;

@@ -58,6 +58,12 @@ namespace {
 // the device has no room.  That batch with 1 / 4 / 8 / 16 branches: 2.92 / 2.13 /
 // 2.02 / 1.87 ms a call.
 constexpr uint32_t MAX_BRANCHES = 16;
+// Signature joins of fewer pairs (probes x candidates) are units of the shared
+// launch, a warp per probe, the others launches of their own (launch_join).  A
+// batch of one such join of plain / short / long sets at Jaccard 0.8 and 64 bits,
+// in us, shared and own: 2,000 sets (4M) 23 / 20 / 63 and 26 / 34 / 69, 6,000 sets
+// (36M) 41 / 32 / 122 and 27 / 35 / 120, 24,000 sets 170 / 162 / 516 and 54 / 61 / 610.
+constexpr uint64_t WINDOW_PAIRS = 8ull << 20;
 constexpr size_t BRANCH_BYTES = 2ull << 30;
 
 // While it lives, the context's stream and scratch are a branch's.
@@ -89,9 +95,9 @@ hyset_status side_streams(hyset_ctx* ctx, size_t n) {
     return HYSET_OK;
 }
 
-// A join's index and signatures on the context's stream; a signature-technique
-// join runs there too (k_window over its own launch: in the shared launch each
-// of its probes was a unit that one warp walked).
+// A join's index and signatures on the context's stream; a large
+// signature-technique join runs there too (in the shared launch each of its
+// probes would be a unit that one warp walks).
 hyset_status build_batch_join(hyset_ctx* ctx, BatchPlan& bp, uint32_t k) {
     BatchJoin& bj = *bp.joins[bp.order[k]];
     if (bj.ktech == TECH_FGSS) {
@@ -150,8 +156,9 @@ hyset_status batch_record(hyset_ctx* ctx, BatchPlan& bp) {
         P.work = bp.work.as<unsigned int>() + 4 + 4 * k;
         CK(launch_join(P, TECH_FGSS, bj.vmode, ctx->sm_count, s));
     }
-    CK(launch_batch_join(bp.desc.as<BatchDesc>(), bp.unit_off.as<uint32_t>(), n, bp.work.as<unsigned int>(),
-                         ctx->sm_count, s));
+    if (bp.units)
+        CK(launch_batch_join(bp.desc.as<BatchDesc>(), bp.unit_off.as<uint32_t>(), n, bp.work.as<unsigned int>(),
+                             ctx->sm_count, s));
     CK(sort_pairs_clusters(bp.sorts.as<PairSortJob>(), bp.n_sorts, s));
     return HYSET_OK;
 }
@@ -277,7 +284,7 @@ hyset_status batch_prepare(hyset_ctx* ctx, const hyset_join_desc* joins, uint32_
             const uint32_t hf = std::max(P.heavy_from, P.p_lo);
             nheavy = P.p_hi > hf ? P.p_hi - hf : 0u;
         }
-        bj->window = bj->ktech == TECH_BITMAP && bj->words > 0;
+        bj->window = bj->ktech == TECH_BITMAP && bj->words > 0 && (uint64_t)np * R->n >= WINDOW_PAIRS;
         bj->units = bj->solo || bj->window ? 0u : nheavy * P.segs + (np - nheavy + desc[j].unit_probes - 1) / desc[j].unit_probes;
         if (bj->ktech == TECH_BITMAP) build[j] += (double)np * (double)R->n / 64.0;  // its pairs, at a token's cost each 64
         if (bj->words) build[j] += (double)R->n_tokens + (bj->self ? 0.0 : (double)S->n_tokens);
@@ -343,6 +350,7 @@ hyset_status batch_prepare(hyset_ctx* ctx, const hyset_join_desc* joins, uint32_
         unit_off[k + 1] = unit_off[k] + bj.units;
         if (bj.o.sort_pairs && !bj.o.count_only) sorts.push_back(pair_sort_job(ordered[k].P));
     }
+    plan->units = unit_off[n];
     plan->host_desc = ordered;
     CK(plan->desc.ensure(n * sizeof(BatchDesc), s));
     CK(plan->unit_off.ensure((n + 1) * 4, s));

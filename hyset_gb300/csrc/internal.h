@@ -135,7 +135,7 @@ struct BatchJoin {
     // graph (the single-join kernel: token records, carried items), not in the
     // shared launch
     bool solo = false;
-    bool window = false;  // a signature-technique join: a launch of its own on its branch of the graph
+    bool window = false;  // a large signature-technique join: launches of its own on its branch of the graph
     int vmode = 1;
     uint32_t batch = 3;
 };
@@ -159,6 +159,7 @@ struct BatchPlan {
     std::vector<std::unique_ptr<BatchJoin>> joins;
     std::vector<uint32_t> order;  // joins[order[k]] is descriptor k (heaviest first)
     DevBuf desc, unit_off, counts, work, sorts;
+    uint32_t units = 0;    // of the shared launch, all joins together
     uint32_t n_sorts = 0;  // joins whose pairs are put in order by the graph (sorts: their PairSortJobs)
     std::vector<BatchDesc> host_desc;  // the joins' descriptors in launch order (solo joins launch from them)
     cudaGraph_t graph = nullptr;
