@@ -34,6 +34,7 @@ void release_plan(hyset_ctx* ctx, BatchPlan& bp) {
         DevBuf* bufs[] = {&bj->ix.list_off, &bj->ix.set, &bj->ix.pos, &bj->ix_mid.list_off, &bj->ix_mid.set,
                           &bj->ix_mid.pos, &bj->ix.rec, &bj->ix_mid.rec, &bj->bits_r, &bj->bits_s, &bj->pairs};
         for (DevBuf* d : bufs) d->release(s);
+        for (DevBuf* d : {&bj->wide_r[0], &bj->wide_r[1], &bj->wide_s[0], &bj->wide_s[1]}) d->release(s);
     }
     DevBuf* bufs[] = {&bp.desc, &bp.unit_off, &bp.counts, &bp.work, &bp.sorts};
     for (DevBuf* d : bufs) d->release(s);
@@ -61,8 +62,10 @@ constexpr uint32_t MAX_BRANCHES = 16;
 // Signature joins of fewer pairs (probes x candidates) are units of the shared
 // launch, a warp per probe, the others launches of their own (launch_join).  A
 // batch of one such join of plain / short / long sets at Jaccard 0.8 and 64 bits,
-// in us, shared and own: 2,000 sets (4M) 23 / 20 / 63 and 26 / 34 / 69, 6,000 sets
-// (36M) 41 / 32 / 122 and 27 / 35 / 120, 24,000 sets 170 / 162 / 516 and 54 / 61 / 610.
+// in us, shared and own: 2,000 sets (4M) 23 / 20 / 63 and 21 / 29 / 64, 6,000 sets
+// (36M) 41 / 32 / 122 and 22 / 30 / 113, 24,000 sets 170 / 162 / 516 and 49 / 53 / 220.
+// (The own ones' longest sets take wider signatures, cut_window; at 64 bits alone
+// 12,000 / 24,000 long sets took 309 / 601, now 172 / 220.)
 constexpr uint64_t WINDOW_PAIRS = 8ull << 20;
 constexpr size_t BRANCH_BYTES = 2ull << 30;
 
@@ -110,10 +113,14 @@ hyset_status build_batch_join(hyset_ctx* ctx, BatchPlan& bp, uint32_t k) {
         CK(generate_signatures(bj.R, bj.words, bj.bits_r.as<uint64_t>(), ctx->stream));
         if (!bj.self) CK(generate_signatures(bj.S, bj.words, bj.bits_s.as<uint64_t>(), ctx->stream));
     }
-    if (bj.window) {
-        JoinParams P = bp.host_desc[k].P;
-        P.work = bp.work.as<unsigned int>() + 4 + 4 * k;
-        split_window(bj.R, bj.S, bj.b, bj.words, P);
+    for (size_t i = 0; i < bj.parts.size(); ++i) {  // up to three launches, a counter each
+        JoinParams P = bj.parts[i];
+        if (P.words != bj.words) {
+            CK(generate_signatures(bj.R, P.words, bj.wide_r[P.words / 8].as<uint64_t>(), ctx->stream));
+            if (!bj.self) CK(generate_signatures(bj.S, P.words, bj.wide_s[P.words / 8].as<uint64_t>(), ctx->stream));
+        }
+        P.out = bp.host_desc[k].P.out;
+        P.work = bp.work.as<unsigned int>() + 4 + 4 * k + i;
         CK(launch_join(P, TECH_BITMAP, 1, ctx->sm_count, ctx->stream));
     }
     return HYSET_OK;
@@ -285,6 +292,24 @@ hyset_status batch_prepare(hyset_ctx* ctx, const hyset_join_desc* joins, uint32_
             nheavy = P.p_hi > hf ? P.p_hi - hf : 0u;
         }
         bj->window = bj->ktech == TECH_BITMAP && bj->words > 0 && (uint64_t)np * R->n >= WINDOW_PAIRS;
+        if (bj->window) {
+            split_window(R, S, bj->b, bj->words, P);
+            cut_window(R, S, bj->b, P, bj->parts);
+            for (size_t i = 1; i < bj->parts.size(); ++i) {
+                JoinParams& W = bj->parts[i];
+                DevBuf& wr = bj->wide_r[W.words / 8];
+                DevBuf& ws = bj->wide_s[W.words / 8];
+                if (wr.ensure(sig_bytes(R->n, W.words), s) != cudaSuccess ||
+                    (!bj->self && ws.ensure(sig_bytes(S->n, W.words), s) != cudaSuccess)) {  // no room: the narrow ones
+                    while (bj->parts.size() > i) drop_widest(bj->parts);
+                    break;
+                }
+                W.bits_R = wr.as<uint64_t>();
+                W.bits_S = bj->self ? W.bits_R : ws.as<uint64_t>();
+                build[j] += (double)R->n_tokens + (bj->self ? 0.0 : (double)S->n_tokens);
+            }
+            order_widths(bj->parts);
+        }
         bj->units = bj->solo || bj->window ? 0u : nheavy * P.segs + (np - nheavy + desc[j].unit_probes - 1) / desc[j].unit_probes;
         if (bj->ktech == TECH_BITMAP) build[j] += (double)np * (double)R->n / 64.0;  // its pairs, at a token's cost each 64
         if (bj->words) build[j] += (double)R->n_tokens + (bj->self ? 0.0 : (double)S->n_tokens);

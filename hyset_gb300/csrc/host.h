@@ -153,9 +153,16 @@ uint64_t joined_count(const hyset_ctx* ctx);
 // The signature technique's probes that are taken in small units
 // (JoinParams::heavy_from, heavy_lo); words: 64-bit words per signature.
 void split_window(const hyset_coll* R, const hyset_coll* S, const Bounds* b, int words, JoinParams& P);
-// A signature join whose probes of full signatures are taken by wider ones:
-// one launch's parameters per width, the widest first (empty: P alone).  The
-// wider signatures are generated on `gen`.
+// A signature join whose probes of full signatures are taken by wider ones: one
+// launch's parameters per width, P's own first (P alone: one), the wider ones'
+// signatures yet to be set.  drop_widest: the last width's probes go to the one
+// before it; order_widths: the widest first, without empty ranges.
+void cut_window(const hyset_coll* R, const hyset_coll* S, const Bounds* b, const JoinParams& P,
+                std::vector<JoinParams>& parts);
+void drop_widest(std::vector<JoinParams>& parts);
+void order_widths(std::vector<JoinParams>& parts);
+// The same for a join with the collections' own signature buffers (one width:
+// empty); the wider signatures are generated on `gen`.
 hyset_status widen_window(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const Bounds* b, const JoinParams& P,
                           cudaStream_t gen, std::vector<JoinParams>& parts);
 // The pairs of a finished join (res->count of them in the context's pair

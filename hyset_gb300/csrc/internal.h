@@ -136,6 +136,8 @@ struct BatchJoin {
     // shared launch
     bool solo = false;
     bool window = false;  // a large signature-technique join: launches of its own on its branch of the graph
+    std::vector<hs::JoinParams> parts;  // these launches (without outputs and counters), the widest signatures first
+    DevBuf wide_r[2], wide_s[2];        // their signatures of 4 and 8 words where the join's own are narrower
     int vmode = 1;
     uint32_t batch = 3;
 };

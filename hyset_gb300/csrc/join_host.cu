@@ -187,8 +187,8 @@ static uint32_t filled_from(const Bounds* b, int words) {
 // generation and launch cost (at half as many, joins of 8,000 long sets lost
 // 10 to 20 us; with 128 bits between 64 and 256, 100,000 long sets took 3.3 ms
 // instead of 2.8 at cosine 0.75).
-hyset_status widen_window(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const Bounds* b, const JoinParams& P,
-                          cudaStream_t gen, std::vector<JoinParams>& parts) {
+void cut_window(const hyset_coll* R, const hyset_coll* S, const Bounds* b, const JoinParams& P,
+                std::vector<JoinParams>& parts) {
     constexpr uint64_t WIDE_PAIRS = 16ull << 20;
     parts.assign(1, P);
     for (int words = std::max(4, 2 * P.words); words <= 8; words *= 2) {
@@ -198,29 +198,49 @@ hyset_status widen_window(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const Bo
         if (from >= P.p_hi) break;
         const uint32_t least = std::min(b->minsize[size_at(S, from)], R->max_size + 1);
         if ((uint64_t)(P.p_hi - from) * (R->n - R->h_first_ge[least]) < WIDE_PAIRS) break;
-        // without room for them the narrow ones do
-        if (R->bitmaps[words].ensure(sig_bytes(R->n, words), ctx->stream) != cudaSuccess ||
-            (S != R && S->bitmaps[words].ensure(sig_bytes(S->n, words), ctx->stream) != cudaSuccess)) {
-            (void)cudaGetLastError();
-            break;
-        }
         JoinParams W = P;
-        const uint64_t *br = nullptr, *bs = nullptr;
-        ST(get_bitmaps(ctx, R, words, &br, gen));
-        if (S == R) bs = br;
-        else ST(get_bitmaps(ctx, S, words, &bs, gen));
-        W.bits_R = br;
-        W.bits_S = bs;
+        W.bits_R = W.bits_S = nullptr;
         W.words = words;
         W.p_lo = from;
         split_window(R, S, b, words, W);
         parts.back().p_hi = from;
         parts.push_back(W);
     }
-    if (parts.size() == 1) parts.clear();
+}
+
+void drop_widest(std::vector<JoinParams>& parts) {
+    const uint32_t hi = parts.back().p_hi;
+    parts.pop_back();
+    parts.back().p_hi = hi;
+}
+
+void order_widths(std::vector<JoinParams>& parts) {
     std::reverse(parts.begin(), parts.end());  // the longest sets first
     parts.erase(std::remove_if(parts.begin(), parts.end(), [](const JoinParams& q) { return q.p_lo >= q.p_hi; }),
                 parts.end());
+}
+
+hyset_status widen_window(hyset_ctx* ctx, hyset_coll* R, hyset_coll* S, const Bounds* b, const JoinParams& P,
+                          cudaStream_t gen, std::vector<JoinParams>& parts) {
+    cut_window(R, S, b, P, parts);
+    auto room = [&](hyset_coll* c, int words) {
+        return c->bitmaps[words].ensure(sig_bytes(c->n, words), ctx->stream) == cudaSuccess;
+    };
+    for (size_t k = 1; k < parts.size(); ++k) {
+        JoinParams& W = parts[k];
+        if (!room(R, W.words) || (S != R && !room(S, W.words))) {  // without room for them the narrow ones do
+            while (parts.size() > k) drop_widest(parts);
+            break;
+        }
+        const uint64_t *br = nullptr, *bs = nullptr;
+        ST(get_bitmaps(ctx, R, W.words, &br, gen));
+        if (S == R) bs = br;
+        else ST(get_bitmaps(ctx, S, W.words, &bs, gen));
+        W.bits_R = br;
+        W.bits_S = bs;
+    }
+    if (parts.size() == 1) parts.clear();
+    order_widths(parts);
     return HYSET_OK;
 }
 

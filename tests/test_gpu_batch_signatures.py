@@ -2,8 +2,10 @@
 launches of their own, at every width, beside joins of the other techniques."""
 import pytest
 
+import hyset_gb300 as hs
 import oracle
 from hyset_gb300 import synth
+from test_gpu_short_memory import failing
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +54,33 @@ def test_rs_signature_joins(ctx, n_r, n_s):
             assert _set(r.pairs) == want
     R.free()
     S.free()
+
+
+@pytest.mark.parametrize("bits", [64, 128, 256])
+def test_joins_in_three_widths(ctx, bits):
+    """Long sets whose probes fill their signatures, as in test_gpu_window_three_widths.py, beside small ones."""
+    tau = 0.5
+    big = synth.generate(synth.C3, n_sets=24_001, universe=24_000, seed=5)
+    small = synth.generate(synth.C3, n_sets=1_500, universe=3_000, seed=6)
+    B, A = ctx.upload(big.tokens, big.sizes, big.starts), ctx.upload(small.tokens, small.sizes, small.starts)
+    want = oracle.as_set(oracle.join(big.tokens, big.starts, big.sizes, tau))
+    want_a = oracle.as_set(oracle.join(small.tokens, small.starts, small.sizes, tau))
+    want_rs = oracle.as_set(oracle.brute_rs((small.tokens, small.starts, small.sizes),
+                                            (big.tokens, big.starts, big.sizes), tau))
+    kw = dict(threshold=tau, technique="bitmap", bitmap=bits)
+    joins = [(B, None, kw), (A, None, kw), (A, B, kw), (B, None, dict(kw, probe_range=(20_000, 24_001)))]
+    for _ in range(2):
+        got = [_set(r.pairs) for r in ctx.batch_join(joins)]
+        assert got == [want, want_a, want_rs, {p for p in want if p[0] >= 20_000}]
+    wider = {64: (3, 4), 128: (3, 4), 256: (3,)}[bits]  # the allocations after the join's own signatures and its pairs
+    for k in range(1, 30):
+        ctx.batch_join([(A, None, dict(threshold=0.9))])  # another batch: the plan is made again
+        with failing(k):
+            try:
+                got = ctx.batch_join([(B, None, kw)])
+            except hs.HysetError as e:
+                assert e.status == 3 and k not in wider
+                continue
+        assert _set(got[0].pairs) == want
+    B.free()
+    A.free()
