@@ -803,9 +803,9 @@ __global__ void __launch_bounds__(BITMAP_THREADS) k_validate_bitmaps(CollView c,
     }
 }
 
-// Whether the l tokens at t ascend strictly, LPS lanes (g: the lane's place)
-// with VALIDATE_UNROLL pairs of loads in flight each (a token's successor is an
-// L1 hit); every lane sees its own part.
+// Whether the l tokens at t fail to ascend strictly somewhere, LPS lanes (g: the
+// lane's place) with VALIDATE_UNROLL pairs of loads in flight each (a token's
+// successor is an L1 hit); every lane sees its own part.
 template <int LPS>
 __device__ __forceinline__ bool unordered(const uint32_t* __restrict__ t, uint32_t l, int g) {
     bool bad = false;
@@ -823,18 +823,21 @@ __device__ __forceinline__ bool unordered(const uint32_t* __restrict__ t, uint32
     return bad;
 }
 
-// A warp per four sets, eight lanes each, or the whole warp one after the
-// other when one of them has 128 tokens or more: checks the input contract and
-// writes the sets' (start, size) pairs.  The largest token is kept per lane and
-// reduced once per warp, so the kernel makes one atomic per warp, not one per
-// set.  (A warp per set had one pair of loads per lane in flight: 44 us for
-// 200,000 long sets, 2 TB/s.)
+// A warp per four sets, eight lanes each (LPS 8; the whole warp one after the
+// other when one of them has 128 tokens or more), or a warp per set (LPS 32):
+// checks the input contract and writes the sets' (start, size) pairs.  The
+// largest token is kept per lane and reduced once per warp, so the kernel makes
+// one atomic per warp, not one per set.  (A warp per set and one pair of loads
+// per lane in flight: 44 us for 200,000 long sets, 2 TB/s.)
+template <int LPS>
 __global__ void __launch_bounds__(256) k_validate(CollView c, uint64_t n_tokens, uint32_t* flags, uint2* meta) {
-    const int lane = threadIdx.x & 31, g = lane & 7;
+    constexpr int SETS = 32 / LPS;
+    const int lane = threadIdx.x & 31, g = lane & (LPS - 1);
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     uint32_t f = 0, mx = 0;
-    for (uint64_t s0 = (uint64_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 4; s0 < c.n; s0 += (uint64_t)warps * 4) {
-        const uint64_t s = s0 + (lane >> 3);
+    for (uint64_t s0 = (uint64_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * SETS; s0 < c.n;
+         s0 += (uint64_t)warps * SETS) {
+        const uint64_t s = s0 + lane / LPS;
         uint32_t l = 0, st = 0;
         if (s < c.n) {
             l = c.sizes[s];
@@ -849,11 +852,11 @@ __global__ void __launch_bounds__(256) k_validate(CollView c, uint64_t n_tokens,
                 mx = max(mx, c.tokens[st + l - 1]);
             }
         }
-        if (__any_sync(FULL, l >= SIG_WARP_SIZE)) {
+        if (LPS < 32 && __any_sync(FULL, l >= SIG_WARP_SIZE)) {
 #pragma unroll 1
-            for (int q = 0; q < 4; ++q)
-                if (unordered<32>(c.tokens + __shfl_sync(FULL, st, q * 8), __shfl_sync(FULL, l, q * 8), lane)) f |= 2;
-        } else if (unordered<8>(c.tokens + st, l, g)) {
+            for (int q = 0; q < SETS; ++q)
+                if (unordered<32>(c.tokens + __shfl_sync(FULL, st, q * LPS), __shfl_sync(FULL, l, q * LPS), lane)) f |= 2;
+        } else if (unordered<LPS>(c.tokens + st, l, g)) {
             f |= 2;
         }
     }
@@ -1249,7 +1252,14 @@ cudaError_t sort_pair_list(uint2* pairs, uint64_t n, int first_bits, int second_
 cudaError_t validate_collection(CollView c, uint64_t n_tokens, uint32_t* flags, uint2* meta, cudaStream_t s) {
     if (c.n == 0) return cudaSuccess;
     note_launches();
-    k_validate<<<grid_for((uint64_t)c.n * 8, 256), 256, 0, s>>>(c, n_tokens, flags, meta);
+    // few sets of many tokens: four to a warp left most of the GPU idle (an upload of
+    // 500 / 2,000 / 4,000 / 6,000 / 9,000 long sets, mean 112, 63 / 68 / 78 / 82 / 93 us,
+    // a warp each 55 / 60 / 65 / 73 / 91; short sets, mean 29, the same up to 4,000 and
+    // 59 against 66 us at 6,000)
+    if (c.n <= 8192 && n_tokens >= 64ull * c.n)
+        k_validate<32><<<grid_for((uint64_t)c.n * 32, 256), 256, 0, s>>>(c, n_tokens, flags, meta);
+    else
+        k_validate<8><<<grid_for((uint64_t)c.n * 8, 256), 256, 0, s>>>(c, n_tokens, flags, meta);
     return cudaGetLastError();
 }
 
