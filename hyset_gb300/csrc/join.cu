@@ -192,15 +192,21 @@ cudaError_t dispatch_words(const JoinParams& P, int sm_count, cudaStream_t s) {
 // survivors merged by the few warps that found them, so a launch of few tiles
 // lasts as long as one of them; a warp per probe fills the GPU sooner.  Kernel of
 // k_window / enumeration in us, by probes x candidates (250 x 250 short sets,
-// cosine 0.6, 64 bits: 87 / 24; 500 plain sets, Jaccard 0.95: 15 / 11), and as the
-// mean ratio over three shapes of set and seven thresholds:
+// cosine 0.6, 64 bits: 87 / 24; 500 plain sets, Jaccard 0.95: 15 / 11).  Where
+// many probes are heavy, most pairs are verified and the tiles catch up sooner
+// (1,500 x 1,500 long sets, cosine 0.6, 64 bits: 330 / 520).  The bounds are those
+// that cost least over three shapes of set, seven thresholds and 20 sizes: on
+// average 3 % over the faster of the two, as a mean ratio of the two kernels
 //   64 to 256 bits: self-joins 0.64M 1.11, 1.2M 1.00, 1.7M 0.97, 3.2M 0.84,
 //                   R-S joins 0.64M 1.24, 1.7M 1.08, 2.6M 1.02, 4.8M 0.94;
 //   512 bits:       self-joins 0.36M 1.28, 0.64M 1.12, 1.2M 0.95,
 //                   R-S joins 0.42M 1.13, 0.56M 1.04, 0.81M 0.91.
 static bool small_window(const JoinParams& P) {
-    const uint64_t pairs = (uint64_t)(P.p_hi - P.p_lo) * (P.r_hi > P.r_lo ? P.r_hi - P.r_lo : 0u);
-    return pairs < (P.words > 4 ? 3ull << 18 : P.self ? 5ull << 18 : 3ull << 20);
+    const uint64_t probes = P.p_hi - P.p_lo, heavy = P.p_hi - std::max(P.p_lo, std::min(P.p_hi, P.heavy_from));
+    const uint64_t pairs = probes * (P.r_hi > P.r_lo ? P.r_hi - P.r_lo : 0u);
+    if (P.words > 4) return pairs < 3ull << 18;
+    if (P.self) return pairs < (4 * heavy >= probes ? 1ull << 18 : 5ull << 19);
+    return pairs < (2 * heavy >= probes ? 5ull << 17 : 3ull << 20);
 }
 
 uint32_t join_resident_warps(int sm_count) { return (uint32_t)sm_count * HS_JOIN_MIN_BLOCKS * JOIN_WARPS; }
