@@ -30,8 +30,8 @@ namespace hs {
 
 namespace {
 
-// BD: the index is token records in the bound layout (IndexView::bound;
-// prefix-index joins only).
+// BD: the index's entries, in records or lists, are in the bound layout
+// (IndexView::bound; prefix-index joins only).
 template <int TECH, int VMODE, int W, bool ST, bool BD = false>
 __global__ void __launch_bounds__(JOIN_THREADS, HS_JOIN_MIN_BLOCKS) k_join(JoinParams P) {
     extern __shared__ uint32_t smem[];

@@ -270,14 +270,14 @@ cudaError_t launch_window_w(const JoinParams& P, int sm_count, cudaStream_t s) {
     const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_window<VMODE, W>, WIN_THREADS, 0);
     if (e != cudaSuccess) return e;
     const uint32_t blocks = (uint32_t)(sm_count * std::max(per_sm, 1));
-    // units small enough that the blocks have several each, down to 16 probes x 1,024 candidates
     const uint64_t ncand = P.r_hi > P.r_lo ? P.r_hi - P.r_lo : 1;
     const uint32_t split = std::max(P.p_lo, std::min(P.p_hi, P.heavy_from));
     auto segments = [](uint64_t cands, uint32_t seg) { return (cands + 31 + seg - 1) / seg; };  // a window starts up to 31 ids early
     auto units = [&](uint64_t probes, uint64_t cands, uint32_t tile, uint32_t seg) {
         return (probes + tile - 1) / tile * segments(cands, seg);
     };
-    // small enough that the blocks have several each, down to 16 probes x 1,024 candidates
+    // units small enough that the blocks have several each: down to 16 probes x 1,024
+    // candidates, the heavy probes' down to one x 1,024 (below)
     WinCut rest{WIN_TILE, 8192, 0}, heavy{16, 1024, 0};
     const uint64_t np = split - P.p_lo, nh = P.p_hi - split;
     const uint64_t hcand = P.r_hi > std::max(P.r_lo, P.heavy_lo) ? P.r_hi - std::max(P.r_lo, P.heavy_lo) : 1;

@@ -84,7 +84,9 @@ typedef struct {
     uint32_t sort_pairs;       /* 1 = return pairs sorted by (first, second) */
     uint64_t pair_capacity;    /* initial device pair buffer; 0 = automatic (grows on demand) */
     uint32_t device_pairs;     /* 1 = leave the pairs in device memory (hyset_result_device_pairs) */
-    uint32_t collect_stats;    /* 1 = count filter work (hyset_result_stats); costs a few atomics */
+    uint32_t collect_stats;    /* 1 = count filter work (hyset_result_stats); costs a few atomics.  A
+                                  signature join is then run a warp per probe at the asked width
+                                  (as small ones are), and its counters and times are that kernel's */
     uint32_t probe_begin;      /* probe id range [probe_begin, probe_end) of this call; */
     uint32_t probe_end;        /* 0, 0 = every probe (a shard of a join, e.g. one rank's part) */
     uint32_t probe_major;      /* technique FGSS: 1 = probe-major kernel (set-id-sorted index, one warp
@@ -194,7 +196,10 @@ uint64_t hyset_result_count(const hyset_result* r);
 const hyset_pair* hyset_result_pairs(const hyset_result* r); /* NULL when count_only */
 hyset_technique hyset_result_technique(const hyset_result* r);
 uint32_t hyset_result_bitmap_bits(const hyset_result* r);   /* signature width used (0 = none) */
-uint32_t hyset_result_verify_mode(const hyset_result* r);   /* verification mode used (1 lane, 2 warp, 3 staged) */
+/* verification mode used (1 lane, 2 warp, 3 staged); of a host-input join the mode its
+ * whole range was given: its pieces that reach sets of 1,000 tokens verify with warps
+ * where verify_mode was 0 */
+uint32_t hyset_result_verify_mode(const hyset_result* r);
 /* Probes per warp batch of the probe-major prefix-filter kernel (the tile the
  * reference sizes with --block for its block-pair launches, src/fgss.cu and
  * device_algorithms.hpp:147-148); 0 when the join ran another kernel.  With
