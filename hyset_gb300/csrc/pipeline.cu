@@ -41,11 +41,16 @@ std::vector<uint64_t> chunk_ends(uint64_t n_tokens) {
 
 // Chunks of a text of `tiles` parser tiles copied from the host: 16 MB (32 MB
 // from pageable memory, whose copies each cost the host some work), then a third
-// of what is left, down to 4 MB (8 MB), in tiles before the end of each.
+// of what is left, down to 4 MB (8 MB), in tiles before the end of each.  A text of
+// up to 48 MB is one chunk: a chunk's launches take as long as the copy they would
+// overlap (19 / 32 / 44 / 54 / 64 MB pinned, chunks 311 / 413 / 493 / 539 / 603 us, one
+// 285 / 386 / 481 / 557 / 652; pageable 340 / 447 / 541 / 613 / 702 and 308 / 421 / 526 /
+// 620 / 715).
 constexpr uint64_t PARSE_TILE_BYTES = 4096;
 std::vector<uint64_t> parse_chunk_ends(uint64_t tiles, bool pinned) {
     const uint64_t MOST = (pinned ? 16ull << 20 : 32ull << 20) / PARSE_TILE_BYTES;
     const uint64_t LEAST = (pinned ? 4ull << 20 : 8ull << 20) / PARSE_TILE_BYTES;
+    if (tiles <= (48ull << 20) / PARSE_TILE_BYTES) return {tiles};
     std::vector<uint64_t> ends;
     for (uint64_t t = 0; t < tiles;) {
         const uint64_t left = tiles - t;
