@@ -120,6 +120,7 @@ hyset_status hyset_collection_parse(hyset_ctx* ctx, const char* text, uint64_t n
     auto landed = on_exit([&] {  // no return while a copy may still write the staged text
         if (copied) cudaStreamSynchronize(ctx->aux);
     });
+    ST(copy_chunks(pinned ? n_chunks : 2));  // on their way while the scratch is set up
     if (n_bytes && (reinterpret_cast<uintptr_t>(d_text) & 15u)) {  // tiles load 16-byte words
         DevBuf aligned;
         CK(aligned.ensure(n_bytes + 16, s));
@@ -169,7 +170,7 @@ hyset_status hyset_collection_parse(hyset_ctx* ctx, const char* text, uint64_t n
         uint32_t tok_cap = 0, line_cap = 0;
         for (uint64_t k = 0; k < n_chunks; ++k) {
             const uint64_t t0 = k ? ends[k - 1] : 0, t1 = ends[k];
-            ST(copy_chunks(pinned ? n_chunks : k + 2));
+            ST(copy_chunks(k + 2));
             CK(cudaStreamWaitEvent(s, pipe_event(ctx, std::min(k + 1, n_chunks - 1)), 0));
             CK(parse_count(d_text, n_bytes, tile_toks, tile_lines, flags, first_bad, s, t0, t1));
             CK(parse_chunk_scan(tile_toks, tile_lines, t0, t1, carry, k, s));
