@@ -389,6 +389,9 @@ hyset_status batch_prepare(hyset_ctx* ctx, const hyset_join_desc* joins, uint32_
     CK(cudaStreamSynchronize(s));
     ctx->batch = std::move(plan);
     BatchPlan& bp = *ctx->batch;
+    auto installed = on_exit([&] {  // a plan without its graph is not kept: the same batch would replay nothing
+        if (ctx->batch && !ctx->batch->exec) batch_release(ctx);
+    });
     // indexes whose list path is not known yet are built once here, outside
     // the capture, so that the path is read back and remembered: the graph then
     // holds only the kernels of the path each index takes
@@ -413,15 +416,11 @@ hyset_status batch_prepare(hyset_ctx* ctx, const hyset_join_desc* joins, uint32_
     cudaError_t e = cudaStreamEndCapture(s, &g);
     if (st != HYSET_OK || e != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
-        batch_release(ctx);
         return st != HYSET_OK ? st : fail(ctx, HYSET_E_CUDA, "batch graph capture", e);
     }
     bp.graph = g;
     e = cudaGraphInstantiate(&bp.exec, g, 0);
-    if (e != cudaSuccess) {
-        batch_release(ctx);
-        return fail(ctx, HYSET_E_CUDA, "batch graph instantiation", e);
-    }
+    if (e != cudaSuccess) return fail(ctx, HYSET_E_CUDA, "batch graph instantiation", e);
     return HYSET_OK;
 }
 }  // namespace
